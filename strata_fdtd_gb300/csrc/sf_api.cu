@@ -106,6 +106,7 @@ void sf_defer_graph(cudaGraphExec_t exec, cudaGraph_t graph) {
 }
 
 extern "C" int sf_release_deferred(void) {
+    sf_voxel_release_kept();
     std::lock_guard<std::mutex> lock(g_def_mu);
     release_deferred_locked();
     return 0;
@@ -1113,44 +1114,12 @@ int sf_plan_energy(sf_plan* P, double rho, double c, double dx, double* scratch,
 
 namespace {
 
-// Upload the program (and the cell centres of a nonuniform grid), voxelise,
-// and report a malformed program.
 int voxelize_impl(const sf_sdf_node* nodes, int n_nodes, int nx, int ny, int nz,
                   double res, const double* const* coords, int invert, uint8_t* out_dev,
                   cudaStream_t st) {
     if (!nodes || n_nodes < 1 || !out_dev) return sf_fail("sf_voxelize: bad program or output");
     if (nx < 1 || ny < 1 || nz < 1 || nx > 65535) return sf_fail("sf_voxelize: bad grid");
-    const size_t prog_bytes = (sizeof(sf_sdf_node) * n_nodes + 15) / 16 * 16;
-    const size_t coord_bytes = coords ? sizeof(double) * ((size_t)nx + ny + nz) : 0;
-    char* buf = nullptr;  // stream-ordered: no device-wide wait on release
-    SF_CUDA_OK(cudaMallocAsync(reinterpret_cast<void**>(&buf), prog_bytes + 16 + coord_bytes, st));
-    sf_sdf_node* prog = reinterpret_cast<sf_sdf_node*>(buf);
-    int* err = reinterpret_cast<int*>(buf + prog_bytes);
-    double* cdev = coords ? reinterpret_cast<double*>(buf + prog_bytes + 16) : nullptr;
-    int rc = 0;
-    int herr = 0;
-    if (cudaMemcpyAsync(prog, nodes, sizeof(sf_sdf_node) * n_nodes, cudaMemcpyHostToDevice, st) !=
-            cudaSuccess ||
-        cudaMemsetAsync(err, 0, sizeof(int), st) != cudaSuccess) {
-        rc = sf_fail("sf_voxelize: upload failed");
-    }
-    if (!rc && coords) {
-        const int n3[3] = {nx, ny, nz};
-        size_t off = 0;
-        for (int a = 0; a < 3 && !rc; ++a) {
-            if (cudaMemcpyAsync(cdev + off, coords[a], sizeof(double) * n3[a],
-                                cudaMemcpyHostToDevice, st) != cudaSuccess)
-                rc = sf_fail("sf_voxelize: coordinate upload failed");
-            off += n3[a];
-        }
-    }
-    if (!rc) rc = sf_launch_voxelize(prog, n_nodes, nx, ny, nz, res, cdev, invert, out_dev, err, st);
-    if (!rc && (cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-                cudaStreamSynchronize(st) != cudaSuccess))
-        rc = sf_fail("sf_voxelize: kernel failed");
-    cudaFreeAsync(buf, st);
-    if (!rc && herr) rc = sf_fail("sf_voxelize: malformed SDF program (stack error)");
-    return rc;
+    return sf_launch_voxelize(nodes, n_nodes, nx, ny, nz, res, coords, invert, out_dev, st);
 }
 
 }  // namespace

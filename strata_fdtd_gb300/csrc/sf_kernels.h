@@ -123,9 +123,9 @@ long long sf_energy_blocks(long long n, int sms);
 int sf_launch_energy(const float* p, const float* vx, const float* vy, const float* vz,
                      const uint8_t* flags, long long n, int sms, double* scratch, double* out2,
                      cudaStream_t st);
-int sf_launch_voxelize(const sf_sdf_node* prog_dev, int n_nodes, int nx, int ny, int nz,
-                       double res, const double* coords_dev, int invert, uint8_t* out,
-                       int* err_dev, cudaStream_t st);
+int sf_launch_voxelize(const sf_sdf_node* nodes, int n_nodes, int nx, int ny, int nz, double res,
+                       const double* const* coords, int invert, uint8_t* out, cudaStream_t st);
+void sf_voxel_release_kept();
 int sf_launch_voxelize_materials(const sf_sdf_node* prog_dev, const int* off_dev,
                                  const uint8_t* ids_dev, int n_regions, int nx, int ny, int nz,
                                  double res, const double* coords_dev, uint8_t* geom,
