@@ -276,7 +276,9 @@ const char* sf_kernel_config_name(int config);
  * dependency wait expired" in sf_last_error(); the state of that call is
  * void and the next call starts clean.  hold_first_item != 0 is a test hook:
  * the first work item also waits on a device flag that nothing sets, so the
- * expiry path runs without any fault.  No counterpart in the reference. */
+ * expiry path runs without any fault.  The state-on-chip kernel's waits count
+ * polls of about half a microsecond against the same bound (default 2^23) and
+ * report through sf_plan_status.  No counterpart in the reference. */
 int sf_plan_set_wait_limit(sf_plan* plan, int64_t spins, int hold_first_item);
 
 /* Autotuner: times every single-step configuration (the multi-step
@@ -308,6 +310,19 @@ int sf_plan_step(sf_plan* plan, int64_t n_steps, const double* src_values_dev,
  * (may be NULL). */
 int sf_plan_step_ex(sf_plan* plan, int64_t n_steps, const double* src_values_dev,
                     float* trace_dev, float* mic_trace_dev, void* stream);
+
+/* Whether sf_plan_step_ex with n_steps steps (and, with_mics != 0, microphone
+ * rows) on this stream now runs the state-on-chip kernel, which advances all of
+ * them in one launch (automatic kernel choice, grids that fit on the SMs, no
+ * ADE poles, plane boundaries or weighted sources, no stream capture): 1 or 0.
+ * A caller that replays captured launches of its own need not do so then.  No
+ * counterpart in the reference. */
+int sf_plan_resident(sf_plan* plan, int64_t n_steps, int with_mics, void* stream);
+/* Nonzero, once, when a bounded wait of an earlier state-on-chip launch of this
+ * plan expired (that call's results are void).  The launch itself is
+ * asynchronous; sf_plan_step_ex and sf_plan_energy report it too.  No
+ * counterpart in the reference. */
+int sf_plan_status(sf_plan* plan);
 
 /* Acoustic energy of the current state, (1/2) sum(p^2/(rho c^2) + rho v^2)
  * dV over air cells, as compute_energy (core/solver.py:2689-2705); result

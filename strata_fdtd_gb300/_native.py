@@ -18,7 +18,7 @@ ROOT = os.path.dirname(PKG)
 BUILD = os.path.join(PKG, "_build")
 LIB_PATH = os.path.join(BUILD, "libsf_gb300.so")
 SOURCES = ("sf_step.cu", "sf_step_march.cu", "sf_step_col.cu", "sf_step_tile.cu", "sf_step_pipe.cu",
-           "sf_step_tb.cu", "sf_voxel.cu", "sf_batch.cu", "sf_adjoint.cu", "sf_api.cu")
+           "sf_step_tb.cu", "sf_step_resident.cu", "sf_voxel.cu", "sf_batch.cu", "sf_adjoint.cu", "sf_api.cu")
 ARCH = "-gencode=arch=compute_103a,code=sm_103a"
 NVCC_FLAGS = ["-O3", "-lineinfo", "-fmad=false", "-std=c++17", "-Xcompiler", "-fPIC",
               "--expt-relaxed-constexpr"]
@@ -123,6 +123,8 @@ SIGNATURES = {
     "sf_kernel_config_count": (_I, []),
     "sf_kernel_config_name": (ctypes.c_char_p, [_I]),
     "sf_plan_autotune": (_I, [_P, _I, _P, _P, _P]),
+    "sf_plan_resident": (_I, [_P, _I64, _I, _P]),
+    "sf_plan_status": (_I, [_P]),
     "sf_plan_step": (_I, [_P, _I64, _P, _P, _P]),
     "sf_plan_step_ex": (_I, [_P, _I64, _P, _P, _P, _P]),
     "sf_plan_set_microphones": (_I, [_P, _I, _P, _P]),

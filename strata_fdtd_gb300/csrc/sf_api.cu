@@ -54,6 +54,11 @@ int sf_fail_cuda(cudaError_t e, const char* what, const char* file, int line) {
 
 int sf_noalloc_setup(int dev);  // defined with the no-alloc energy array below
 
+namespace {
+void resident_release();  // defined with the state-on-chip launches below
+void resident_slot_free(sf_plan* P);
+}  // namespace
+
 // Deferred device frees.  cudaFree waits for all work on the device, so a
 // plan or a batch released while other solves' kernels run would stall the
 // host until they finish (a served stream retires and builds solves while
@@ -107,10 +112,97 @@ void sf_defer_graph(cudaGraphExec_t exec, cudaGraph_t graph) {
 
 extern "C" int sf_release_deferred(void) {
     sf_voxel_release_kept();
+    resident_release();
     std::lock_guard<std::mutex> lock(g_def_mu);
     release_deferred_locked();
     return 0;
 }
+
+// ---- state-on-chip launches (sf_step_resident.cu) ---------------------------
+//
+// Per device: the mailboxes every launch uses (grown on demand, released with
+// the deferred frees when idle), the next message tag, an event that orders the
+// launches of all streams and threads one after another (each takes every SM
+// its cut names, so two at once could wait for each other's SMs), and a page of
+// host-mapped error words, one per plan.
+namespace {
+constexpr int kResDevices = 64, kResSlots = 4096;
+constexpr size_t kResMailMax = size_t(64) << 20;
+constexpr int kResChunk = 4096;        // steps per launch
+constexpr int kResMinSteps = 8;        // shorter calls step launch by launch
+constexpr long long kResPolls = 1LL << 23;  // polls (about 0.5 us each) before a wait gives up
+struct ResDevice {
+    char* mail = nullptr;
+    size_t bytes = 0;
+    unsigned tag = 1;
+    cudaEvent_t done = nullptr;
+    int* err_host = nullptr;
+    int* err_dev = nullptr;
+    std::vector<int> free_slots;
+};
+std::mutex g_res_mu;
+ResDevice g_res[kResDevices];
+
+// The plan's error word; without one (no page, or none left) no resident steps.
+bool resident_slot(sf_plan* P) {
+    if (P->res_slot >= 0) return true;
+    if (P->device < 0 || P->device >= kResDevices) return false;
+    std::lock_guard<std::mutex> lock(g_res_mu);
+    ResDevice& D = g_res[P->device];
+    if (!D.err_host) {
+        void* h = nullptr;
+        if (cudaHostAlloc(&h, sizeof(int) * kResSlots, cudaHostAllocMapped | cudaHostAllocPortable) !=
+            cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        void* d = nullptr;
+        if (cudaHostGetDevicePointer(&d, h, 0) != cudaSuccess ||
+            cudaEventCreateWithFlags(&D.done, cudaEventDisableTiming) != cudaSuccess) {
+            (void)cudaGetLastError();
+            cudaFreeHost(h);
+            return false;
+        }
+        std::memset(h, 0, sizeof(int) * kResSlots);
+        D.err_host = static_cast<int*>(h);
+        D.err_dev = static_cast<int*>(d);
+        for (int q = kResSlots - 1; q >= 0; --q) D.free_slots.push_back(q);
+    }
+    if (D.free_slots.empty()) return false;
+    P->res_slot = D.free_slots.back();
+    D.free_slots.pop_back();
+    P->res_err = D.err_host + P->res_slot;
+    P->res_err_dev = D.err_dev + P->res_slot;
+    *P->res_err = 0;
+    return true;
+}
+
+void resident_slot_free(sf_plan* P) {
+    if (P->res_slot < 0) return;
+    std::lock_guard<std::mutex> lock(g_res_mu);
+    g_res[P->device].free_slots.push_back(P->res_slot);
+    P->res_slot = -1;
+}
+
+// Whether an earlier launch of this plan gave up on a wait (reported once).
+int resident_status(sf_plan* P) {
+    if (P->res_slot < 0 || *static_cast<volatile int*>(P->res_err) == 0) return 0;
+    *static_cast<volatile int*>(P->res_err) = 0;
+    return sf_fail("k_resident: a dependency wait expired (results of that call are invalid)");
+}
+
+void resident_release() {
+    std::lock_guard<std::mutex> lock(g_res_mu);
+    for (int d = 0; d < kResDevices; ++d) {
+        ResDevice& D = g_res[d];
+        if (!D.mail || cudaEventQuery(D.done) != cudaSuccess) continue;
+        DeviceGuard g(d);
+        cudaFree(D.mail);
+        D.mail = nullptr;
+        D.bytes = 0;
+    }
+}
+}  // namespace
 
 namespace {
 
@@ -204,6 +296,7 @@ int sf_plan_destroy(sf_plan* P) {
         sf_defer_free(P->wsrc_cells[q], 0);
         sf_defer_free(P->wsrc_w[q], 0);
     }
+    resident_slot_free(P);
     sf_defer_free(P->pipe_ring, P->pipe_ring_floats * sizeof(float));
     sf_defer_free(P->pipe_ctrl, 0);
     sf_defer_free(P->pipe_err, 0);
@@ -842,9 +935,98 @@ int pipe_check(sf_plan* P, cudaStream_t st) {
     return sf_fail("k_step_pipe: a dependency wait expired (results of this call are invalid)");
 }
 
+// Whether n steps of this plan run on the state-on-chip path: automatic
+// kernel choice, nothing between the steps but probes, no ADE poles, a grid
+// whose blocks fit on the SMs, enough steps to pay for loading the state, and
+// no stream capture (a captured launch would keep its message tags).
+bool resident_fits(sf_plan* P, const SfStepArgs& a, int64_t n_steps, bool deferred, bool mics,
+                   cudaStream_t st) {
+    if (P->variant != SF_CFG_AUTO || P->i_chunk != 0 || P->poles.n > 0 || deferred || mics ||
+        n_steps < kResMinSteps || P->n_probe > 1024 || stream_capturing(st))
+        return false;
+    const int key[2] = {a.n_probe, P->nu != nullptr};
+    if (P->res_key[0] != key[0] || P->res_key[1] != key[1]) {
+        P->res_cut = sf_resident_cut(P->d.nx, P->d.ny, P->d.nz, a.n_probe, P->nu != nullptr, P->sms);
+        P->res_key[0] = key[0];
+        P->res_key[1] = key[1];
+    }
+    return P->res_cut.kind >= 0 && resident_slot(P);
+}
+
+// n steps of the plan from its current set, in launches of at most kResChunk.
+int step_resident(sf_plan* P, const SfStepArgs& a0, int64_t n_steps, const double* src_values,
+                  float* trace, cudaStream_t st) {
+    const SfResCut& c = P->res_cut;
+    const size_t mail = (size_t)2 * c.bi * c.bj * c.bk * 6 * c.side_max * 4 * sizeof(unsigned long long);
+    if (mail > kResMailMax) return sf_fail("k_resident: mailboxes too large");
+    std::lock_guard<std::mutex> lock(g_res_mu);
+    ResDevice& D = g_res[P->device];
+    SF_CUDA_OK(cudaStreamWaitEvent(st, D.done, 0));
+    if (D.bytes < mail) {
+        cudaFree(D.mail);  // waits for the launches that use it
+        D.mail = nullptr;
+        D.bytes = 0;
+        SF_CUDA_OK(cudaMalloc(&D.mail, mail));
+        D.bytes = mail;
+        D.tag = 0xffffffffu;  // cleared below
+    }
+    for (int64_t s = 0; s < n_steps;) {
+        const int n = (int)std::min<int64_t>(kResChunk, n_steps - s);
+        if (D.tag > 0xffffffffu - kResChunk) {  // new mailboxes, or the tags wrapped
+            SF_CUDA_OK(cudaMemsetAsync(D.mail, 0, D.bytes, st));
+            D.tag = 1;
+        }
+        SfResArgs A{};
+        A.a = a0;
+        const int out = P->cur ^ (n & 1);  // the set n single steps would end on
+        set_io(P, A.a, P->cur);
+        A.a.po = P->f[out][0];
+        A.a.vxo = P->f[out][1];
+        A.a.vyo = P->f[out][2];
+        A.a.vzo = P->f[out][3];
+        A.a.src_val = P->src.n > 0 ? src_values + s * P->src.n : nullptr;
+        A.a.trace_prev = a0.n_probe > 0 ? trace + s * a0.n_probe : nullptr;
+        A.n_steps = n;
+        A.mail = reinterpret_cast<unsigned long long*>(D.mail);
+        A.tag = D.tag;
+        A.err = P->res_err_dev;
+        A.poll_limit = P->pipe_spin_limit > 0 ? P->pipe_spin_limit : kResPolls;
+        A.hold = P->pipe_hold ? 1 : 0;
+        if (int rc = sf_launch_resident(A, P->src, c, st)) return rc;
+        D.tag += (unsigned)n;
+        P->cur = out;
+        P->steps_done += n;
+        s += n;
+    }
+    SF_CUDA_OK(cudaEventRecord(D.done, st));
+    return 0;
+}
+
+bool defers(const sf_plan* P) {  // plane boundaries or weighted sources act after the fused kernel
+    bool d = P->n_plane > 0;
+    for (int q = 0; q < P->src.n; ++q) d = d || P->src.s[q].kind == 2;
+    return d;
+}
+
 }  // namespace
 
 extern "C" {
+
+int sf_plan_resident(sf_plan* P, int64_t n_steps, int with_mics, void* stream) {
+    if (!P || !P->bound) return 0;
+    DeviceGuard g(P->device);
+    SfStepArgs a;
+    fill_args(P, a, P->n_probe > 0);
+    return resident_fits(P, a, n_steps, defers(P), with_mics != 0 && P->n_mic > 0,
+                         static_cast<cudaStream_t>(stream))
+               ? 1
+               : 0;
+}
+
+int sf_plan_status(sf_plan* P) {
+    if (!P) return sf_fail("sf_plan_status: NULL plan");
+    return resident_status(P);
+}
 
 int sf_plan_step(sf_plan* P, int64_t n_steps, const double* src_values, float* trace,
                  void* stream) {
@@ -858,16 +1040,18 @@ int sf_plan_step_ex(sf_plan* P, int64_t n_steps, const double* src_values, float
     if (n_steps < 0) return sf_fail("sf_plan_step: negative step count");
     if (P->src.n > 0 && !src_values) return sf_fail("sf_plan_step: sources need src_values");
     if (n_steps == 0) return 0;
+    if (int rc = resident_status(P)) return rc;
     DeviceGuard g(P->device);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     SfStepArgs a;
     fill_args(P, a, trace != nullptr);
     set_io(P, a, P->cur);  // both sets: the alignment check covers every field
-    const int cfg0 = effective_config(P, a);
     const bool mics = mic_trace != nullptr && P->n_mic > 0;
     // plane boundaries or weighted sources: sources move after the fused kernel
-    bool deferred = P->n_plane > 0;
-    for (int q = 0; q < P->src.n; ++q) deferred = deferred || P->src.s[q].kind == 2;
+    const bool deferred = defers(P);
+    if (resident_fits(P, a, n_steps, deferred, mics, st))
+        return step_resident(P, a, n_steps, src_values, trace, st);
+    const int cfg0 = effective_config(P, a);
     // A pipeline configuration runs whole groups of its steps per launch when
     // nothing has to happen between steps; remaining steps (and plans with
     // microphones, plane boundaries or weighted sources) run single steps
@@ -1105,6 +1289,7 @@ int sf_plan_energy(sf_plan* P, double rho, double c, double dx, double* scratch,
     double sums[2];
     SF_CUDA_OK(cudaMemcpyAsync(sums, scratch + 2 * nb, sizeof(sums), cudaMemcpyDeviceToHost, st));
     SF_CUDA_OK(cudaStreamSynchronize(st));
+    if (int rc = resident_status(P)) return rc;
     const double dV = dx * dx * dx;
     *out_host = 0.5 * sums[0] / (rho * c * c) * dV + 0.5 * rho * sums[1] * dV;
     return 0;

@@ -96,6 +96,43 @@ bool sf_tb_supported(const SfStepArgs& a);
 int sf_launch_step_tb(const SfStepArgs& a, const SfSources& src, bool geom, int cfg, int ich,
                       float* trace1, cudaStream_t st);
 
+// Many steps of a small grid in one launch, its state on the chip
+// (sf_step_resident.cu).  A cut says how the grid is divided into blocks.
+// Shared memory of a block: offsets in floats (multiples of 4).
+struct SfResLayout {
+    int src;             // this step's source values (doubles)
+    int ctl;             // [1] probes, [2] a wait expired
+    int side;            // (decay, coefficient) of each side's faces
+    int P, UX, UY, UZ;   // pressures; x faces at chunk ends, y faces, z faces
+    int dx, dy, dz;      // PML decays of the block's planes, rows, cells
+    int cx, cy, cz, sx, sy, sz;  // NU: face coefficients, cell scales
+    int probe;           // (trace column, cell in P)
+    int end;
+};
+struct SfResCut {
+    int kind;          // planes per thread and thread counts (kKinds), < 0: does not fit
+    int bi, bj, bk;    // blocks along x, y, z
+    int chunks, quads; // chunks of planes and quads of k cells in the grid
+    int threads;
+    int side_max;      // message units of the largest block side
+    int units;         // message units of a block at most
+    SfResLayout lay;
+    size_t smem;
+};
+struct SfResArgs {
+    SfStepArgs a;      // a.src_val, a.trace_prev: the first step's rows
+    int n_steps;
+    int bi, bj, bk, chunks, quads, side_max;
+    SfResLayout lay;
+    unsigned long long* mail;  // 2 x blocks x 6 x side_max x 4 words
+    unsigned tag;      // the first step's tag
+    int* err;          // set when a wait expired
+    long long poll_limit;
+    int hold;          // expiry test hook: block 0 waits for tags nothing sends
+};
+SfResCut sf_resident_cut(int nx, int ny, int nz, int n_probe, bool nu, int sms);
+int sf_launch_resident(SfResArgs& A, const SfSources& src, const SfResCut& c, cudaStream_t st);
+
 int sf_launch_build_flags(const uint8_t* geom, uint8_t* flags, int nx, int ny, int nz,
                           cudaStream_t st);
 int sf_launch_step(const SfStepArgs& a, const SfSources& src, const SfPoles& poles, bool geom,

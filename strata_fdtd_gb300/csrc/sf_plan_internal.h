@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "sf_common.cuh"
+#include "sf_kernels.h"
 
 struct sf_plan {
     sf_grid_desc d{};
@@ -53,6 +54,12 @@ struct sf_plan {
     int pipe_key[4] = {0, 0, 0, 0};  // levels, planes per chunk, lag, ring chunks of the order
     int pipe_grid[2] = {0, 0};       // configuration + 1, resident blocks
     int probe_tile_max = 0;          // most probes in one 32 k x 4 row tile column
+    // state-on-chip path (sf_step_resident.cu)
+    SfResCut res_cut{};              // of the probe count and spacing in res_key
+    int res_key[2] = {-1, -1};
+    int* res_err = nullptr;          // host-mapped word, set when a wait expired
+    int* res_err_dev = nullptr;      // its device address
+    int res_slot = -1;
 };
 
 // Planes per block: enough (j,k)-tile x i-chunk blocks for about four waves

@@ -301,10 +301,17 @@ class FDTDSolver:
         if not self._host_fresh[name]:
             src = self._dev[self._cur()][_FIELDS.index(name)]
             self._torch.from_numpy(self._host[name]).copy_(src)
+            self._check_status()
             self._host_fresh[name] = True
         self._host_exposed[name] = True
         self._vz_seen = self._vz_seen or name == "vz"
         return self._host[name]
+
+    def _check_status(self):
+        """Raise when an earlier asynchronous run of this solver failed."""
+        twin = getattr(self, "_pad_twin", None)
+        for plan in (self._plan,) if twin is None else (self._plan, twin.plan):
+            _native.check(self._lib.sf_plan_status(plan), "sf_plan_step")
 
     def _set_field(self, name, value):
         arr = np.asarray(value)
@@ -381,6 +388,7 @@ class FDTDSolver:
 
         def result() -> dict:
             done.synchronize()
+            self._check_status()
             return {n: t.numpy() for n, t in dst.items()}
 
         return result
@@ -826,6 +834,16 @@ class FDTDSolver:
     _TWIN_MIN_STEPS = 32  # runs this long go through the padded twin (two state copies)
     _GRAPH_STEPS = 50     # steps per captured CUDA graph (even: the current set comes back)
 
+    def _graph_cache(self, owner) -> dict:
+        """``owner``'s captured graphs, emptied when the tables or the kernel
+        choice have changed since they were captured."""
+        stamp = (self._tables_version, self._graph_epoch)
+        cache = owner.__dict__.setdefault("_graphs", {})
+        if cache.get("stamp") != stamp:
+            cache.clear()
+            cache["stamp"] = stamp
+        return cache
+
     def _graph_for(self, owner, plan, n_src: int, n_probe: int):
         """A CUDA graph of _GRAPH_STEPS steps of ``plan`` from its current
         set, reading the source values of those steps from a device buffer
@@ -836,11 +854,7 @@ class FDTDSolver:
         overhead."""
         torch = self._torch
         cur = int(self._lib.sf_plan_current(plan))
-        stamp = (self._tables_version, self._graph_epoch)
-        cache = owner.__dict__.setdefault("_graphs", {})
-        if cache.get("stamp") != stamp:
-            cache.clear()
-            cache["stamp"] = stamp
+        cache = self._graph_cache(owner)
         key = (cur, n_src, n_probe)
         if key in cache:
             return cache[key]
@@ -867,6 +881,7 @@ class FDTDSolver:
         vz_handed_out = self._host_exposed["vz"]
         self._sync_tables()
         self._upload_exposed()
+        n_mic = getattr(self, "_mic_rows", 0)
         twin = None
         if n >= self._TWIN_MIN_STEPS and self._kernel_auto:
             twin = self._padded_twin(vz_handed_out)
@@ -874,15 +889,19 @@ class FDTDSolver:
         n_probe = len(self._probe_order)
         trace = (torch.empty((n, n_probe), dtype=torch.float32, device=self._device)
                  if n_probe else None)
-        n_mic = getattr(self, "_mic_rows", 0)
         mic_trace = (torch.empty((n, n_mic), dtype=torch.float32, device=self._device)
                      if n_mic else None)
         if twin is not None:
             twin.copy_in(self)
         plan = self._plan if twin is None else twin.plan
+        # a grid that fits on the chip runs all n steps in one launch
+        resident = bool(self._lib.sf_plan_resident(plan, n, n_mic, self._stream()))
+        if resident:
+            self._graph_cache(self)  # graphs of earlier tables are dropped here too
         G = self._GRAPH_STEPS
         n_graph = 0
-        if mic_trace is None and self._kernel_auto and not torch.cuda.is_current_stream_capturing():
+        if (mic_trace is None and self._kernel_auto and not resident
+                and not torch.cuda.is_current_stream_capturing()):
             n_graph = n - n % G  # (inside a caller's capture the launches go into its graph)
         if n_graph:
             g, gsrc, gtrace = self._graph_for(twin if twin is not None else self, plan,
@@ -915,6 +934,7 @@ class FDTDSolver:
     def _flush_traces(self):
         for trace, names in self._pending_traces:
             host = trace.cpu().numpy()
+            self._check_status()
             for q, name in enumerate(names):
                 if name in self._probes:
                     self._probes[name]._samples.extend(host[:, q].tolist())
@@ -1109,6 +1129,7 @@ class FDTDSolver:
 
     def synchronize(self) -> None:
         self._torch.cuda.synchronize(self._device)
+        self._check_status()
 
     # ----------------------------------------------------------------- outputs
     def probe_data_async(self):
@@ -1132,6 +1153,7 @@ class FDTDSolver:
 
         def result() -> dict:
             done.synchronize()
+            self._check_status()
             for host, names in copies:
                 arr = host.numpy()
                 for q, name in enumerate(names):
