@@ -28,6 +28,7 @@
 #define SF_CFG_DEFAULT (SF_CFG_COL_FIRST + 0)
 #define SF_CFG_TILE_FIRST (SF_CFG_COL_FIRST + kSfColConfigCount)
 #define SF_CFG_TILE_DEFAULT (SF_CFG_TILE_FIRST + 2)
+#define SF_CFG_TILE_WALLS (SF_CFG_TILE_FIRST + 14)
 #define SF_CFG_TILE1_DEFAULT (SF_CFG_TILE_FIRST + 11)
 #define SF_CFG_PIPE_FIRST (SF_CFG_TILE_FIRST + kSfTileConfigCount)
 #define SF_CFG_TB_FIRST (SF_CFG_PIPE_FIRST + kSfPipeConfigCount)
@@ -639,9 +640,16 @@ bool is_tb(int cfg) { return cfg >= SF_CFG_TB_FIRST; }
 bool tb_fits(const sf_plan* P, const SfStepArgs& a) {
     return P->poles.n == 0 && P->nu == nullptr && sf_tb_supported(a);
 }
+// float4 warp tiles of 8 blocks per SM (64 registers) without flag bytes, of 6
+// blocks (80) and write-back stores with them, whose masks spill at 64: GB300,
+// 400^3 enclosure 411 -> 336 us a step, 256^3 with a wall 102 -> 92, 120 x 300 x
+// 260 63 -> 57; without walls 320 x 256 x 200 88.5 against 93, 150^3 20.8
+// against 21.9.  Nonuniform grids (more coefficients in registers) take the
+// second too: 240 x 200 x 128 without walls 39.2 -> 35.1.
 int default_single(const SfStepArgs& a) {
-    return sf_tile_supported(a, 4) ? SF_CFG_TILE_DEFAULT
-                                   : (sf_tile_supported(a, 1) ? SF_CFG_TILE1_DEFAULT : SF_CFG_DEFAULT);
+    if (sf_tile_supported(a, 4))
+        return a.flags != nullptr || a.nu_cv[0] != nullptr ? SF_CFG_TILE_WALLS : SF_CFG_TILE_DEFAULT;
+    return sf_tile_supported(a, 1) ? SF_CFG_TILE1_DEFAULT : SF_CFG_DEFAULT;
 }
 bool pipe_fits(sf_plan* P, int cfg, const SfStepArgs& a);
 int chunk_for(const sf_plan* P, int cfg);
@@ -650,8 +658,7 @@ int effective_config(const sf_plan* P, const SfStepArgs& a) {
     int cfg;
     if (P->variant != SF_CFG_AUTO) cfg = P->variant;
     else if (P->tuned > 0) cfg = P->tuned;
-    else if (sf_tile_supported(a, 4)) cfg = SF_CFG_TILE_DEFAULT;
-    else cfg = sf_tile_supported(a, 1) ? SF_CFG_TILE1_DEFAULT : SF_CFG_DEFAULT;
+    else cfg = default_single(a);
     if (is_pipe(cfg)) {  // when the pipeline fits the plan; else the default choice
         if (pipe_fits(const_cast<sf_plan*>(P), cfg, a)) return cfg;
         cfg = default_single(a);
@@ -696,6 +703,32 @@ void ade_region(const sf_plan* P, int cfg, int ich, int lo[3], int hi[3]) {
 }
 
 
+// Planes per block of a float4 warp-tile configuration: of 4 to 8 and
+// auto_chunk's choice where that is larger, the number with the best product of
+// (blocks / whole waves of resident blocks) and (planes / planes + half a plane
+// for the chunk's prologue), among those that fill one wave.  Against
+// auto_chunk alone (4 planes for these): 203 x 167 x 184 with walls 40.8 -> 39.9
+// us a step, 176 x 152 x 144 27.2 -> 26.3, free 300 x 90 x 120 20.5 -> 18.7.
+int tile_chunk(const sf_plan* P, const SfTileConfig& t) {
+    const int jspan = 4 * t.rows * t.warps;
+    const long long cols = (long long)((P->d.nz + 31) / 32) * ((P->d.ny + jspan - 1) / jspan);
+    const long long wave = (long long)t.minb * P->sms;
+    int cand[6] = {4, 5, 6, 7, 8, auto_chunk(P, 32, jspan)};
+    int best = P->d.nx < 4 ? P->d.nx : 4;
+    double best_eff = 0.0;
+    for (int ich : cand) {
+        if (ich > P->d.nx) continue;
+        const long long blocks = cols * ((P->d.nx + ich - 1) / ich);
+        if (blocks < 0.95 * wave) continue;
+        const double eff = (double)blocks / (double)((blocks + wave - 1) / wave * wave) * ich / (ich + 0.5);
+        if (eff > best_eff) {
+            best_eff = eff;
+            best = ich;
+        }
+    }
+    return best;
+}
+
 int chunk_for(const sf_plan* P, int cfg) {
     if (P->i_chunk > 0) return P->i_chunk;
     if (cfg == P->tuned && P->tuned_ich > 0) return P->tuned_ich;
@@ -719,7 +752,7 @@ int chunk_for(const sf_plan* P, int cfg) {
     if (cfg >= SF_CFG_TILE_FIRST) {
         const SfTileConfig& t = kSfTileConfigs[cfg - SF_CFG_TILE_FIRST];
         if (t.vec == 1) return auto_chunk(P, 32, t.rows * t.warps);
-        if (P->d.nz % 4 == 0) return auto_chunk(P, 32, 4 * t.rows * t.warps);
+        if (P->d.nz % 4 == 0) return tile_chunk(P, t);
         return auto_chunk(P, 32);
     }
     int kspan = 32;
