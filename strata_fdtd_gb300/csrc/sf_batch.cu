@@ -5,21 +5,22 @@
 // per time step.  Every grid is cut into work items (i-chunk x a block of
 // rows x 32 columns); the warps of the persistent kernel claim items one at a
 // time from a device-wide work queue (one atomic counter, no block
-// barriers), so uneven grids load-balance across the SMs.  Items that meet a
-// grid's material box run the ADE column path (the arithmetic and order of
-// core/solver.py:2135-2193 and ade.cpp); the others run the batch's plain
-// path: thread columns or warp tiles (sf_tile.cuh).  Every path is the
-// per-cell arithmetic of k_step, so a grid's result is bit-identical alone
-// or in the batch.
+// barriers), so uneven grids load-balance across the SMs.  The items run the
+// batch's plain path: thread columns or warp tiles (sf_tile.cuh).  Tiles that
+// meet a grid's material box go to k_batch_ade instead, cut into short columns
+// (the arithmetic and order of core/solver.py:2135-2193 and ade.cpp).  Every
+// path is the per-cell arithmetic of k_step, so a grid's result is
+// bit-identical alone or in the batch.
 //
 // Per step the batch enqueues: the ADE density pre-pass over the material
-// boxes (if any grid has density poles), the persistent kernel, the probe
-// gather, and a one-thread kernel that advances the device step counter and
-// resets the queue.  The kernels read the step number from device memory, so
-// a run of steps can be captured once as a CUDA graph and replayed.  Grids
-// drop out of the work when they reach their own step count: members are
-// listed longest run first, so a finished grid's items end their segment of
-// the queue, and the first warp to claim one skips the rest of the segment.
+// boxes (if any grid has density poles) and k_batch_ade, beside them (a parallel
+// branch of a captured graph) the persistent kernel, then the probe gather and
+// a one-thread kernel that advances the device step counter and resets the
+// queue.  The kernels read the step number from device memory, so a run of
+// steps can be captured once as a CUDA graph and replayed.  Grids drop out of
+// the work when they reach their own step count: members are listed longest
+// run first, so a finished grid's items end the queue, and the first warp to
+// claim one stops there.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -77,13 +78,11 @@ __device__ __forceinline__ float ade_face_g(float v, const SfPoles& P, uint8_t m
 // One row of an item: lane l of the warp walks cells (i0..i1-1, j, kb*32 + l)
 // of grid g at step s, as k_step_col does.
 template <bool GEOM, bool ADE>
-__device__ void batch_column(const SfGridDev& g, long long s, int chunk, int j, int kb,
+__device__ void batch_column(const SfGridDev& g, long long s, int i0, int i1, int j, int kb,
                              bool trial) {
     const int k = kb * 32 + (threadIdx.x & 31);
     const int nx = g.nx, ny = g.ny, nz = g.nz;
     if (k >= nz || j >= ny) return;
-    const int i0 = chunk * g.ich;
-    const int i1 = min(i0 + g.ich, nx);
     const int in = (int)((g.cur0 + s) & 1);
     const float* __restrict__ P = g.f[in][0];
     const float* __restrict__ VX = g.f[in][1];
@@ -214,34 +213,61 @@ __device__ void batch_column(const SfGridDev& g, long long s, int chunk, int j, 
     }
 }
 
-// Does the tile (with a one-cell margin, for the neighbours' faces) reach
-// the grid's material box?  Outside it every ADE term is absent, so such
-// tiles go to the plain kernel.
-__host__ __device__ __forceinline__ bool tile_meets_box(const SfGridDev& g, int chunk, int jb,
-                                                        int kb) {
-    const int by = g.jspan;
-    const int i0 = chunk * g.ich - 1, i1 = chunk * g.ich + g.ich + 1;
-    const int j0 = jb * by - 1, j1 = jb * by + by + 1;
-    const int k0 = kb * 32 - 1, k1 = kb * 32 + 33;
-    return i1 > g.ade_lo[0] && i0 < g.ade_hi[0] && j1 > g.ade_lo[1] && j0 < g.ade_hi[1] &&
-           k1 > g.ade_lo[2] && k0 < g.ade_hi[2];
+// Do the cells i0..i1-1, j0..j1-1 of k block kb (with a one-cell margin, for
+// the neighbours' faces) reach the grid's material box?  Outside it every ADE
+// term is absent.
+bool meets_box(const SfGridDev& g, int i0, int i1, int j0, int j1, int kb) {
+    return i1 + 1 > g.ade_lo[0] && i0 - 1 < g.ade_hi[0] && j1 + 1 > g.ade_lo[1] &&
+           j0 - 1 < g.ade_hi[1] && kb * 32 + 33 > g.ade_lo[2] && kb * 32 - 1 < g.ade_hi[2];
+}
+
+// A tile that reaches the material box is cut into column items of one row and
+// at most kColumnPlanes planes, each marked as ADE or plain: (grid, first plane
+// | planes << 16 | plain << 24, row, k block).
+constexpr int kColumnPlanes = 4;
+constexpr int kColumnPlain = 1 << 24;
+
+// The column items, one warp each.  A warp walks its column plane after plane,
+// each a chain of dependent loads, so the length of an item bounds the step: as
+// items of the persistent kernel as large as a tile (16 planes x 4 rows), 16
+// grids of 27.6 M cells took 0.41 ms a step and 5 of 3.7 M cells 0.27; in items
+// of 4 planes, in a kernel beside the persistent one (whose registers they
+// raised until it spilled), 0.21 and 0.07.
+__global__ void __launch_bounds__(128) k_batch_ade(const SfGridDev* __restrict__ grids,
+                                                   const int4* __restrict__ items, int n_items,
+                                                   const long long* __restrict__ step_ptr, int trial) {
+    const int it = blockIdx.x * 4 + threadIdx.y;
+    if (it >= n_items) return;
+    const int4 T = items[it];
+    const SfGridDev& g = grids[T.x];
+    const long long s = *step_ptr;
+    if (s >= g.n_steps) return;
+    const int i0 = T.y & 0xffff, i1 = i0 + (T.y >> 16 & 0xff);
+    const bool ade = !(T.y & kColumnPlain);
+    if (g.flags != nullptr) {
+        if (ade) batch_column<true, true>(g, s, i0, i1, T.z, T.w, trial != 0);
+        else batch_column<true, false>(g, s, i0, i1, T.z, T.w, trial != 0);
+    } else {
+        if (ade) batch_column<false, true>(g, s, i0, i1, T.z, T.w, trial != 0);
+        else batch_column<false, false>(g, s, i0, i1, T.z, T.w, trial != 0);
+    }
 }
 
 // Persistent warp loop over the step's work items (grid, i-chunk, row block,
 // k block).  Every warp claims items on its own -- one atomic per item, no
 // block barrier -- so items of all sizes and kinds balance across the SMs.
-// Items that meet a grid's material box come first in the list and run the
-// ADE column path; the others run the batch's plain path: thread columns
-// (KIND 0) or warp tiles (sf_tile.cuh; KIND 1, and 2 with the next plane
-// loaded ahead; 3 the same with fewer registers and more resident warps),
-// float4 tiles where the grid's fields allow them.  The grid
-// descriptor is read in place (global memory, L1-resident while a warp
-// works through its items).
+// They run the batch's plain path: thread columns (KIND 0) or warp tiles
+// (sf_tile.cuh; KIND 1, and 2 with the next plane loaded ahead; 3 the same with
+// fewer registers and more resident warps), float4 tiles where the grid's
+// fields allow them.  The grid descriptor is read in place (global memory,
+// L1-resident while a warp works through its items).
 template <int W, int MINB, int KIND>
 __global__ void __launch_bounds__(32 * W, MINB) k_batch_warp(
-    const SfGridDev* __restrict__ grids, const int4* __restrict__ items, int n_items, int n_ade,
-    int* __restrict__ queue, const long long* __restrict__ step_ptr, int trial) {
-    constexpr bool PF = KIND >= 2;
+    const SfGridDev* __restrict__ grids, const int4* __restrict__ items, int n_items,
+    int* __restrict__ queue, const long long* __restrict__ step_ptr) {
+    // loading the next plane ahead pays on scalar tiles; on float4 ones it takes
+    // registers that the walls' masks need
+    constexpr bool PF = KIND >= 2, PF4 = KIND == 3;
     const int lane = threadIdx.x;
     const long long s = *step_ptr;
     for (;;) {
@@ -249,37 +275,23 @@ __global__ void __launch_bounds__(32 * W, MINB) k_batch_warp(
         if (lane == 0) {
             it = atomicAdd(queue, 1);
             // members are listed longest run first, so a finished member's
-            // item is followed by finished members' items only: skip to the
-            // plain items, or stop after them
-            if (it < n_items && s >= grids[items[it].x].n_steps) {
-                if (it < n_ade) {
-                    atomicMax(queue, n_ade);
-                    it = -1;
-                } else {
-                    it = n_items;
-                }
-            }
+            // item is followed by finished members' items only: stop there
+            if (it < n_items && s >= grids[items[it].x].n_steps) it = n_items;
         }
         it = __shfl_sync(0xffffffffu, it, 0);
         if (it >= n_items) return;  // warp-uniform
-        if (it < 0) continue;
         const int4 T = items[it];   // grid, i-chunk, row block, k block
         const SfGridDev& g = grids[T.x];
         if (s >= g.n_steps) continue;
         const bool geom = g.flags != nullptr;
         const int j0 = T.z * g.jspan;
-        if (it < n_ade || KIND == 0) {
+        if (KIND == 0) {
             const int j_end = min(j0 + g.jspan, g.ny);
-            const bool ade = it < n_ade;
+            const int c0 = T.y * g.ich, c1 = min(c0 + g.ich, g.nx);
 #pragma unroll 1
             for (int j = j0; j < j_end; ++j) {
-                if (geom) {
-                    if (ade) batch_column<true, true>(g, s, T.y, j, T.w, trial != 0);
-                    else batch_column<true, false>(g, s, T.y, j, T.w, trial != 0);
-                } else {
-                    if (ade) batch_column<false, true>(g, s, T.y, j, T.w, trial != 0);
-                    else batch_column<false, false>(g, s, T.y, j, T.w, trial != 0);
-                }
+                if (geom) batch_column<true, false>(g, s, c0, c1, j, T.w, false);
+                else batch_column<false, false>(g, s, c0, c1, j, T.w, false);
             }
             continue;
         }
@@ -308,8 +320,8 @@ __global__ void __launch_bounds__(32 * W, MINB) k_batch_warp(
         const int i1 = min(i0 + g.ich, g.nx);
         if (g.vec4) {
             const SfPlainMem mem{io.ny * io.nz};
-            if (geom) tile4_run<true, 1, PF, false, true>(io, g.src, i0, i1, j0, T.w * 32, mem);
-            else tile4_run<false, 1, PF, false, true>(io, g.src, i0, i1, j0, T.w * 32, mem);
+            if (geom) tile4_run<true, 1, PF4, false, true>(io, g.src, i0, i1, j0, T.w * 32, mem);
+            else tile4_run<false, 1, PF4, false, true>(io, g.src, i0, i1, j0, T.w * 32, mem);
         } else {
             const int k = T.w * 32 + lane;
             if (geom) tile1_run<true, 2, PF>(io, g.src, i0, i1, j0, k);
@@ -467,9 +479,9 @@ struct sf_batch {
     int device = 0;
     bool built = false;
     SfGridDev* d_grids = nullptr;
-    int4* d_tiles = nullptr;  // work items: those meeting a material box first
-    int n_tiles = 0;          // all work items
-    int n_tiles_ade = 0;      // items that meet a material box
+    int4* d_tiles = nullptr;  // column items around the material boxes, plain items, nonuniform items
+    int n_tiles = 0;          // column and plain items
+    int n_tiles_ade = 0;      // column items of the tiles that meet a material box
     int n_tiles_nu = 0;       // items of nonuniform members, after the others in d_tiles
     int blocks_nu = 0;        // persistent grid size of k_batch_warp_nu
     int* d_ade_ids = nullptr;
@@ -506,8 +518,10 @@ void free_device(sf_batch* B) {
 
 int chunk_for_grid(const sf_batch* B, const sf_plan* P) {
     if (B->i_chunk > 0) return B->i_chunk;
-    // about 16 planes per tile, fewer for thin grids
-    return P->d.nx < 32 ? (P->d.nx + 1) / 2 : 16;
+    // 8 planes per tile, fewer for thin grids (with the column items apart, 8
+    // against 16 planes: 24 grids of 49.5 M cells 0.336 against 0.335 ms a step,
+    // 10 of 8.9 M 0.090 against 0.097, 5 of 3.7 M 0.060 against 0.066)
+    return P->d.nx < 16 ? (P->d.nx + 1) / 2 : 8;
 }
 
 template <typename K>
@@ -619,15 +633,24 @@ int build(sf_batch* B) {
         for (int ch = 0; ch < nch; ++ch)
             for (int jb = 0; jb < njb; ++jb)
                 for (int kb = 0; kb < nkb; ++kb) {
-                    const bool ade = g.poles.n > 0 && tile_meets_box(g, ch, jb, kb);
-                    if (g.nu_cv[0] != nullptr) tiles_nu.push_back(make_int4(gi, ch, jb, kb));
-                    else (ade ? tiles_ade : tiles).push_back(make_int4(gi, ch, jb, kb));
+                    const int i0 = ch * g.ich, i1 = std::min(i0 + g.ich, g.nx);
+                    const int j0 = jb * g.jspan, j1 = std::min(j0 + g.jspan, g.ny);
+                    if (g.nu_cv[0] != nullptr) {
+                        tiles_nu.push_back(make_int4(gi, ch, jb, kb));
+                    } else if (g.poles.n == 0 || !meets_box(g, i0, i1, j0, j1, kb)) {
+                        tiles.push_back(make_int4(gi, ch, jb, kb));
+                    } else {
+                        for (int i = i0; i < i1; i += kColumnPlanes)
+                            for (int j = j0; j < j1; ++j) {
+                                const int n = std::min(kColumnPlanes, i1 - i);
+                                const int plain = meets_box(g, i, i + n, j, j + 1, kb) ? 0 : kColumnPlain;
+                                tiles_ade.push_back(make_int4(gi, i | n << 16 | plain, j, kb));
+                            }
+                    }
                 }
     }
     if (tiles.size() + tiles_ade.size() + tiles_nu.size() > 0x7fffffff)
         return sf_fail("sf_batch: too many tiles");
-    // items meeting a material box first: they are the slowest, so they
-    // start early and the step ends on short plain items
     B->n_tiles_ade = (int)tiles_ade.size();
     tiles_ade.insert(tiles_ade.end(), tiles.begin(), tiles.end());
     tiles.swap(tiles_ade);
@@ -659,35 +682,75 @@ int build(sf_batch* B) {
 
 int launch_step_kernel(sf_batch* B, cudaStream_t st, int trial) {
     constexpr int W = kBatchWarps;
+    const int4* plain = B->d_tiles + B->n_tiles_ade;
+    const int n_plain = B->n_tiles - B->n_tiles_ade;
     if (B->n_tiles_nu > 0 && !trial) {  // nonuniform members: their own persistent kernel
         const int blocks = std::min(B->blocks_nu, (B->n_tiles_nu + W - 1) / W);
         k_batch_warp_nu<W, kMinBlocksTile><<<blocks, dim3(32, W), 0, st>>>(
             B->d_grids, B->d_tiles + B->n_tiles, B->n_tiles_nu, B->d_queue + 1, B->d_step);
         if (cudaGetLastError() != cudaSuccess) return sf_fail("k_batch_warp_nu launch failed");
     }
-    if (B->n_tiles == 0) return 0;
+    if (n_plain == 0) return 0;
     const dim3 blk(32, W);
     if (B->plain_kernel == 1)
         k_batch_warp<W, kMinBlocksTile, 1><<<B->blocks, blk, 0, st>>>(
-            B->d_grids, B->d_tiles, B->n_tiles, B->n_tiles_ade, B->d_queue, B->d_step, trial);
+            B->d_grids, plain, n_plain, B->d_queue, B->d_step);
     else if (B->plain_kernel == 2)
         k_batch_warp<W, kMinBlocksTile, 2><<<B->blocks, blk, 0, st>>>(
-            B->d_grids, B->d_tiles, B->n_tiles, B->n_tiles_ade, B->d_queue, B->d_step, trial);
+            B->d_grids, plain, n_plain, B->d_queue, B->d_step);
     else if (B->plain_kernel == 3)
         k_batch_warp<W, kMinBlocksLean, 3><<<B->blocks, blk, 0, st>>>(
-            B->d_grids, B->d_tiles, B->n_tiles, B->n_tiles_ade, B->d_queue, B->d_step, trial);
+            B->d_grids, plain, n_plain, B->d_queue, B->d_step);
     else
         k_batch_warp<W, kMinBlocksColumn, 0><<<B->blocks, blk, 0, st>>>(
-            B->d_grids, B->d_tiles, B->n_tiles, B->n_tiles_ade, B->d_queue, B->d_step, trial);
+            B->d_grids, plain, n_plain, B->d_queue, B->d_step);
     return cudaGetLastError() == cudaSuccess ? 0 : sf_fail("k_batch_warp launch failed");
 }
 
-// One batch step: ADE density pass, step, probes, advance.
-int enqueue_step(sf_batch* B, cudaStream_t st) {
-    if (B->n_ade > 0)
+// The ADE part of a step: density pass, then the column items.
+int launch_ade(sf_batch* B, cudaStream_t st, int trial) {
+    if (B->n_ade > 0 && !trial)
         k_batch_ade_density<<<dim3(B->ade_blocks, B->n_ade), 256, 0, st>>>(B->d_grids, B->d_ade_ids,
                                                                            B->d_step);
+    if (B->n_tiles_ade > 0)
+        k_batch_ade<<<(B->n_tiles_ade + 3) / 4, dim3(32, 4), 0, st>>>(B->d_grids, B->d_tiles, B->n_tiles_ade,
+                                                                    B->d_step, trial);
+    return cudaGetLastError() == cudaSuccess ? 0 : sf_fail("k_batch_ade launch failed");
+}
+
+// A second stream for the ADE part, which runs beside the plain items (the two
+// read the same input set and write disjoint cells).
+struct SideBranch {
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+    int open() {
+        SF_CUDA_OK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+        SF_CUDA_OK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+        SF_CUDA_OK(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
+        return 0;
+    }
+    ~SideBranch() {
+        if (fork) cudaEventDestroy(fork);
+        if (join) cudaEventDestroy(join);
+        if (side) cudaStreamDestroy(side);
+    }
+};
+
+// One batch step: ADE part (on its own branch when there is one), plain
+// items, probes, advance.
+int enqueue_step(sf_batch* B, cudaStream_t st, const SideBranch* br = nullptr) {
+    const bool ade = B->n_tiles_ade > 0;
+    if (ade && br) {
+        SF_CUDA_OK(cudaEventRecord(br->fork, st));
+        SF_CUDA_OK(cudaStreamWaitEvent(br->side, br->fork, 0));
+    }
+    if (ade)
+        if (int rc = launch_ade(B, br ? br->side : st, 0)) return rc;
     if (int rc = launch_step_kernel(B, st, 0)) return rc;
+    if (ade && br) {
+        SF_CUDA_OK(cudaEventRecord(br->join, br->side));
+        SF_CUDA_OK(cudaStreamWaitEvent(st, br->join, 0));
+    }
     k_batch_post<<<(int)B->members.size(), 64, 0, st>>>(B->d_grids, B->d_step);
     k_batch_advance<<<1, 1, 0, st>>>(B->d_step, B->d_queue);
     return cudaGetLastError() == cudaSuccess ? 0 : sf_fail("sf_batch: launch failed");
@@ -775,6 +838,12 @@ int sf_batch_run(sf_batch* B, int64_t n_steps, int graph_steps, void* stream) {
     if (n_steps <= 0) return 0;
     SF_CUDA_OK(cudaMemsetAsync(B->d_step, 0, sizeof(long long), st));
     SF_CUDA_OK(cudaMemsetAsync(B->d_queue, 0, 2 * sizeof(int), st));
+    SideBranch branch;
+    const SideBranch* ade = nullptr;
+    if (B->n_tiles_ade > 0) {
+        if (int rc = branch.open()) return rc;
+        ade = &branch;
+    }
     int64_t done = 0;
     if (graph_steps > 0 && n_steps >= graph_steps) {
         if (!B->graph_exec || B->graph_steps != graph_steps) {
@@ -788,7 +857,7 @@ int sf_batch_run(sf_batch* B, int64_t n_steps, int graph_steps, void* stream) {
             if (cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
                 rc = sf_fail("sf_batch_run: stream capture failed to begin");
             } else {
-                for (int q = 0; q < graph_steps && !rc; ++q) rc = enqueue_step(B, cap);
+                for (int q = 0; q < graph_steps && !rc; ++q) rc = enqueue_step(B, cap, ade);
                 if (cudaStreamEndCapture(cap, &B->graph) != cudaSuccess && !rc)
                     rc = sf_fail("sf_batch_run: stream capture failed");
             }
@@ -803,7 +872,7 @@ int sf_batch_run(sf_batch* B, int64_t n_steps, int graph_steps, void* stream) {
         }
     }
     for (; done < n_steps; ++done)
-        if (int rc = enqueue_step(B, st)) return rc;
+        if (int rc = enqueue_step(B, st, ade)) return rc;
     // the members' current sets and step counts move with the batch
     for (auto& m : B->members) {
         const long long ran = std::min<long long>(m.steps, n_steps);
@@ -846,7 +915,8 @@ int sf_batch_autotune(sf_batch* B, int launches, void* stream, float* ms_out, in
             for (int q = 0; q <= launches && !rc; ++q) {
                 if (q == 1) cudaEventRecord(e0, st);
                 cudaMemsetAsync(B->d_queue, 0, 2 * sizeof(int), st);
-                rc = launch_step_kernel(B, st, 1);
+                rc = launch_ade(B, st, 1);
+                if (!rc) rc = launch_step_kernel(B, st, 1);
             }
             if (rc) break;
             cudaEventRecord(e1, st);
