@@ -135,6 +135,8 @@ constexpr long long kResPolls = 1LL << 23;  // polls (about 0.5 us each) before 
 struct ResDevice {
     char* mail = nullptr;
     size_t bytes = 0;
+    float* corners = nullptr;  // microphone corners of one launch (at most 8 MB)
+    size_t corner_bytes = 0;
     unsigned tag = 1;
     cudaEvent_t done = nullptr;
     int* err_host = nullptr;
@@ -201,6 +203,9 @@ void resident_release() {
         cudaFree(D.mail);
         D.mail = nullptr;
         D.bytes = 0;
+        cudaFree(D.corners);
+        D.corners = nullptr;
+        D.corner_bytes = 0;
     }
 }
 }  // namespace
@@ -361,6 +366,7 @@ int sf_plan_set_pml(sf_plan* P, const float* sx, const float* sy, const float* s
 
 int sf_plan_set_nonuniform(sf_plan* P, const float* const* cv_face, const float* const* inv_cell) {
     if (!P) return sf_fail("sf_plan_set_nonuniform: NULL plan");
+    ++P->tables;
     DeviceGuard g(P->device);
     cudaFree(P->nu);
     P->nu = nullptr;
@@ -392,6 +398,16 @@ int sf_plan_set_weighted_source(sf_plan* P, int slot, int64_t n, const int64_t* 
     for (int64_t q = 0; q < n; ++q)
         if (cells[q] < 0 || cells[q] >= P->n)
             return sf_fail("sf_plan_set_weighted_source: cell outside the grid");
+    ++P->tables;
+    int* box = P->wsrc_box[slot];
+    for (int64_t q = 0; q < n; ++q) {
+        const long long plane = (long long)P->d.ny * P->d.nz, r = cells[q] % plane;
+        const int at[3] = {(int)(cells[q] / plane), (int)(r / P->d.nz), (int)(r % P->d.nz)};
+        for (int a = 0; a < 3; ++a) {
+            box[a] = q == 0 ? at[a] : std::min(box[a], at[a]);
+            box[3 + a] = q == 0 ? at[a] + 1 : std::max(box[3 + a], at[a] + 1);
+        }
+    }
     DeviceGuard g(P->device);
     cudaFree(P->wsrc_cells[slot]);
     cudaFree(P->wsrc_w[slot]);
@@ -409,6 +425,7 @@ int sf_plan_set_weighted_source(sf_plan* P, int slot, int64_t n, const int64_t* 
 
 int sf_plan_set_plane_boundaries(sf_plan* P, int n, const sf_plane_bc* ops) {
     if (!P) return sf_fail("sf_plan_set_plane_boundaries: NULL plan");
+    ++P->tables;
     if (n < 0 || n > SF_MAX_PLANE_OPS || (n > 0 && !ops))
         return sf_fail("sf_plan_set_plane_boundaries: at most 8 operations");
     const int dims[3] = {P->d.nx, P->d.ny, P->d.nz};
@@ -453,6 +470,7 @@ int sf_plan_set_pml_decay(sf_plan* P, const float* dx, const float* dy, const fl
 
 int sf_plan_set_sources(sf_plan* P, int n, const sf_source* s) {
     if (!P) return sf_fail("sf_plan_set_sources: NULL plan");
+    ++P->tables;
     if (n < 0 || n > SF_MAX_SOURCES) return sf_fail("sf_plan_set_sources: at most 16 sources");
     if (n > 0 && !s) return sf_fail("sf_plan_set_sources: NULL source table");
     const int dims[3] = {P->d.nx, P->d.ny, P->d.nz};
@@ -478,6 +496,7 @@ int sf_plan_set_sources(sf_plan* P, int n, const sf_source* s) {
 
 int sf_plan_set_probes(sf_plan* P, int n, const int64_t* cells) {
     if (!P) return sf_fail("sf_plan_set_probes: NULL plan");
+    ++P->tables;
     if (n < 0 || (n > 0 && !cells)) return sf_fail("sf_plan_set_probes: bad probe table");
     for (int q = 0; q < n; ++q)
         if (cells[q] < 0 || cells[q] >= P->n) return sf_fail("sf_plan_set_probes: cell outside the grid");
@@ -968,28 +987,67 @@ int pipe_check(sf_plan* P, cudaStream_t st) {
     return sf_fail("k_step_pipe: a dependency wait expired (results of this call are invalid)");
 }
 
+// What acts between this plan's steps, for the state-on-chip kernel; false when
+// that kernel cannot do it (a source weighted on a velocity, too many rows).
+bool resident_extra(const sf_plan* P, bool mics, SfResExtra& x) {
+    x = SfResExtra{};
+    x.n_plane = P->n_plane;
+    for (int q = 0; q < P->n_plane; ++q) {
+        x.ops[q] = P->plane_ops[q];
+        for (int side = 0; side < 2; ++side) x.prev[q][side] = P->plane_prev + P->plane_off[q][side];
+    }
+    for (int q = 0; q < P->src.n; ++q) {
+        const sf_source& S = P->src.s[q];
+        if (S.kind != 2) continue;
+        if (S.b != 0 || P->wsrc_n[S.a] > INT_MAX) return false;
+        x.wcells[q] = P->wsrc_cells[S.a];
+        x.ww[q] = P->wsrc_w[S.a];
+        x.wn[q] = (int)P->wsrc_n[S.a];
+        if (x.wn[q] == 0) continue;
+        for (int a = 0; a < 3; ++a) {
+            const int* box = P->wsrc_box[S.a];
+            x.wbox[a] = x.w_slots ? std::min(x.wbox[a], box[a]) : box[a];
+            x.wbox[3 + a] = x.w_slots ? std::max(x.wbox[3 + a], box[3 + a]) : box[3 + a];
+        }
+        ++x.w_slots;
+    }
+    if (mics) {
+        if (P->n_mic > 64) return false;
+        x.n_mic = P->n_mic;
+        x.mic_field = P->mic_field;
+        x.mic_idx = P->mic_idx;
+    }
+    return true;
+}
+
 // Whether n steps of this plan run on the state-on-chip path: automatic
-// kernel choice, nothing between the steps but probes, no ADE poles, a grid
-// whose blocks fit on the SMs, enough steps to pay for loading the state, and
-// no stream capture (a captured launch would keep its message tags).
+// kernel choice, no ADE poles, a grid whose blocks fit on the SMs, enough steps
+// to pay for loading the state, and no stream capture (a captured launch would
+// keep its message tags).
 bool resident_fits(sf_plan* P, const SfStepArgs& a, int64_t n_steps, bool deferred, bool mics,
                    cudaStream_t st) {
-    if (P->variant != SF_CFG_AUTO || P->i_chunk != 0 || P->poles.n > 0 || deferred || mics ||
-        n_steps < kResMinSteps || P->n_probe > 1024 || stream_capturing(st))
+    if (P->variant != SF_CFG_AUTO || P->i_chunk != 0 || P->poles.n > 0 || n_steps < kResMinSteps ||
+        P->n_probe > 1024 || stream_capturing(st))
         return false;
-    const int key[2] = {a.n_probe, P->nu != nullptr};
-    if (P->res_key[0] != key[0] || P->res_key[1] != key[1]) {
-        P->res_cut = sf_resident_cut(P->d.nx, P->d.ny, P->d.nz, a.n_probe, P->nu != nullptr, P->sms);
-        P->res_key[0] = key[0];
-        P->res_key[1] = key[1];
+    const long long key = P->tables * 4 + (mics ? 2 : 0) + (a.n_probe > 0 ? 1 : 0);
+    if (P->res_key != key) {
+        SfResExtra x;
+        const bool extra = deferred || mics;
+        P->res_cut.kind = -1;
+        if (!extra || resident_extra(P, mics, x))
+            P->res_cut = sf_resident_cut(P->d.nx, P->d.ny, P->d.nz, a.n_probe, P->nu != nullptr, P->sms,
+                                         extra ? &x : nullptr);
+        P->res_key = key;
     }
     return P->res_cut.kind >= 0 && resident_slot(P);
 }
 
 // n steps of the plan from its current set, in launches of at most kResChunk.
 int step_resident(sf_plan* P, const SfStepArgs& a0, int64_t n_steps, const double* src_values,
-                  float* trace, cudaStream_t st) {
+                  float* trace, float* mic_trace, cudaStream_t st) {
     const SfResCut& c = P->res_cut;
+    SfResExtra x{};
+    if (c.extra) resident_extra(P, mic_trace != nullptr, x);
     const size_t mail = (size_t)2 * c.bi * c.bj * c.bk * 6 * c.side_max * 4 * sizeof(unsigned long long);
     if (mail > kResMailMax) return sf_fail("k_resident: mailboxes too large");
     std::lock_guard<std::mutex> lock(g_res_mu);
@@ -1002,6 +1060,17 @@ int step_resident(sf_plan* P, const SfStepArgs& a0, int64_t n_steps, const doubl
         SF_CUDA_OK(cudaMalloc(&D.mail, mail));
         D.bytes = mail;
         D.tag = 0xffffffffu;  // cleared below
+    }
+    if (x.n_mic > 0) {
+        const size_t need = sizeof(float) * 8 * x.n_mic * (size_t)std::min<int64_t>(kResChunk, n_steps);
+        if (D.corner_bytes < need) {
+            cudaFree(D.corners);
+            D.corners = nullptr;
+            D.corner_bytes = 0;
+            SF_CUDA_OK(cudaMalloc(&D.corners, need));
+            D.corner_bytes = need;
+        }
+        x.corners = D.corners;
     }
     for (int64_t s = 0; s < n_steps;) {
         const int n = (int)std::min<int64_t>(kResChunk, n_steps - s);
@@ -1025,7 +1094,11 @@ int step_resident(sf_plan* P, const SfStepArgs& a0, int64_t n_steps, const doubl
         A.err = P->res_err_dev;
         A.poll_limit = P->pipe_spin_limit > 0 ? P->pipe_spin_limit : kResPolls;
         A.hold = P->pipe_hold ? 1 : 0;
+        A.x = x;
         if (int rc = sf_launch_resident(A, P->src, c, st)) return rc;
+        if (x.n_mic > 0)
+            if (int rc = sf_launch_resident_mics(x.corners, P->mic_w, x.n_mic, n, mic_trace + s * x.n_mic, st))
+                return rc;
         D.tag += (unsigned)n;
         P->cur = out;
         P->steps_done += n;
@@ -1083,7 +1156,7 @@ int sf_plan_step_ex(sf_plan* P, int64_t n_steps, const double* src_values, float
     // plane boundaries or weighted sources: sources move after the fused kernel
     const bool deferred = defers(P);
     if (resident_fits(P, a, n_steps, deferred, mics, st))
-        return step_resident(P, a, n_steps, src_values, trace, st);
+        return step_resident(P, a, n_steps, src_values, trace, mics ? mic_trace : nullptr, st);
     const int cfg0 = effective_config(P, a);
     // A pipeline configuration runs whole groups of its steps per launch when
     // nothing has to happen between steps; remaining steps (and plans with
@@ -1178,6 +1251,7 @@ int sf_plan_set_microphones(sf_plan* P, int n, const int64_t* idx8, const float*
 int sf_plan_set_microphones_ex(sf_plan* P, int n, const int32_t* field, const int64_t* idx8,
                                const float* w8) {
     if (!P) return sf_fail("sf_plan_set_microphones: NULL plan");
+    ++P->tables;
     if (n < 0 || (n > 0 && (!idx8 || !w8))) return sf_fail("sf_plan_set_microphones: bad table");
     if (field)
         for (int q = 0; q < n; ++q)

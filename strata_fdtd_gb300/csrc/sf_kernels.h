@@ -101,16 +101,36 @@ int sf_launch_step_tb(const SfStepArgs& a, const SfSources& src, bool geom, int 
 // Shared memory of a block: offsets in floats (multiples of 4).
 struct SfResLayout {
     int src;             // this step's source values (doubles)
-    int ctl;             // [1] probes, [2] a wait expired
+    int ctl;             // [0] weighted cells, [1] probes, [2] a wait expired, [3] microphone corners
     int side;            // (decay, coefficient) of each side's faces
     int P, UX, UY, UZ;   // pressures; x faces at chunk ends, y faces, z faces
     int dx, dy, dz;      // PML decays of the block's planes, rows, cells
     int cx, cy, cz, sx, sy, sz;  // NU: face coefficients, cell scales
     int probe;           // (trace column, cell in P)
+    int prev[SF_MAX_PLANE_OPS][2];  // plane boundaries: stored planes, low and high
+    int wlist;           // weighted sources: (cell in P, source, weight) entries
+    int mic;             // microphone corners (int4)
     int end;
+};
+// What acts between the steps: pressure-plane boundaries, weighted sources on
+// the pressure, microphone corners.
+struct SfResExtra {
+    int n_plane;
+    sf_plane_bc ops[SF_MAX_PLANE_OPS];
+    float* prev[SF_MAX_PLANE_OPS][2];
+    const long long* wcells[SF_MAX_SOURCES];  // by source
+    const double* ww[SF_MAX_SOURCES];
+    int wn[SF_MAX_SOURCES];
+    int wbox[6];       // cells lo, hi (exclusive) per axis of all weighted sources, empty: none
+    int w_slots;       // how many sources are weighted
+    int n_mic;         // microphone rows
+    const int* mic_field;
+    const long long* mic_idx;
+    float* corners;    // [step][row][8]
 };
 struct SfResCut {
     int kind;          // planes per thread and thread counts (kKinds), < 0: does not fit
+    bool extra;        // for a plan with something between the steps
     int bi, bj, bk;    // blocks along x, y, z
     int chunks, quads; // chunks of planes and quads of k cells in the grid
     int threads;
@@ -129,8 +149,11 @@ struct SfResArgs {
     int* err;          // set when a wait expired
     long long poll_limit;
     int hold;          // expiry test hook: block 0 waits for tags nothing sends
+    SfResExtra x;
 };
-SfResCut sf_resident_cut(int nx, int ny, int nz, int n_probe, bool nu, int sms);
+SfResCut sf_resident_cut(int nx, int ny, int nz, int n_probe, bool nu, int sms, const SfResExtra* x);
+int sf_launch_resident_mics(const float* corners, const float* w, int n_mic, long long n_steps,
+                            float* mic_trace, cudaStream_t st);
 int sf_launch_resident(SfResArgs& A, const SfSources& src, const SfResCut& c, cudaStream_t st);
 
 int sf_launch_build_flags(const uint8_t* geom, uint8_t* flags, int nx, int ny, int nz,

@@ -41,6 +41,8 @@ struct sf_plan {
     long long* wsrc_cells[SF_MAX_SOURCES] = {nullptr};  // owned, weighted (membrane) sources
     double* wsrc_w[SF_MAX_SOURCES] = {nullptr};
     long long wsrc_n[SF_MAX_SOURCES] = {0};
+    int wsrc_box[SF_MAX_SOURCES][6];    // cells lo, hi (exclusive) per axis
+    long long tables = 0;               // bumped by the setters the state-on-chip cut depends on
     // multi-step pipeline (sf_step_pipe.cu)
     float* pipe_ring = nullptr;  // owned: rings of planes between levels
     size_t pipe_ring_floats = 0;
@@ -55,8 +57,8 @@ struct sf_plan {
     int pipe_grid[2] = {0, 0};       // configuration + 1, resident blocks
     int probe_tile_max = 0;          // most probes in one 32 k x 4 row tile column
     // state-on-chip path (sf_step_resident.cu)
-    SfResCut res_cut{};              // of the probe count and spacing in res_key
-    int res_key[2] = {-1, -1};
+    SfResCut res_cut{};              // of the tables as of res_key
+    long long res_key = -1;          // bumped with everything the cut depends on
     int* res_err = nullptr;          // host-mapped word, set when a wait expired
     int* res_err_dev = nullptr;      // its device address
     int res_slot = -1;

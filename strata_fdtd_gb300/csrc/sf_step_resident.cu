@@ -143,7 +143,12 @@ __host__ __device__ constexpr int z_row(int L, int nq) { return z_shared(L) ? 4 
 __host__ __device__ constexpr int z_low(int L) { return z_shared(L) ? 3 : 0; }
 __host__ __device__ constexpr int z_high(int L, int nq) { return z_shared(L) ? 4 * nq + 3 : nq; }
 
-inline Layout layout(int L, int nci, int nj, int nq, int n_probe, bool nu) {
+// Cells of a block's share of the plane perpendicular to an axis
+__host__ __device__ inline int plane_cells(int axis, int planes, int nj, int row) {
+    return axis == 0 ? nj * row : (axis == 1 ? planes * row : planes * nj);
+}
+
+inline Layout layout(int L, int nci, int nj, int nq, int n_probe, bool nu, const SfResExtra* x) {
     const int planes = nci * L;
     Layout l;
     int o = 0;
@@ -172,6 +177,21 @@ inline Layout layout(int L, int nci, int nj, int nq, int n_probe, bool nu) {
         l.sz = take(nq * 4);
     }
     l.probe = take(n_probe * 2);
+    for (int q = 0; q < SF_MAX_PLANE_OPS; ++q)
+        for (int side = 0; side < 2; ++side)
+            l.prev[q][side] =
+                x && q < x->n_plane ? take(plane_cells(x->ops[q].axis, planes, nj, nq * 4)) : 0;
+    long long wcap = 0;  // entries a block can have: its overlap with the sources' box
+    if (x && x->w_slots > 0) {
+        const int dims[3] = {planes, nj, nq * 4};
+        wcap = x->w_slots;
+        for (int a = 0; a < 3; ++a) {
+            const int e = x->wbox[3 + a] - x->wbox[a];
+            wcap *= e < dims[a] ? e : dims[a];
+        }
+    }
+    l.wlist = wcap > 16000 ? (o = 1 << 28) : take((int)wcap * 4);
+    l.mic = take(x ? x->n_mic * 8 * 4 : 0);
     l.end = o;
     return l;
 }
@@ -393,6 +413,84 @@ __device__ __forceinline__ void phase_p(const SfStepArgs& a, const Layout& S, co
     }
 }
 
+// ---- between the steps --------------------------------------------------------
+
+// One plane boundary over the block's share of its planes (k_plane_bc's
+// arithmetic: the low end, then the high one).
+__device__ __forceinline__ void plane_op(const SfStepArgs& a, const Layout& S, const Place& g,
+                                         const sf_plane_bc& op, const int (&prev)[2]) {
+    const int ax = op.axis;
+    const bool lo = !g.b.lo[ax] && (op.kind == 0 || op.side == 0);
+    const bool hi = !g.b.hi[ax] && (op.kind == 0 || op.side == 1);
+    if (!lo && !hi) return;
+    const int cnt = plane_cells(ax, g.planes, g.b.nj, g.row);
+    const int n = ax == 0 ? a.nx - g.gi0 : (ax == 1 ? g.b.nj : a.nz - g.gk0);  // cells up to the grid's end
+    const int stride = ax == 0 ? g.plane : (ax == 1 ? g.row : 1);
+    for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
+        int base;  // the plane's cell at position 0 along the axis
+        if (ax == 0) {
+            if (g.gk0 + t % g.row >= a.nz) continue;
+            base = t;
+        } else if (ax == 1) {
+            const int i = t / g.row;
+            if (g.gi0 + i >= a.nx || g.gk0 + t % g.row >= a.nz) continue;
+            base = i * g.plane + t % g.row;
+        } else {
+            const int i = t / g.b.nj;
+            if (g.gi0 + i >= a.nx) continue;
+            base = i * g.plane + t % g.b.nj * g.row;
+        }
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+            if (!(side ? hi : lo)) continue;
+            float& pb = smem[S.P + base + (side ? n - 1 : 0) * stride];
+            const float pi = smem[S.P + base + (side ? n - 2 : 1) * stride];
+            float& was = smem[prev[side] + t];
+            const double abc = d_add((double)was, d_mul(op.coeff, (double)f_sub(pi, pb)));
+            if (op.kind == 0) {
+                pb = __double2float_rn(abc);
+            } else {
+                const float rig = f_mul(__double2float_rn(op.reflection), pi);
+                pb = __double2float_rn(d_add((double)rig, d_mul(d_sub(1.0, op.reflection), abc)));
+            }
+            was = pi;
+        }
+    }
+}
+
+// The stored planes between global memory (t over the grid's plane) and the block.
+__device__ __forceinline__ void move_prev(const SfStepArgs& a, const SfResExtra& x, const Layout& S,
+                                          const Place& g, bool store) {
+    for (int q = 0; q < x.n_plane; ++q) {
+        const sf_plane_bc& op = x.ops[q];
+        const int ax = op.axis, nv = ax == 2 ? a.ny : a.nz;
+        const int cnt = plane_cells(ax, g.planes, g.b.nj, g.row);
+        for (int side = 0; side < 2; ++side) {
+            if (side ? g.b.hi[ax] : g.b.lo[ax]) continue;
+            if (op.kind == 1 && op.side != side) continue;
+            float* f = op.kind == 1 ? x.prev[q][0] : x.prev[q][side];
+            for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
+                const int per = ax == 2 ? g.b.nj : g.row;
+                const int u = (ax == 0 ? g.b.j0 : g.gi0) + t / per, v = (ax == 2 ? g.b.j0 : g.gk0) + t % per;
+                if (u >= (ax == 0 ? a.ny : a.nx) || v >= nv) continue;
+                float& here = smem[S.prev[q][side] + t];
+                float& there = f[(long long)u * nv + v];
+                if (store) there = here;
+                else here = there;
+            }
+        }
+    }
+}
+
+// The place of cell c in the block's P, or -1 outside the block.
+__device__ __forceinline__ int place_of(const SfStepArgs& a, const Place& g, long long c) {
+    const int i = (int)(c / a.plane), r = (int)(c % a.plane), j = r / a.nz, k = r % a.nz;
+    if (i < g.gi0 || i >= g.gi0 + g.planes || j < g.b.j0 || j >= g.b.j0 + g.b.nj || k < g.gk0 ||
+        k >= g.gk0 + g.row)
+        return -1;
+    return (i - g.gi0) * g.plane + (j - g.b.j0) * g.row + (k - g.gk0);
+}
+
 // The sources that reach this thread's cells, in order, after the decays.
 template <int L>
 __device__ void add_sources(const SfSources& src, const Layout& S, const Tile& T, int i0, int k0,
@@ -538,7 +636,9 @@ __device__ __forceinline__ Unit make_unit(const SfResArgs& A, const Place& g, in
                 (to * 6 + (side ^ 1)) * words + u * 4, ((int)blockIdx.x * 6 + side) * words + u * 4};
 }
 
-template <int L, int MAXT, bool NU>
+// EXTRA: plane boundaries, weighted sources or microphones between the steps
+// (sources then follow the plane boundaries, as in sf_plan_step).
+template <int L, int MAXT, bool NU, bool EXTRA>
 __global__ void __launch_bounds__(MAXT, 1) k_resident(const __grid_constant__ SfResArgs A,
                                                       const __grid_constant__ SfSources src) {
     const SfStepArgs& a = A.a;
@@ -616,6 +716,46 @@ __global__ void __launch_bounds__(MAXT, 1) k_resident(const __grid_constant__ Sf
             make_int2(t, (i - gi0) * plane + (jj - b.j0) * row + (k - gk0));
     }
 
+    // ---- what acts between the steps
+    const SfResExtra& x = A.x;
+    // microphone corners: (number, value, its decay, -1) in shared memory, or
+    // (number, field << 8 | plane << 2 | cell, its decay, thread) in a thread's registers
+    int4* mics = reinterpret_cast<int4*>(smem + S.mic);
+    int4* wlist = reinterpret_cast<int4*>(smem + S.wlist);  // (place in P, source, weight)
+    if (EXTRA) {
+        move_prev(a, x, S, g, false);
+        for (int q = 0; q < src.n; ++q)
+            if (src.s[q].kind == 2)
+                for (int t = tid; t < x.wn[q]; t += nthreads) {
+                    const int at = place_of(a, g, x.wcells[q][t]);
+                    if (at < 0) continue;
+                    const long long w = __double_as_longlong(x.ww[q][t]);
+                    wlist[atomicAdd(const_cast<int*>(ctl), 1)] = make_int4(at, q, (int)w, (int)(w >> 32));
+                }
+        for (int t = tid; t < x.n_mic * 8; t += nthreads) {
+            const int at = place_of(a, g, x.mic_idx[t]);
+            if (at < 0) continue;
+            const int i = at / plane, r = at % plane, jj = r / row, k = r % row, l = i % L;
+            const int f = x.mic_field ? x.mic_field[t / 8] : 0;
+            int4 m = make_int4(t, S.P + at, -1, -1);
+            if (f == 2) {
+                m.y = S.UY + (i * (b.nj + 1) + jj + 1) * row + k;
+                m.z = S.dy + jj;
+            } else if (f != 0) {
+                m.z = f == 1 ? S.dx + i : S.dz + k;
+                const bool slot = f == 1 ? i == planes - 1 && b.hi[0] : z_shared(L) || (k == row - 1 && b.hi[2]);
+                if (slot) {
+                    m.y = f == 1 ? S.UX + b.nci * plane + jj * row + k
+                                 : S.UZ + (i * b.nj + jj) * zr + (z_shared(L) ? 4 + k : b.nq);
+                } else {
+                    m.y = f << 8 | l << 2 | (k % 4);
+                    m.w = (i / L * b.nj + jj) * b.nq + k / 4;
+                }
+            }
+            mics[atomicAdd(const_cast<int*>(ctl) + 3, 1)] = m;
+        }
+    }
+
     // ---- this thread's cells
     const bool active = tid < b.nci * b.nj * b.nq;
     Tile T;
@@ -664,6 +804,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_resident(const __grid_constant__ Sf
         if (i0 + L >= a.nx || gj == a.ny - 1 || k0 + 4 >= a.nz) mode = 2;
         for (int s = 0; s < src.n; ++s) {
             const sf_source& Q = src.s[s];
+            if (EXTRA && Q.kind == 2) continue;
             const int at = Q.kind == 0 ? Q.a : Q.b;
             const bool in_i = at >= i0 && at < i0 + L;
             bool can;
@@ -680,6 +821,32 @@ __global__ void __launch_bounds__(MAXT, 1) k_resident(const __grid_constant__ Sf
     __syncthreads();
     const int probes = ctl[1];
     const bool has_units = U[0].d != 0;
+    const int n_w = EXTRA ? ctl[0] : 0, n_mics = EXTRA ? ctl[3] : 0;
+    bool my_mics = false;
+    for (int t = 0; t < n_mics; ++t) my_mics = my_mics || mics[t].w == tid;
+    // the state's values at the microphone corners after step s
+    auto record_mics = [&](int s) {
+        float* out = x.corners + (size_t)s * x.n_mic * 8;
+        for (int t = tid; t < n_mics; t += nthreads) {
+            const int4 m = mics[t];
+            if (m.w >= 0) continue;
+            out[m.x] = m.z < 0 ? smem[m.y] : f_mul(smem[m.y], smem[m.z]);
+        }
+        if (!my_mics) return;
+        for (int t = 0; t < n_mics; ++t) {
+            const int4 m = mics[t];
+            if (m.w != tid) continue;
+            float v = 0.0f;
+#pragma unroll
+            for (int l = 0; l < L; ++l) {
+                if (l != (m.y >> 2 & 63)) continue;
+                const Quad f = m.y >> 8 == 1 ? o.vx[l] : o.vz[z_shared(L) ? 0 : l];
+                const int e = m.y & 3;
+                v = e == 0 ? f[0] : (e == 1 ? f[1] : (e == 2 ? f[2] : f[3]));
+            }
+            out[m.x] = f_mul(v, smem[m.z]);
+        }
+    };
     const int z_ps = L >= 4 ? plane : row, z_fs = L >= 4 ? b.nj * zr : zr;
     const size_t parity = (size_t)gridDim.x * 6 * A.side_max * 4;
 
@@ -753,14 +920,40 @@ __global__ void __launch_bounds__(MAXT, 1) k_resident(const __grid_constant__ Sf
         // ---- P
         if (active) {
             p_any<L, NU>(a, S, T, g, o, mode, pml);
-            if (smask) add_sources<L>(src, S, T, i0, k0, o.flags, smask);
+            if (!EXTRA && smask) add_sources<L>(src, S, T, i0, k0, o.flags, smask);
         }
         __syncthreads();
+        if (EXTRA) {
+            for (int q = 0; q < x.n_plane; ++q) {
+                plane_op(a, S, g, x.ops[q], S.prev[q]);
+                __syncthreads();
+            }
+            for (int q = 0; q < src.n; ++q) {
+                if (src.s[q].kind == 2) {  // k_inject_weighted's arithmetic
+                    const double v = reinterpret_cast<const double*>(smem + S.src)[q];
+                    for (int t = tid; t < n_w; t += nthreads) {
+                        const int4 w = wlist[t];
+                        if (w.y != q) continue;
+                        float& p = smem[S.P + w.x];
+                        const double ww = __longlong_as_double(((long long)w.w << 32) | (unsigned)w.z);
+                        p = __double2float_rn(d_add((double)p, d_mul(v, ww)));
+                    }
+                } else if (smask >> q & 1u) {
+                    add_sources<L>(src, S, T, i0, k0, o.flags, 1u << q);
+                }
+                __syncthreads();
+            }
+            if (n_mics > 0) {  // before the next step moves the faces between blocks
+                record_mics(s);
+                __syncthreads();
+            }
+        }
     }
 
     // ---- back to global memory, velocities decayed
     for (int t = tid; t < probes; t += nthreads)
         a.trace_prev[(size_t)(A.n_steps - 1) * a.n_probe + probe[t].x] = smem[S.P + probe[t].y];
+    if (EXTRA) move_prev(a, x, S, g, true);
     if (!active) return;
     const Quad dk = lds_q(S.dz + T.q * 4);
     const float fj = smem[S.dy + T.j];
@@ -796,24 +989,55 @@ constexpr int kKindCount = sizeof(kKinds) / sizeof(kKinds[0]);
 constexpr size_t kSmemMax = 227 * 1024;
 
 template <int L, int MAXT>
-const void* kernel_of(bool nu) {
-    return nu ? reinterpret_cast<const void*>(k_resident<L, MAXT, true>)
-              : reinterpret_cast<const void*>(k_resident<L, MAXT, false>);
+const void* kernel_of(bool nu, bool extra) {
+    if (extra)
+        return nu ? reinterpret_cast<const void*>(k_resident<L, MAXT, true, true>)
+                  : reinterpret_cast<const void*>(k_resident<L, MAXT, false, true>);
+    return nu ? reinterpret_cast<const void*>(k_resident<L, MAXT, true, false>)
+              : reinterpret_cast<const void*>(k_resident<L, MAXT, false, false>);
 }
-const void* kernel_of(int kind, bool nu) {
+const void* kernel_of(int kind, bool nu, bool extra) {
     switch (kind) {
-        case 0: return kernel_of<1, 768>(nu);
-        case 1: return kernel_of<2, 768>(nu);
-        case 2: return kernel_of<4, 640>(nu);
-        default: return kernel_of<8, 512>(nu);
+        case 0: return kernel_of<1, 768>(nu, extra);
+        case 1: return kernel_of<2, 768>(nu, extra);
+        case 2: return kernel_of<4, 640>(nu, extra);
+        default: return kernel_of<8, 512>(nu, extra);
     }
+}
+
+// Microphone rows from the recorded corners (k_mic_gather's sum).
+__global__ void k_resident_mics(const float* __restrict__ corners, const float* __restrict__ w, int n_mic,
+                                long long total, float* __restrict__ out) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= total) return;
+    const int m = (int)(t % n_mic);
+    float s = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) s = f_add(s, f_mul(w[8 * m + q], corners[8 * t + q]));
+    out[t] = s;
 }
 
 }  // namespace
 
+// Whether each plane boundary's end plane and the one inside it lie in one block.
+static bool planes_fit(const SfResExtra& x, int nx, int ny, int nz, int L, int chunks, int quads, int bi,
+                       int bj, int bk) {
+    for (int q = 0; q < x.n_plane; ++q) {
+        const int ax = x.ops[q].axis;
+        const int n = ax == 0 ? nx : (ax == 1 ? ny : nz);
+        if (n < 4) return false;
+        const int units = ax == 0 ? chunks : (ax == 1 ? ny : quads), b = ax == 0 ? bi : (ax == 1 ? bj : bk);
+        const int per = ax == 0 ? L : (ax == 1 ? 1 : 4);
+        const int first = (int)((long long)units / b) * per;
+        const int last = n - (int)((long long)(b - 1) * units / b) * per;
+        if ((first < n ? first : n) < 2 || last < 2) return false;
+    }
+    return true;
+}
+
 // The cut of an nx x ny x nz grid into at most `sms` blocks, or kind < 0 when
 // no kind's blocks hold it.
-SfResCut sf_resident_cut(int nx, int ny, int nz, int n_probe, bool nu, int sms) {
+SfResCut sf_resident_cut(int nx, int ny, int nz, int n_probe, bool nu, int sms, const SfResExtra* x) {
     SfResCut best{};
     best.kind = -1;
     const int quads = (nz + 3) / 4;
@@ -828,6 +1052,7 @@ SfResCut sf_resident_cut(int nx, int ny, int nz, int n_probe, bool nu, int sms) 
                 for (int bk = 1; bk <= bk_max; ++bk) {
                     const int nci = (chunks + bi - 1) / bi, nj = (ny + bj - 1) / bj,
                               nq = (quads + bk - 1) / bk;
+                    if (x && !planes_fit(*x, nx, ny, nz, K.L, chunks, quads, bi, bj, bk)) continue;
                     const long long tiles = (long long)nci * nj * nq;
                     if (tiles > K.threads) continue;
                     int units = 0, side = 0;
@@ -840,13 +1065,14 @@ SfResCut sf_resident_cut(int nx, int ny, int nz, int n_probe, bool nu, int sms) 
                     // the phases' cells, and the messages
                     const long long cost = (tiles + 31) / 32 * 32 * K.L + units;
                     if (best.kind >= 0 && cost >= best_cost) continue;
-                    const Layout lay = layout(K.L, nci, nj, nq, n_probe, nu);
+                    const Layout lay = layout(K.L, nci, nj, nq, n_probe, nu, x);
                     const size_t bytes = sizeof(float) * (size_t)lay.end;
                     if (bytes > kSmemMax) continue;
                     const long long need = std::max<long long>(tiles, (units + kUnits - 1) / kUnits);
                     if (need > K.threads) continue;
                     best_cost = cost;
                     best.kind = kind;
+                    best.extra = x != nullptr;
                     best.bi = bi;
                     best.bj = bj;
                     best.bk = bk;
@@ -871,11 +1097,18 @@ int sf_launch_resident(SfResArgs& A, const SfSources& src, const SfResCut& c, cu
     A.quads = c.quads;
     A.side_max = c.side_max;
     A.lay = c.lay;
-    const void* k = kernel_of(c.kind, A.a.nu_cv[0] != nullptr);
+    const void* k = kernel_of(c.kind, A.a.nu_cv[0] != nullptr, c.extra);
     SF_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
     SfSources s = src;
     void* args[] = {&A, &s};
     const cudaError_t e = cudaLaunchCooperativeKernel(k, dim3(c.bi * c.bj * c.bk), dim3(c.threads), args,
                                                       c.smem, st);
     return e == cudaSuccess ? 0 : sf_fail_cuda(e, "k_resident launch", __FILE__, __LINE__);
+}
+
+int sf_launch_resident_mics(const float* corners, const float* w, int n_mic, long long n_steps,
+                            float* mic_trace, cudaStream_t st) {
+    const long long total = n_steps * n_mic;
+    k_resident_mics<<<(unsigned)((total + 127) / 128), 128, 0, st>>>(corners, w, n_mic, total, mic_trace);
+    return cudaGetLastError() == cudaSuccess ? 0 : sf_fail("k_resident_mics launch failed");
 }
