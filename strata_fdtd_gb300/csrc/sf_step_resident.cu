@@ -29,7 +29,7 @@
 // message through L2 (about 1 us) and two barriers; the shared-memory reads and
 // writes of 15 000 cells take about 3 us of an SM.  Measured on GB300, whole
 // run_steps calls per step, single-step kernels -> this one: 52 x 44 x 48 7.1 ->
-// 2.3 us, 100^3 9.7 -> 4.7 us, stretched 144 x 120 x 132 20.3 -> 10.0 us.
+// 2.3 us, 100^3 9.7 -> 3.9 us, stretched 144 x 120 x 132 20.3 -> 10.0 us.
 //
 // Messages carry each 32-bit value beside a 32-bit step tag in one 64-bit
 // word, so a reader that sees the tag has the value: no fence and no flag.
@@ -541,6 +541,9 @@ __device__ __forceinline__ void p_any(const SfStepArgs& a, const Layout& S, cons
 // Message units a thread has at most.
 constexpr int kUnits = 2;
 
+// A mailbox holds the first two words of every unit of its side, then the last
+// two, so that neighbouring threads' 16-byte accesses are adjacent.
+//
 // A message unit: its first pressure and first face in shared memory, its words in
 // the neighbour's mailbox and in this block's, and
 // side | open faces << 3 | values in the unit << 7 (0: no unit).
@@ -557,15 +560,15 @@ struct Unit {
 
 // Waits for the words of this thread's units to carry the tag `want`; false when
 // the wait ran out (or another thread's did).
-__device__ __forceinline__ bool receive(const u64* mail, const Unit (&U)[kUnits], unsigned want,
+__device__ __forceinline__ bool receive(const u64* mail, const Unit (&U)[kUnits], int half, unsigned want,
                                         long long limit, const volatile int* stop, Quad (&r)[kUnits]) {
     for (long long polls = 0;; ++polls) {
         ulonglong2 m[kUnits][2];
         bool ready = true;
 #pragma unroll
         for (int w = 0; w < kUnits; ++w) {
-            m[w][0] = recv2(mail + U[w].recv);  // a missing unit reads the first one's words
-            m[w][1] = recv2(mail + U[w].recv + 2);
+            m[w][0] = recv2(mail + U[w].recv);  // a missing unit reads word 0
+            m[w][1] = recv2(mail + U[w].recv + half);
         }
 #pragma unroll
         for (int w = 0; w < kUnits; ++w) {
@@ -633,7 +636,7 @@ __device__ __forceinline__ Unit make_unit(const SfResArgs& A, const Place& g, in
     const int step[3] = {A.bj * A.bk, A.bk, 1}, words = A.side_max * 4;
     const int to = (int)blockIdx.x + (high ? step[ax] : -step[ax]);
     return Unit{(unsigned)t.p | ((unsigned)t.f << 16), (unsigned)side | (open << 3) | ((unsigned)n << 7),
-                (to * 6 + (side ^ 1)) * words + u * 4, ((int)blockIdx.x * 6 + side) * words + u * 4};
+                (to * 6 + (side ^ 1)) * words + u * 2, ((int)blockIdx.x * 6 + side) * words + u * 2};
 }
 
 // EXTRA: plane boundaries, weighted sources or microphones between the steps
@@ -849,6 +852,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_resident(const __grid_constant__ Sf
     };
     const int z_ps = L >= 4 ? plane : row, z_fs = L >= 4 ? b.nj * zr : zr;
     const size_t parity = (size_t)gridDim.x * 6 * A.side_max * 4;
+    const int half = A.side_max * 2;
 
     for (int s = 0; s < A.n_steps; ++s) {
         // ---- V
@@ -869,7 +873,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_resident(const __grid_constant__ Sf
                              smem[p + min(3, n) * z_ps]);
                 }
                 send2(mail + U[w].send, tagged(v[0], tag), tagged(v[1], tag));
-                send2(mail + U[w].send + 2, tagged(v[2], tag), tagged(v[3], tag));
+                send2(mail + U[w].send + half, tagged(v[2], tag), tagged(v[3], tag));
             }
         }
         if (s > 0)
@@ -879,7 +883,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_resident(const __grid_constant__ Sf
         if (has_units) {
             const unsigned want = tag + ((A.hold && blockIdx.x == 0) ? 0x40000000u : 0u);
             Quad r[kUnits];
-            if (!receive(mail, U, want, A.poll_limit, ctl + 2, r)) ctl[2] = 1;
+            if (!receive(mail, U, half, want, A.poll_limit, ctl + 2, r)) ctl[2] = 1;
 #pragma unroll
             for (int w = 0; w < kUnits; ++w) {
                 if (U[w].d == 0) continue;
@@ -977,14 +981,17 @@ __global__ void __launch_bounds__(MAXT, 1) k_resident(const __grid_constant__ Sf
 
 // ---- partition ----------------------------------------------------------------
 
-// Planes per thread, threads at most.
+// Planes per thread, threads at most (512 of 128 registers: with 640 to 768 the
+// kernels spilled, 52 x 44 x 48 0.73 ms against 0.69 for 250 steps, 100^3 2.44
+// against 2.22 for 500; loading operands ahead of the stores spilled again, 2.36
+// to 2.46).
 // More planes hold more cells per SM (the registers of a thread grow more
 // slowly than its cells) but make a longer chain per phase: the smallest L
 // whose blocks fit is taken.
 struct ResKind {
     int L, threads;
 };
-const ResKind kKinds[] = {{1, 768}, {2, 768}, {4, 640}, {8, 512}};
+const ResKind kKinds[] = {{1, 512}, {2, 512}, {4, 512}, {8, 512}};
 constexpr int kKindCount = sizeof(kKinds) / sizeof(kKinds[0]);
 constexpr size_t kSmemMax = 227 * 1024;
 
@@ -998,9 +1005,9 @@ const void* kernel_of(bool nu, bool extra) {
 }
 const void* kernel_of(int kind, bool nu, bool extra) {
     switch (kind) {
-        case 0: return kernel_of<1, 768>(nu, extra);
-        case 1: return kernel_of<2, 768>(nu, extra);
-        case 2: return kernel_of<4, 640>(nu, extra);
+        case 0: return kernel_of<1, 512>(nu, extra);
+        case 1: return kernel_of<2, 512>(nu, extra);
+        case 2: return kernel_of<4, 512>(nu, extra);
         default: return kernel_of<8, 512>(nu, extra);
     }
 }
