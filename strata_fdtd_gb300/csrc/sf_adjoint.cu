@@ -33,6 +33,7 @@
 // or double for dwf.
 #include <cuda_runtime.h>
 
+#include <initializer_list>
 #include <type_traits>
 
 #include "sf_common.cuh"
@@ -203,6 +204,9 @@ __global__ void k_dcoef(const E* __restrict__ theta, const uint8_t* __restrict__
     cvz[c] = (k < nz - 1) ? face(c + 1) : T(0);
 }
 
+// Launches take the planes in alternate order (`reverse`), so that each begins
+// with what the one before it wrote last, still in L2.
+//
 // Forward step (per cell, ping-pong): out = step(in); p_store, when given,
 // receives the step's input pressure; with n_fused > 0 the cells listed in
 // probe_cells write their new pressure into trace_row (else k_dprobe samples
@@ -260,10 +264,11 @@ __global__ void __launch_bounds__(256, (kFwdMinBlocks<T, I>)) k_dfwd(DiffPtrs<T>
                        const T* __restrict__ vy, const T* __restrict__ vz, T* __restrict__ po,
                        T* __restrict__ vxo, T* __restrict__ vyo, T* __restrict__ vzo,
                        long long src_cell, const T* __restrict__ src_val, T* __restrict__ p_store,
-                       const int64_t* __restrict__ probe_cells, int n_fused, E* __restrict__ trace_row) {
+                       const int64_t* __restrict__ probe_cells, int n_fused, E* __restrict__ trace_row,
+                       int reverse) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int i = blockIdx.z;
+    const int i = reverse ? (int)(gridDim.z - 1 - blockIdx.z) : (int)blockIdx.z;
     const bool unit = kUnitBodies<T> && block_in_unit_decay(g, i);
     if (k >= g.nz || j >= g.ny) return;
     if (unit)
@@ -272,6 +277,224 @@ __global__ void __launch_bounds__(256, (kFwdMinBlocks<T, I>)) k_dfwd(DiffPtrs<T>
     else
         dfwd_cell<false, T, I, E>(g, i, j, k, p, vx, vy, vz, po, vxo, vyo, vzo, src_cell, src_val,
                                   p_store, probe_cells, n_fused, trace_row);
+}
+
+// ---- two cells per thread (double-word) ---------------------------------------
+//
+// A thread takes cells k and k + 1 of a row and runs both through the packed FP32
+// instructions (dw2, sf_dw.cuh): half the issue slots per operation, one load for
+// both cells where rows are 16-byte aligned, and the face between the two formed
+// once (the per-cell kernels issue 619 and 1075 instructions per cell).
+// Bit-identical to the per-cell kernels.  What is left is memory latency, so
+// resident warps count: at 128^3 the forward takes 46.7 us with 3 blocks per SM
+// (70 registers), 42.3 with 4, 39.7 with 5 (48 registers), 40.8 with 6; the
+// adjoint 87.1 with 2, 70.5 with 3, 69.2 with 4.  Per cell, planes in alternate
+// order: 45.6 and 73.3; in one order 49.7 and 77.3.  Measured slower: blocks that
+// walk planes and share faces through shared memory (57.9 to 67.1 and 112 to
+// 125), threads that carry the x face and p over 2 or 4 planes (42.7 to 50.1).
+
+// ALIGNED: nz is even and the arrays are 16-byte aligned, so that a pair is one
+// access and always whole.
+template <bool ALIGNED>
+__device__ __forceinline__ dw2 ld2(const dwf* __restrict__ f, int c, bool two) {
+    if (ALIGNED) {
+        const float4 t = *reinterpret_cast<const float4*>(f + c);
+        return {sf_dw::pair(t.x, t.z), sf_dw::pair(t.y, t.w)};
+    }
+    const float2 a = *reinterpret_cast<const float2*>(f + c);
+    const float2 b = two ? *reinterpret_cast<const float2*>(f + c + 1) : make_float2(0.0f, 0.0f);
+    return {sf_dw::pair(a.x, b.x), sf_dw::pair(a.y, b.y)};
+}
+template <bool ALIGNED>
+__device__ __forceinline__ void st2(dwf* __restrict__ f, int c, bool two, dw2 v) {
+    using namespace sf_dw;
+    if (ALIGNED) {
+        *reinterpret_cast<float4*>(f + c) = make_float4(lane0(v.hi), lane0(v.lo), lane1(v.hi), lane1(v.lo));
+        return;
+    }
+    *reinterpret_cast<float2*>(f + c) = make_float2(lane0(v.hi), lane0(v.lo));
+    if (two) *reinterpret_cast<float2*>(f + c + 1) = make_float2(lane1(v.hi), lane1(v.lo));
+}
+__device__ __forceinline__ dw2 zero2() { return {0ull, 0ull}; }
+// lane e of a where its condition holds, else of b
+__device__ __forceinline__ dw2 pick(bool c0, bool c1, dw2 a, dw2 b) {
+    using namespace sf_dw;
+    return join(c0 ? first(a) : first(b), c1 ? second(a) : second(b));
+}
+
+template <bool UNIT, bool ALIGNED>
+__device__ __forceinline__ void dfwd_pair(const DiffPtrs<dwf>& g, int i, int j, int k, const dwf* __restrict__ p,
+                                          const dwf* __restrict__ vx, const dwf* __restrict__ vy,
+                                          const dwf* __restrict__ vz, dwf* __restrict__ po,
+                                          dwf* __restrict__ vxo, dwf* __restrict__ vyo,
+                                          dwf* __restrict__ vzo, long long src_cell,
+                                          const dwf* __restrict__ src_val, dwf* __restrict__ p_store,
+                                          const int64_t* __restrict__ probe_cells, int n_fused,
+                                          double* __restrict__ trace_row) {
+    using namespace sf_dw;
+    const int plane = (int)g.plane, nz = g.nz;
+    const int c = i * plane + j * nz + k;
+    const bool two = ALIGNED || k + 1 < nz;
+    const dw2 pc = ld2<ALIGNED>(p, c, two);
+    if (p_store) st2<ALIGNED>(p_store, c, two, pc);
+    dw2 ux = ld2<ALIGNED>(vx, c, two), uy = ld2<ALIGNED>(vy, c, two), uz = ld2<ALIGNED>(vz, c, two);
+    if (i < g.nx - 1) ux = ux + ld2<ALIGNED>(g.cvx, c, two) * (ld2<ALIGNED>(p, c + plane, two) - pc);
+    if (j < g.ny - 1) uy = uy + ld2<ALIGNED>(g.cvy, c, two) * (ld2<ALIGNED>(p, c + nz, two) - pc);
+    {
+        const dw2 up = join(second(pc), k + 2 < nz ? p[c + 2] : dwf(0));
+        uz = pick(k < nz - 1, k + 1 < nz - 1, uz + ld2<ALIGNED>(g.cvz, c, two) * (up - pc), uz);
+    }
+    dw2 uxm = zero2(), uym = zero2();
+    if (i > 0)
+        uxm = ld2<ALIGNED>(vx, c - plane, two) +
+              ld2<ALIGNED>(g.cvx, c - plane, two) * (pc - ld2<ALIGNED>(p, c - plane, two));
+    if (j > 0)
+        uym = ld2<ALIGNED>(vy, c - nz, two) + ld2<ALIGNED>(g.cvy, c - nz, two) * (pc - ld2<ALIGNED>(p, c - nz, two));
+    dwf low(0);
+    if (k > 0) low = vz[c - 1] + g.cvz[c - 1] * (first(pc) - p[c - 1]);
+    const dw2 uzm = join(low, first(uz));
+    dw2 pn = pc + both(g.cp) * (((ux - uxm) + (uy - uym)) + (uz - uzm));
+    if constexpr (!UNIT) {
+        const dw2 di = both(g.dx[i]), dj = both(g.dy[j]), dk = join(g.dz[k], two ? g.dz[k + 1] : dwf(0));
+        ux = ux * di;
+        uy = uy * dj;
+        uz = uz * dk;
+        pn = ((pn * di) * dj) * dk;
+    }
+    st2<ALIGNED>(vxo, c, two, ux);
+    st2<ALIGNED>(vyo, c, two, uy);
+    st2<ALIGNED>(vzo, c, two, uz);
+    const long long at = c;
+    if (src_val != nullptr && (at == src_cell || (two && at + 1 == src_cell)))
+        pn = at == src_cell ? join(first(pn) + *src_val, second(pn)) : join(first(pn), second(pn) + *src_val);
+    st2<ALIGNED>(po, c, two, pn);
+    for (int q = 0; q < n_fused; ++q) {
+        if (at == probe_cells[q]) trace_row[q] = first(pn).to_double();
+        if (two && at + 1 == probe_cells[q]) trace_row[q] = second(pn).to_double();
+    }
+}
+
+// Whether the block's cells (64 k x 8 j) and their neighbours have unit decays.
+__device__ __forceinline__ bool pair_block_unit(const DiffPtrs<dwf>& g, int i) {
+    const int j0 = blockIdx.y * 8, k0 = blockIdx.x * 64;
+    const int j1 = min(j0 + 8, g.ny) - 1, k1 = min(k0 + 64, g.nz) - 1;
+    return i >= g.unit_lo[0] && i < g.unit_hi[0] && j0 >= g.unit_lo[1] && j1 < g.unit_hi[1] &&
+           k0 >= g.unit_lo[2] && k1 < g.unit_hi[2];
+}
+
+template <bool ALIGNED>
+__global__ void __launch_bounds__(256, 5)
+    k_dfwd_pair(DiffPtrs<dwf> g, const dwf* __restrict__ p, const dwf* __restrict__ vx,
+                const dwf* __restrict__ vy, const dwf* __restrict__ vz, dwf* __restrict__ po,
+                dwf* __restrict__ vxo, dwf* __restrict__ vyo, dwf* __restrict__ vzo, long long src_cell,
+                const dwf* __restrict__ src_val, dwf* __restrict__ p_store,
+                const int64_t* __restrict__ probe_cells, int n_fused, double* __restrict__ trace_row,
+                int reverse) {
+    const int k = 2 * (blockIdx.x * 32 + threadIdx.x);
+    const int j = blockIdx.y * 8 + threadIdx.y;
+    const int i = reverse ? (int)(gridDim.z - 1 - blockIdx.z) : (int)blockIdx.z;
+    if (k >= g.nz || j >= g.ny) return;
+    if (pair_block_unit(g, i))
+        dfwd_pair<true, ALIGNED>(g, i, j, k, p, vx, vy, vz, po, vxo, vyo, vzo, src_cell, src_val, p_store,
+                                 probe_cells, n_fused, trace_row);
+    else
+        dfwd_pair<false, ALIGNED>(g, i, j, k, p, vx, vy, vz, po, vxo, vyo, vzo, src_cell, src_val, p_store,
+                                  probe_cells, n_fused, trace_row);
+}
+
+// GradAcc<dwf>::add for both cells (c0, c1: which of them have the face)
+template <bool ALIGNED>
+__device__ __forceinline__ void grad2(double* g, int c, bool two, bool c0, bool c1, dw2 a, dw2 b) {
+    dwf* f = reinterpret_cast<dwf*>(g);
+    const dw2 x = ld2<ALIGNED>(f, c, two);
+    st2<ALIGNED>(f, c, two, pick(c0, c1, sf_dw::add(x, a * b), x));
+}
+
+template <bool UNIT, bool ALIGNED>
+__device__ __forceinline__ void dadj_pair(const DiffPtrs<dwf>& g, int i, int j, int k, const dwf* __restrict__ lp,
+                                          const dwf* __restrict__ lx, const dwf* __restrict__ ly,
+                                          const dwf* __restrict__ lz, dwf* __restrict__ lpo,
+                                          dwf* __restrict__ lxo, dwf* __restrict__ lyo,
+                                          dwf* __restrict__ lzo, const dwf* __restrict__ pst,
+                                          double* __restrict__ gx, double* __restrict__ gy,
+                                          double* __restrict__ gz) {
+    using namespace sf_dw;
+    const int nx = g.nx, ny = g.ny, nz = g.nz, plane = (int)g.plane;
+    const int c = i * plane + j * nz + k;
+    const bool two = ALIGNED || k + 1 < nz;
+    const bool z0 = k < nz - 1, z1 = k + 1 < nz - 1;  // the cells' high z faces exist
+    const dw2 cp = both(g.cp);
+    const dw2 dk = UNIT ? zero2() : join(g.dz[k], two ? g.dz[k + 1] : dwf(0));
+    auto mup2 = [&](int ii, int jj, int q) -> dw2 {
+        const dw2 v = ld2<ALIGNED>(lp, q, two);
+        if constexpr (UNIT) return v;
+        else return both(g.dx[ii] * g.dy[jj]) * dk * v;
+    };
+    auto mup1 = [&](int kk, int q) -> dwf {
+        if constexpr (UNIT) return lp[q];
+        else return g.dx[i] * g.dy[j] * g.dz[kk] * lp[q];
+    };
+    auto dec = [&](dw2 v, const dwf& d) -> dw2 {
+        if constexpr (UNIT) return v;
+        else return both(d) * v;
+    };
+    const dw2 m0 = mup2(i, j, c);
+    const dw2 mxp = i < nx - 1 ? mup2(i + 1, j, c + plane) : zero2();
+    const dw2 myp = j < ny - 1 ? mup2(i, j + 1, c + nz) : zero2();
+    const dw2 mzp = join(z0 ? second(m0) : dwf(0), z1 ? mup1(k + 2, c + 2) : dwf(0));
+    const dw2 vx_hi = dec(ld2<ALIGNED>(lx, c, two), g.dx[i]) + cp * (m0 - mxp);
+    const dw2 vy_hi = dec(ld2<ALIGNED>(ly, c, two), g.dy[j]) + cp * (m0 - myp);
+    dw2 zl = ld2<ALIGNED>(lz, c, two);
+    if constexpr (!UNIT) zl = dk * zl;
+    const dw2 vz_hi = zl + cp * (m0 - mzp);
+    st2<ALIGNED>(lxo, c, two, vx_hi);
+    st2<ALIGNED>(lyo, c, two, vy_hi);
+    st2<ALIGNED>(lzo, c, two, vz_hi);
+    dw2 acc = m0;
+    if (i > 0) {
+        const dw2 v = dec(ld2<ALIGNED>(lx, c - plane, two), UNIT ? dwf(1) : g.dx[i - 1]) +
+                      cp * (mup2(i - 1, j, c - plane) - m0);
+        acc = acc + ld2<ALIGNED>(g.cvx, c - plane, two) * v;
+    }
+    if (j > 0) {
+        const dw2 v = dec(ld2<ALIGNED>(ly, c - nz, two), UNIT ? dwf(1) : g.dy[j - 1]) +
+                      cp * (mup2(i, j - 1, c - nz) - m0);
+        acc = acc + ld2<ALIGNED>(g.cvy, c - nz, two) * v;
+    }
+    const dw2 cz = ld2<ALIGNED>(g.cvz, c, two);
+    {
+        dwf v(0), w(0);
+        if (k > 0) {
+            dwf l = lz[c - 1];
+            if constexpr (!UNIT) l = g.dz[k - 1] * l;
+            v = l + g.cp * (mup1(k - 1, c - 1) - first(m0));
+            w = g.cvz[c - 1];
+        }
+        acc = pick(k > 0, true, acc + join(w, first(cz)) * join(v, first(vz_hi)), acc);
+    }
+    acc = acc - (ld2<ALIGNED>(g.cvx, c, two) * vx_hi + ld2<ALIGNED>(g.cvy, c, two) * vy_hi + cz * vz_hi);
+    st2<ALIGNED>(lpo, c, two, acc);
+    const dw2 p0 = ld2<ALIGNED>(pst, c, two);
+    if (i < nx - 1) grad2<ALIGNED>(gx, c, two, true, true, vx_hi, ld2<ALIGNED>(pst, c + plane, two) - p0);
+    if (j < ny - 1) grad2<ALIGNED>(gy, c, two, true, true, vy_hi, ld2<ALIGNED>(pst, c + nz, two) - p0);
+    if (z0) grad2<ALIGNED>(gz, c, two, true, z1, vz_hi, join(second(p0), z1 ? pst[c + 2] : dwf(0)) - p0);
+}
+
+template <bool ALIGNED>
+__global__ void __launch_bounds__(256, 4)
+    k_dadj_pair(DiffPtrs<dwf> g, const dwf* __restrict__ lp, const dwf* __restrict__ lx,
+                const dwf* __restrict__ ly, const dwf* __restrict__ lz, dwf* __restrict__ lpo,
+                dwf* __restrict__ lxo, dwf* __restrict__ lyo, dwf* __restrict__ lzo,
+                const dwf* __restrict__ pst, double* __restrict__ gx, double* __restrict__ gy,
+                double* __restrict__ gz, int reverse) {
+    const int k = 2 * (blockIdx.x * 32 + threadIdx.x);
+    const int j = blockIdx.y * 8 + threadIdx.y;
+    const int i = reverse ? (int)(gridDim.z - 1 - blockIdx.z) : (int)blockIdx.z;
+    if (k >= g.nz || j >= g.ny) return;
+    if (pair_block_unit(g, i))
+        dadj_pair<true, ALIGNED>(g, i, j, k, lp, lx, ly, lz, lpo, lxo, lyo, lzo, pst, gx, gy, gz);
+    else
+        dadj_pair<false, ALIGNED>(g, i, j, k, lp, lx, ly, lz, lpo, lxo, lyo, lzo, pst, gx, gy, gz);
 }
 
 template <typename T, typename E = typename Ext<T>::E>
@@ -357,10 +580,10 @@ __global__ void k_dadj(DiffPtrs<T> g, const T* __restrict__ lp, const T* __restr
                        const T* __restrict__ ly, const T* __restrict__ lz, T* __restrict__ lpo,
                        T* __restrict__ lxo, T* __restrict__ lyo, T* __restrict__ lzo,
                        const T* __restrict__ pst, double* __restrict__ gx,
-                       double* __restrict__ gy, double* __restrict__ gz) {
+                       double* __restrict__ gy, double* __restrict__ gz, int reverse) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int i = blockIdx.z;
+    const int i = reverse ? (int)(gridDim.z - 1 - blockIdx.z) : (int)blockIdx.z;
     const bool unit = kUnitBodies<T> && block_in_unit_decay(g, i);
     if (k >= g.nz || j >= g.ny) return;
     if (unit)
@@ -448,6 +671,15 @@ DiffPtrs<T> ptrs(const sf_diff_desc* d, const void* const* cv) {
     return g;
 }
 
+dim3 pair_grid(const sf_diff_desc* d) { return dim3((d->nz + 63) / 64, (d->ny + 7) / 8, d->nx); }
+// Whether a double-word pair is one 16-byte access in all these arrays.
+bool pairs_aligned(const sf_diff_desc* d, std::initializer_list<const void*> arrays) {
+    if (d->nz % 2 != 0) return false;
+    for (const void* a : arrays)
+        if (reinterpret_cast<uintptr_t>(a) & 15u) return false;
+    return true;
+}
+
 dim3 grid_of(const sf_diff_desc* d) { return dim3((d->nz + 31) / 32, (d->ny + 7) / 8, d->nx); }
 
 template <typename T>
@@ -465,11 +697,21 @@ int forward(const sf_diff_desc* d, const void* const* cv, void* const* set0, voi
         void* const* in = cur ? set1 : set0;
         void* const* out = cur ? set0 : set1;
         auto kernel = narrow ? k_dfwd<T, int> : k_dfwd<T, long long>;
-        kernel<<<grid_of(d), dim3(32, 8), 0, st>>>(
+        dim3 grid = grid_of(d);
+        if constexpr (std::is_same<T, dwf>::value) {
+            if (narrow) {  // two cells per thread (32-bit cell indices)
+                grid = pair_grid(d);
+                kernel = pairs_aligned(d, {in[0], in[1], in[2], in[3], out[0], out[1], out[2], out[3], g.cvx,
+                                           g.cvy, g.cvz, ps})
+                             ? k_dfwd_pair<true>
+                             : k_dfwd_pair<false>;
+            }
+        }
+        kernel<<<grid, dim3(32, 8), 0, st>>>(
             g, (const T*)in[0], (const T*)in[1], (const T*)in[2], (const T*)in[3], (T*)out[0],
             (T*)out[1], (T*)out[2], (T*)out[3], d->src_cell, sv ? sv + s : nullptr,
             ps ? ps + s * N : nullptr, d->probe_cells, fuse ? d->n_probe : 0,
-            fuse ? tr + s * d->n_probe : nullptr);
+            fuse ? tr + s * d->n_probe : nullptr, (int)(s & 1));
         if (tr && d->n_probe > 0 && !fuse)
             k_dprobe<T><<<(d->n_probe + 127) / 128, 128, 0, st>>>((const T*)out[0], d->probe_cells,
                                                                   d->n_probe, tr + s * d->n_probe);
@@ -497,10 +739,20 @@ int adjoint(const sf_diff_desc* d, const void* const* cv, void* const* lam0, voi
                 (T*)in[0], d->probe_cells, d->n_probe, tr + s * d->n_probe, tg + s * d->n_probe,
                 (E)weight);
         auto kernel = narrow ? k_dadj<T, int> : k_dadj<T, long long>;
-        kernel<<<grid_of(d), dim3(32, 8), 0, st>>>(
+        dim3 grid = grid_of(d);
+        if constexpr (std::is_same<T, dwf>::value) {
+            if (narrow) {
+                grid = pair_grid(d);
+                kernel = pairs_aligned(d, {in[0], in[1], in[2], in[3], out[0], out[1], out[2], out[3], g.cvx,
+                                           g.cvy, g.cvz, ps, grad_cv[0], grad_cv[1], grad_cv[2]})
+                             ? k_dadj_pair<true>
+                             : k_dadj_pair<false>;
+            }
+        }
+        kernel<<<grid, dim3(32, 8), 0, st>>>(
             g, (const T*)in[0], (const T*)in[1], (const T*)in[2], (const T*)in[3], (T*)out[0],
             (T*)out[1], (T*)out[2], (T*)out[3], ps + s * N, (double*)grad_cv[0],
-            (double*)grad_cv[1], (double*)grad_cv[2]);
+            (double*)grad_cv[1], (double*)grad_cv[2], (int)(s & 1));
         cur = 1 - cur;
     }
     return cudaGetLastError() == cudaSuccess ? 0 : sf_fail("sf_diff_adjoint: launch failed");

@@ -108,3 +108,105 @@ __device__ __forceinline__ dwf operator-(dwf a, dwf b) { return sf_dw::add_fast(
 __device__ __forceinline__ dwf operator*(dwf a, dwf b) { return sf_dw::mul(a, b); }
 __device__ __forceinline__ dwf& operator+=(dwf& a, dwf b) { return a = a + b; }
 __device__ __forceinline__ dwf& operator-=(dwf& a, dwf b) { return a = a - b; }
+
+// ---- two double-words side by side --------------------------------------------
+//
+// dw2 holds two cells' values, the high parts in one pair of floats and the low
+// parts in another, for the packed FP32 instructions (two results per issue
+// slot).  Each lane sees the scalar functions' operations in their order, so its
+// value is theirs bit for bit: a - b is formed by subtractions in place of
+// additions of -b, and a product as a * b + (-0) with a -0 that the assembler
+// cannot see (it fuses a packed mul and add into one rounding otherwise, even
+// with .rn and -fmad=false).
+struct dw2 {
+    unsigned long long hi, lo;
+};
+
+namespace sf_dw {
+
+typedef unsigned long long u64;
+static __constant__ u64 kNegZeroPair = 0x8000000080000000ull;
+
+__device__ __forceinline__ u64 pair(float a, float b) {
+    return ((u64)__float_as_uint(b) << 32) | __float_as_uint(a);
+}
+__device__ __forceinline__ float lane0(u64 p) { return __uint_as_float((unsigned)p); }
+__device__ __forceinline__ float lane1(u64 p) { return __uint_as_float((unsigned)(p >> 32)); }
+__device__ __forceinline__ u64 padd(u64 a, u64 b) {
+    u64 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ u64 psub(u64 a, u64 b) {
+    u64 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ u64 pfma(u64 a, u64 b, u64 c) {
+    u64 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ u64 pmul(u64 a, u64 b) { return pfma(a, b, kNegZeroPair); }
+__device__ __forceinline__ u64 pneg(u64 a) { return psub(kNegZeroPair, a); }  // -0 - a = -a, zeros too
+
+__device__ __forceinline__ void ptwo_sum(u64 a, u64 b, u64& s, u64& e) {
+    s = padd(a, b);
+    const u64 bv = psub(s, a);
+    const u64 av = psub(s, bv);
+    e = padd(psub(a, av), psub(b, bv));
+}
+// two_sum(a, -b): fl(-b - bv) = -fl(b + bv)
+__device__ __forceinline__ void ptwo_diff(u64 a, u64 b, u64& s, u64& e) {
+    s = psub(a, b);
+    const u64 bv = psub(s, a);
+    const u64 av = psub(s, bv);
+    e = psub(psub(a, av), padd(b, bv));
+}
+__device__ __forceinline__ void pfast_two_sum(u64 a, u64 b, u64& s, u64& e) {
+    s = padd(a, b);
+    e = psub(b, psub(s, a));
+}
+__device__ __forceinline__ dw2 add(dw2 x, dw2 y) {
+    u64 sh, sl, th, tl, vh, vl;
+    dw2 z;
+    ptwo_sum(x.hi, y.hi, sh, sl);
+    ptwo_sum(x.lo, y.lo, th, tl);
+    pfast_two_sum(sh, padd(sl, th), vh, vl);
+    pfast_two_sum(vh, padd(tl, vl), z.hi, z.lo);
+    return z;
+}
+__device__ __forceinline__ dw2 both(dwf v) { return {pair(v.hi, v.hi), pair(v.lo, v.lo)}; }
+__device__ __forceinline__ dw2 join(dwf a, dwf b) { return {pair(a.hi, b.hi), pair(a.lo, b.lo)}; }
+__device__ __forceinline__ dwf first(dw2 v) { return dwf(lane0(v.hi), lane0(v.lo)); }
+__device__ __forceinline__ dwf second(dw2 v) { return dwf(lane1(v.hi), lane1(v.lo)); }
+
+}  // namespace sf_dw
+
+__device__ __forceinline__ dw2 operator+(dw2 x, dw2 y) {
+    using namespace sf_dw;
+    u64 sh, sl;
+    dw2 z;
+    ptwo_sum(x.hi, y.hi, sh, sl);
+    ptwo_sum(sh, padd(sl, padd(x.lo, y.lo)), z.hi, z.lo);
+    return z;
+}
+__device__ __forceinline__ dw2 operator-(dw2 x, dw2 y) {
+    using namespace sf_dw;
+    u64 sh, sl;
+    dw2 z;
+    ptwo_diff(x.hi, y.hi, sh, sl);
+    ptwo_sum(sh, padd(sl, psub(x.lo, y.lo)), z.hi, z.lo);
+    return z;
+}
+__device__ __forceinline__ dw2 operator*(dw2 x, dw2 y) {
+    using namespace sf_dw;
+    const u64 ch = pmul(x.hi, y.hi);
+    const u64 cl1 = pfma(x.hi, y.hi, pneg(ch));
+    const u64 tl0 = pmul(x.lo, y.lo);
+    const u64 tl1 = pfma(x.hi, y.lo, tl0);
+    const u64 cl2 = pfma(x.lo, y.hi, tl1);
+    dw2 z;
+    pfast_two_sum(ch, padd(cl1, cl2), z.hi, z.lo);
+    return z;
+}
