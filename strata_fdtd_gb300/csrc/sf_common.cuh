@@ -70,6 +70,39 @@ struct SfStepArgs {
     const float* nu_inv[3];           // nonuniform grid: cell inverse spacings per axis
 };
 
+// Programmatic dependent launch: a kernel launched with launch_dependent may be
+// set up while the kernel before it on the stream drains, and calls
+// await_previous() before it touches anything that kernel wrote (or reads).  Every
+// kernel launched so must call it; it also lets the next one be set up, which
+// happens once all its blocks have started.  The pointers are passed through it, so
+// that no load by them can be moved above the wait: a const __restrict__ argument
+// counts as unchanging during the kernel, and its loads are free of the barrier
+// otherwise.
+template <class P>
+__device__ __forceinline__ void launder(P& p) {
+    unsigned long long a = reinterpret_cast<unsigned long long>(p);
+    asm volatile("" : "+l"(a));
+    p = reinterpret_cast<P>(a);
+}
+template <class... P>
+__device__ __forceinline__ void await_previous(P&... pointers) {
+    asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+    (launder(pointers), ...);
+}
+template <class... P, class... A>
+inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = st;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 #define SF_CUDA_OK(expr)                                                   \
     do {                                                                   \
         cudaError_t e_ = (expr);                                           \

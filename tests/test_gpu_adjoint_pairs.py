@@ -30,3 +30,38 @@ def test_double_word_pairs_match_fp64_on_odd_rows(shape):
     # 40 + 40 steps of operations with |error| <= 3 * 2^-48 relative to their operands
     for a, b in ((t0, t1), (p0, p1)):
         assert float((a - b).abs().max()) <= 1e-10 * float(b.abs().max())
+
+
+@pytest.mark.parametrize("dtype", ["dw", torch.float64, torch.float32])
+@pytest.mark.parametrize("shape", [(8, 7, 12), (9, 8, 33), (10, 6, 1), (9, 8, 11)])
+def test_injection_in_the_adjoint_kernel_matches_its_own_launch(dtype, shape):
+    """Up to four probes are injected by the adjoint kernel, more by a launch
+    between two steps.  Probes whose target is their own trace inject exactly
+    zero, so three probes and the same three plus such ones give one gradient:
+    equal bits, but for FP32 atomics, which flush subnormals (1e-6)."""
+    n = 21
+    first = (0, 0, 0)
+    probes = [first, tuple(v // 2 for v in shape), tuple(v - 1 for v in shape)]
+    if dtype == "dw":
+        probes[1] = probes[2]  # two on one cell, added in their order
+    more = [(1, 1, 0), (2, 0, 0), (3, 3, 0)]
+    g = torch.Generator().manual_seed(7)
+    theta = torch.rand(shape, generator=g, dtype=torch.float64)
+    target = 1e-3 * torch.rand((n, 3), generator=g, dtype=torch.float64)
+    grads = []
+    for extra in ([], more):
+        ds = S.DifferentiableSolver(shape, pml_depth=1, frequency=20000.0, probes=probes + extra,
+                                    dtype=dtype, checkpoint_every=8)
+        th = theta.to(ds.ext_dtype).cuda().requires_grad_()
+        goal = target.to(ds.ext_dtype).cuda()
+        if extra:
+            goal = torch.cat([goal, ds.forward(th.detach(), n)[0][:, 3:]], 1)
+        ds.loss(th, goal, n).backward()
+        grads.append(th.grad)
+    a, b = grads
+    if max(shape) < 20:  # (in 21 steps the long grid's corners hear nothing yet)
+        assert float(b.abs().max()) > 0
+    if dtype == torch.float32:
+        assert float((a - b).abs().max()) <= 1e-6 * float(b.abs().max())
+    else:
+        assert torch.equal(a, b)
