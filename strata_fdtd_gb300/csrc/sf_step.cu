@@ -58,6 +58,7 @@ __global__ void __launch_bounds__(BX* BY) k_step(SfStepArgs a, SfSources src, Sf
     const int k = a.reg_lo[2] + blockIdx.x * BX + threadIdx.x;
     const int j = a.reg_lo[1] + blockIdx.y * BY + threadIdx.y;
     const int i = a.reg_lo[0] + blockIdx.z;
+    await_previous();
 
     // Probe values of the input state are the previous step's samples.
     if (a.trace_prev != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
@@ -187,6 +188,7 @@ __global__ void __launch_bounds__(BX* BY) k_step(SfStepArgs a, SfSources src, Sf
 // Walks only the box that holds every material cell.
 __global__ void k_ade_density(SfStepArgs a, SfPoles poles, long long n) {
     const int ey = a.ade_hi[1] - a.ade_lo[1], ez = a.ade_hi[2] - a.ade_lo[2];
+    await_previous();
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
          t += (long long)gridDim.x * blockDim.x) {
         const int i = a.ade_lo[0] + (int)(t / ((long long)ey * ez));
@@ -404,28 +406,30 @@ int sf_launch_step(const SfStepArgs& a, const SfSources& src, const SfPoles& pol
         const long long n = (long long)(a.ade_hi[0] - a.ade_lo[0]) * (a.ade_hi[1] - a.ade_lo[1]) *
                             (a.ade_hi[2] - a.ade_lo[2]);
         const int blocks = (int)((n + 255) / 256 < 152 * 16 ? (n + 255) / 256 : 152 * 16);
-        if (n > 0) k_ade_density<<<blocks, 256, 0, st>>>(a, poles, n);
+        if (n > 0 && launch_dependent(k_ade_density, dim3(blocks), dim3(256), st, a, poles, n) != cudaSuccess)
+            return sf_fail("k_ade_density launch failed");
     }
     const bool nu = a.nu_cv[0] != nullptr;
+    cudaError_t rc;
     if (nu) {
         if (geom)
-            ade ? k_step<true, true, true><<<grd, blk, 0, st>>>(a, src, poles)
-                : k_step<true, false, true><<<grd, blk, 0, st>>>(a, src, poles);
+            ade ? rc = launch_dependent(k_step<true, true, true>, grd, blk, st, a, src, poles)
+                : rc = launch_dependent(k_step<true, false, true>, grd, blk, st, a, src, poles);
         else
-            ade ? k_step<false, true, true><<<grd, blk, 0, st>>>(a, src, poles)
-                : k_step<false, false, true><<<grd, blk, 0, st>>>(a, src, poles);
+            ade ? rc = launch_dependent(k_step<false, true, true>, grd, blk, st, a, src, poles)
+                : rc = launch_dependent(k_step<false, false, true>, grd, blk, st, a, src, poles);
     } else if (geom) {
         if (ade)
-            k_step<true, true, false><<<grd, blk, 0, st>>>(a, src, poles);
+            rc = launch_dependent(k_step<true, true, false>, grd, blk, st, a, src, poles);
         else
-            k_step<true, false, false><<<grd, blk, 0, st>>>(a, src, poles);
+            rc = launch_dependent(k_step<true, false, false>, grd, blk, st, a, src, poles);
     } else {
         if (ade)
-            k_step<false, true, false><<<grd, blk, 0, st>>>(a, src, poles);
+            rc = launch_dependent(k_step<false, true, false>, grd, blk, st, a, src, poles);
         else
-            k_step<false, false, false><<<grd, blk, 0, st>>>(a, src, poles);
+            rc = launch_dependent(k_step<false, false, false>, grd, blk, st, a, src, poles);
     }
-    return cudaGetLastError() == cudaSuccess ? 0 : sf_fail("k_step launch failed");
+    return rc == cudaSuccess ? 0 : sf_fail("k_step launch failed");
 }
 
 int sf_launch_probe_gather(const float* p, const long long* cells, int n, float* out,

@@ -8,6 +8,9 @@
 // Blocks take i-chunks of ich planes, high to low on alternate steps (a step
 // starts on the planes the previous one wrote last, still in L2), and skip
 // the tile-aligned region a split ADE step leaves to the per-cell kernel.
+// A step is set up while the one before it drains (await_previous): 203 x 167 x
+// 181 with walls, 200 steps 8.01 -> 7.84 ms.  Their loads all follow a branch on
+// the thread's position behind that wait, so none can be issued before it.
 #include <cuda_runtime.h>
 
 #include <climits>
@@ -60,6 +63,7 @@ __global__ void __launch_bounds__(32 * W, MINB) k_step_tile(SfStepArgs a, SfSour
     const int chunk = a.reverse ? (int)(gridDim.z - 1 - blockIdx.z) : (int)blockIdx.z;
     const int i0 = chunk * ich;
     const int i1 = min(i0 + ich, a.nx);
+    await_previous();
     if (a.trace_prev != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
         for (int t = threadIdx.y * 32 + threadIdx.x; t < a.n_probe; t += 32 * W)
             a.trace_prev[t] = a.p[a.probe_cells[t]];
@@ -78,6 +82,7 @@ __global__ void __launch_bounds__(32 * W, MINB) k_step_tile1(SfStepArgs a, SfSou
     const int chunk = a.reverse ? (int)(gridDim.z - 1 - blockIdx.z) : (int)blockIdx.z;
     const int i0 = chunk * ich;
     const int i1 = min(i0 + ich, a.nx);
+    await_previous();
     if (a.trace_prev != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
         for (int t = threadIdx.y * 32 + threadIdx.x; t < a.n_probe; t += 32 * W)
             a.trace_prev[t] = a.p[a.probe_cells[t]];
@@ -91,14 +96,15 @@ template <int R, int W, int MINB, bool PF>
 int launch1(const SfStepArgs& a, const SfSources& src, bool geom, int ich, cudaStream_t st) {
     dim3 blk(32, W, 1);
     dim3 grd((a.nz + 31) / 32, (a.ny + R * W - 1) / (R * W), (a.nx + ich - 1) / ich);
+    cudaError_t rc;
     if (a.nu_cv[0] != nullptr) {
-        if (geom) k_step_tile1<true, R, W, MINB, PF, true><<<grd, blk, 0, st>>>(a, src, ich);
-        else k_step_tile1<false, R, W, MINB, PF, true><<<grd, blk, 0, st>>>(a, src, ich);
+        if (geom) rc = launch_dependent(k_step_tile1<true, R, W, MINB, PF, true>, grd, blk, st, a, src, ich);
+        else rc = launch_dependent(k_step_tile1<false, R, W, MINB, PF, true>, grd, blk, st, a, src, ich);
     } else {
-        if (geom) k_step_tile1<true, R, W, MINB, PF, false><<<grd, blk, 0, st>>>(a, src, ich);
-        else k_step_tile1<false, R, W, MINB, PF, false><<<grd, blk, 0, st>>>(a, src, ich);
+        if (geom) rc = launch_dependent(k_step_tile1<true, R, W, MINB, PF, false>, grd, blk, st, a, src, ich);
+        else rc = launch_dependent(k_step_tile1<false, R, W, MINB, PF, false>, grd, blk, st, a, src, ich);
     }
-    return cudaGetLastError() == cudaSuccess ? 0 : sf_fail("k_step_tile1 launch failed");
+    return rc == cudaSuccess ? 0 : sf_fail("k_step_tile1 launch failed");
 }
 
 template <int R, int W, int MINB, bool PF, bool WB = false>
@@ -106,14 +112,15 @@ int launch(const SfStepArgs& a, const SfSources& src, bool geom, int ich, cudaSt
     dim3 blk(32, W, 1);
     const int rows = 4 * R * W;
     dim3 grd((a.nz + 31) / 32, (a.ny + rows - 1) / rows, (a.nx + ich - 1) / ich);
+    cudaError_t rc;
     if (a.nu_cv[0] != nullptr) {
-        if (geom) k_step_tile<true, R, W, MINB, PF, true, WB><<<grd, blk, 0, st>>>(a, src, ich);
-        else k_step_tile<false, R, W, MINB, PF, true, WB><<<grd, blk, 0, st>>>(a, src, ich);
+        if (geom) rc = launch_dependent(k_step_tile<true, R, W, MINB, PF, true, WB>, grd, blk, st, a, src, ich);
+        else rc = launch_dependent(k_step_tile<false, R, W, MINB, PF, true, WB>, grd, blk, st, a, src, ich);
     } else {
-        if (geom) k_step_tile<true, R, W, MINB, PF, false, WB><<<grd, blk, 0, st>>>(a, src, ich);
-        else k_step_tile<false, R, W, MINB, PF, false, WB><<<grd, blk, 0, st>>>(a, src, ich);
+        if (geom) rc = launch_dependent(k_step_tile<true, R, W, MINB, PF, false, WB>, grd, blk, st, a, src, ich);
+        else rc = launch_dependent(k_step_tile<false, R, W, MINB, PF, false, WB>, grd, blk, st, a, src, ich);
     }
-    return cudaGetLastError() == cudaSuccess ? 0 : sf_fail("k_step_tile launch failed");
+    return rc == cudaSuccess ? 0 : sf_fail("k_step_tile launch failed");
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
