@@ -718,24 +718,6 @@ int launch_ade(sf_batch* B, cudaStream_t st, int trial) {
     return cudaGetLastError() == cudaSuccess ? 0 : sf_fail("k_batch_ade launch failed");
 }
 
-// A second stream for the ADE part, which runs beside the plain items (the two
-// read the same input set and write disjoint cells).
-struct SideBranch {
-    cudaStream_t side = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
-    int open() {
-        SF_CUDA_OK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
-        SF_CUDA_OK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
-        SF_CUDA_OK(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
-        return 0;
-    }
-    ~SideBranch() {
-        if (fork) cudaEventDestroy(fork);
-        if (join) cudaEventDestroy(join);
-        if (side) cudaStreamDestroy(side);
-    }
-};
-
 // One batch step: ADE part (on its own branch when there is one), plain
 // items, probes, advance.
 int enqueue_step(sf_batch* B, cudaStream_t st, const SideBranch* br = nullptr) {

@@ -66,6 +66,7 @@ struct SfStepArgs {
     int ade_lo[3], ade_hi[3];         // box holding every material cell
     int reg_lo[3], reg_hi[3];         // per-cell kernel: the cells it updates
     int skip_lo[3], skip_hi[3];       // warp-tile kernels: tile-aligned cells they leave out
+    int serial;                       // host: launched without programmatic serialization
     const float* nu_cv[3];            // nonuniform grid: face coefficients per axis, or null
     const float* nu_inv[3];           // nonuniform grid: cell inverse spacings per axis
 };
@@ -90,7 +91,8 @@ __device__ __forceinline__ void await_previous(P&... pointers) {
     (launder(pointers), ...);
 }
 template <class... P, class... A>
-inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
+inline cudaError_t launch_kernel(bool dependent, void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st,
+                                 A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -99,8 +101,12 @@ inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block,
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = dependent ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <class... P, class... A>
+inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
+    return launch_kernel(true, kernel, grid, block, st, args...);
 }
 
 #define SF_CUDA_OK(expr)                                                   \

@@ -6,6 +6,24 @@
 #include "sf_common.cuh"
 #include "sf_kernels.h"
 
+// A second stream for the ADE part of a step, which runs beside the plain part
+// (the two read the same input set and write disjoint cells).
+struct SideBranch {
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+    int open() {
+        SF_CUDA_OK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+        SF_CUDA_OK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+        SF_CUDA_OK(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
+        return 0;
+    }
+    ~SideBranch() {
+        if (fork) cudaEventDestroy(fork);
+        if (join) cudaEventDestroy(join);
+        if (side) cudaStreamDestroy(side);
+    }
+};
+
 struct sf_plan {
     sf_grid_desc d{};
     long long n = 0;

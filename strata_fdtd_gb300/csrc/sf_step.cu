@@ -406,7 +406,7 @@ int sf_launch_step(const SfStepArgs& a, const SfSources& src, const SfPoles& pol
         const long long n = (long long)(a.ade_hi[0] - a.ade_lo[0]) * (a.ade_hi[1] - a.ade_lo[1]) *
                             (a.ade_hi[2] - a.ade_lo[2]);
         const int blocks = (int)((n + 255) / 256 < 152 * 16 ? (n + 255) / 256 : 152 * 16);
-        if (n > 0 && launch_dependent(k_ade_density, dim3(blocks), dim3(256), st, a, poles, n) != cudaSuccess)
+        if (n > 0 && launch_kernel(!a.serial, k_ade_density, dim3(blocks), dim3(256), st, a, poles, n) != cudaSuccess)
             return sf_fail("k_ade_density launch failed");
     }
     const bool nu = a.nu_cv[0] != nullptr;

@@ -98,11 +98,11 @@ int launch1(const SfStepArgs& a, const SfSources& src, bool geom, int ich, cudaS
     dim3 grd((a.nz + 31) / 32, (a.ny + R * W - 1) / (R * W), (a.nx + ich - 1) / ich);
     cudaError_t rc;
     if (a.nu_cv[0] != nullptr) {
-        if (geom) rc = launch_dependent(k_step_tile1<true, R, W, MINB, PF, true>, grd, blk, st, a, src, ich);
-        else rc = launch_dependent(k_step_tile1<false, R, W, MINB, PF, true>, grd, blk, st, a, src, ich);
+        if (geom) rc = launch_kernel(!a.serial, k_step_tile1<true, R, W, MINB, PF, true>, grd, blk, st, a, src, ich);
+        else rc = launch_kernel(!a.serial, k_step_tile1<false, R, W, MINB, PF, true>, grd, blk, st, a, src, ich);
     } else {
-        if (geom) rc = launch_dependent(k_step_tile1<true, R, W, MINB, PF, false>, grd, blk, st, a, src, ich);
-        else rc = launch_dependent(k_step_tile1<false, R, W, MINB, PF, false>, grd, blk, st, a, src, ich);
+        if (geom) rc = launch_kernel(!a.serial, k_step_tile1<true, R, W, MINB, PF, false>, grd, blk, st, a, src, ich);
+        else rc = launch_kernel(!a.serial, k_step_tile1<false, R, W, MINB, PF, false>, grd, blk, st, a, src, ich);
     }
     return rc == cudaSuccess ? 0 : sf_fail("k_step_tile1 launch failed");
 }
@@ -114,11 +114,11 @@ int launch(const SfStepArgs& a, const SfSources& src, bool geom, int ich, cudaSt
     dim3 grd((a.nz + 31) / 32, (a.ny + rows - 1) / rows, (a.nx + ich - 1) / ich);
     cudaError_t rc;
     if (a.nu_cv[0] != nullptr) {
-        if (geom) rc = launch_dependent(k_step_tile<true, R, W, MINB, PF, true, WB>, grd, blk, st, a, src, ich);
-        else rc = launch_dependent(k_step_tile<false, R, W, MINB, PF, true, WB>, grd, blk, st, a, src, ich);
+        if (geom) rc = launch_kernel(!a.serial, k_step_tile<true, R, W, MINB, PF, true, WB>, grd, blk, st, a, src, ich);
+        else rc = launch_kernel(!a.serial, k_step_tile<false, R, W, MINB, PF, true, WB>, grd, blk, st, a, src, ich);
     } else {
-        if (geom) rc = launch_dependent(k_step_tile<true, R, W, MINB, PF, false, WB>, grd, blk, st, a, src, ich);
-        else rc = launch_dependent(k_step_tile<false, R, W, MINB, PF, false, WB>, grd, blk, st, a, src, ich);
+        if (geom) rc = launch_kernel(!a.serial, k_step_tile<true, R, W, MINB, PF, false, WB>, grd, blk, st, a, src, ich);
+        else rc = launch_kernel(!a.serial, k_step_tile<false, R, W, MINB, PF, false, WB>, grd, blk, st, a, src, ich);
     }
     return rc == cudaSuccess ? 0 : sf_fail("k_step_tile launch failed");
 }
