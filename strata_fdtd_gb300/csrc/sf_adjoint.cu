@@ -286,13 +286,19 @@ __global__ void __launch_bounds__(256, (kFwdMinBlocks<T, I>)) k_dfwd(DiffPtrs<T>
 // instructions (dw2, sf_dw.cuh): half the issue slots per operation, one load for
 // both cells where rows are 16-byte aligned, and the face between the two formed
 // once (the per-cell kernels issue 619 and 1075 instructions per cell).
-// Bit-identical to the per-cell kernels.  What is left is memory latency, so
-// resident warps count: at 128^3 the forward takes 46.7 us with 3 blocks per SM
-// (70 registers), 42.3 with 4, 39.7 with 5 (48 registers), 40.8 with 6; the
-// adjoint 87.1 with 2, 70.5 with 3, 69.2 with 4.  Per cell, planes in alternate
-// order: 45.6 and 73.3; in one order 49.7 and 77.3.  Measured slower: blocks that
-// walk planes and share faces through shared memory (57.9 to 67.1 and 112 to
-// 125), threads that carry the x face and p over 2 or 4 planes (42.7 to 50.1).
+// Bit-identical to the per-cell kernels.  What is left is memory latency: with a
+// branch at each grid edge a thread waited for its loads up to six times in turn
+// (8 of 16 stall cycles per issue, DRAM at half its rate).  So an index past the
+// grid reads the cell itself, the result is dropped by a select, and no branch
+// stands between the loads of the high faces, nor between those of the low ones;
+// and a warp leaves out the decays that are one along i and j (pair_decays).  At
+// 128^3 a gradient of 200 steps takes 27.8 ms with 4 blocks per SM (64 registers),
+// 27.8 with 3, 28.7 to 29.0 with every load first (spills), 32.0 with 5; with
+// branches 30.8 (5 and 4 blocks).  The per-cell kernels gain nothing from it (75 x
+// 66 x 61 in FP32: 3.19 ms against 3.17).  Planes in alternate order save 4 of 50
+// and 77 us of a forward and an adjoint step.  Measured slower: blocks that walk
+// planes and share faces through shared memory (57.9 to 67.1 and 112 to 125 us),
+// threads that carry the x face and p over 2 or 4 planes (42.7 to 50.1).
 
 // ALIGNED: nz is even and the arrays are 16-byte aligned, so that a pair is one
 // access and always whole.
@@ -323,7 +329,17 @@ __device__ __forceinline__ dw2 pick(bool c0, bool c1, dw2 a, dw2 b) {
     return join(c0 ? first(a) : first(b), c1 ? second(a) : second(b));
 }
 
-template <bool UNIT, bool ALIGNED>
+// Which decays a warp's cells and their neighbours have to apply: all, those along
+// k only, none.  A factor of exactly one is left out (sf_dw::is_one); a warp spans
+// 64 cells of k, so that on most grids it meets an absorbing layer there.
+enum { kDecayAll, kDecayK, kDecayNone };
+__device__ __forceinline__ int pair_decays(const DiffPtrs<dwf>& g, int i, int j) {
+    if (i < g.unit_lo[0] || i >= g.unit_hi[0] || j < g.unit_lo[1] || j >= g.unit_hi[1]) return kDecayAll;
+    const int k0 = blockIdx.x * 64, k1 = min(k0 + 64, g.nz) - 1;
+    return k0 >= g.unit_lo[2] && k1 < g.unit_hi[2] ? kDecayNone : kDecayK;
+}
+
+template <int DECAY, bool ALIGNED>
 __device__ __forceinline__ void dfwd_pair(const DiffPtrs<dwf>& g, int i, int j, int k, const dwf* __restrict__ p,
                                           const dwf* __restrict__ vx, const dwf* __restrict__ vy,
                                           const dwf* __restrict__ vz, dwf* __restrict__ po,
@@ -336,31 +352,37 @@ __device__ __forceinline__ void dfwd_pair(const DiffPtrs<dwf>& g, int i, int j, 
     const int plane = (int)g.plane, nz = g.nz;
     const int c = i * plane + j * nz + k;
     const bool two = ALIGNED || k + 1 < nz;
+    // past the grid: the cell itself, dropped below (no branch between the loads)
+    const bool hx = i < g.nx - 1, hy = j < g.ny - 1;
+    const int cxp = hx ? c + plane : c, cyp = hy ? c + nz : c;
+    const int cxm = i > 0 ? c - plane : c, cym = j > 0 ? c - nz : c, czm = k > 0 ? c - 1 : c;
     const dw2 pc = ld2<ALIGNED>(p, c, two);
+    const dw2 vx0 = ld2<ALIGNED>(vx, c, two), vy0 = ld2<ALIGNED>(vy, c, two), vz0 = ld2<ALIGNED>(vz, c, two);
+    const dw2 pxp = ld2<ALIGNED>(p, cxp, two), pyp = ld2<ALIGNED>(p, cyp, two);
+    const dwf pzp = p[k + 2 < nz ? c + 2 : c];
+    const dw2 ax = ld2<ALIGNED>(g.cvx, c, two), ay = ld2<ALIGNED>(g.cvy, c, two), az = ld2<ALIGNED>(g.cvz, c, two);
     if (p_store) st2<ALIGNED>(p_store, c, two, pc);
-    dw2 ux = ld2<ALIGNED>(vx, c, two), uy = ld2<ALIGNED>(vy, c, two), uz = ld2<ALIGNED>(vz, c, two);
-    if (i < g.nx - 1) ux = ux + ld2<ALIGNED>(g.cvx, c, two) * (ld2<ALIGNED>(p, c + plane, two) - pc);
-    if (j < g.ny - 1) uy = uy + ld2<ALIGNED>(g.cvy, c, two) * (ld2<ALIGNED>(p, c + nz, two) - pc);
-    {
-        const dw2 up = join(second(pc), k + 2 < nz ? p[c + 2] : dwf(0));
-        uz = pick(k < nz - 1, k + 1 < nz - 1, uz + ld2<ALIGNED>(g.cvz, c, two) * (up - pc), uz);
-    }
-    dw2 uxm = zero2(), uym = zero2();
-    if (i > 0)
-        uxm = ld2<ALIGNED>(vx, c - plane, two) +
-              ld2<ALIGNED>(g.cvx, c - plane, two) * (pc - ld2<ALIGNED>(p, c - plane, two));
-    if (j > 0)
-        uym = ld2<ALIGNED>(vy, c - nz, two) + ld2<ALIGNED>(g.cvy, c - nz, two) * (pc - ld2<ALIGNED>(p, c - nz, two));
-    dwf low(0);
-    if (k > 0) low = vz[c - 1] + g.cvz[c - 1] * (first(pc) - p[c - 1]);
-    const dw2 uzm = join(low, first(uz));
+    dw2 ux = pick(hx, hx, vx0 + ax * (pxp - pc), vx0);
+    dw2 uy = pick(hy, hy, vy0 + ay * (pyp - pc), vy0);
+    dw2 uz = pick(k < nz - 1, k + 1 < nz - 1, vz0 + az * (join(second(pc), pzp) - pc), vz0);
+    const dw2 pxm = ld2<ALIGNED>(p, cxm, two), vxm = ld2<ALIGNED>(vx, cxm, two), axm = ld2<ALIGNED>(g.cvx, cxm, two);
+    const dw2 pym = ld2<ALIGNED>(p, cym, two), vym = ld2<ALIGNED>(vy, cym, two), aym = ld2<ALIGNED>(g.cvy, cym, two);
+    const dwf pzm = p[czm], vzm = vz[czm], azm = g.cvz[czm];
+    const dw2 uxm = pick(i > 0, i > 0, vxm + axm * (pc - pxm), zero2());
+    const dw2 uym = pick(j > 0, j > 0, vym + aym * (pc - pym), zero2());
+    const dwf low = vzm + azm * (first(pc) - pzm);
+    const dw2 uzm = join(k > 0 ? low : dwf(0), first(uz));
     dw2 pn = pc + both(g.cp) * (((ux - uxm) + (uy - uym)) + (uz - uzm));
-    if constexpr (!UNIT) {
-        const dw2 di = both(g.dx[i]), dj = both(g.dy[j]), dk = join(g.dz[k], two ? g.dz[k + 1] : dwf(0));
+    if constexpr (DECAY == kDecayAll) {
+        const dw2 di = both(g.dx[i]), dj = both(g.dy[j]);
         ux = ux * di;
         uy = uy * dj;
+        pn = (pn * di) * dj;
+    }
+    if constexpr (DECAY != kDecayNone) {
+        const dw2 dk = join(g.dz[k], two ? g.dz[k + 1] : dwf(0));
         uz = uz * dk;
-        pn = ((pn * di) * dj) * dk;
+        pn = pn * dk;
     }
     st2<ALIGNED>(vxo, c, two, ux);
     st2<ALIGNED>(vyo, c, two, uy);
@@ -375,16 +397,8 @@ __device__ __forceinline__ void dfwd_pair(const DiffPtrs<dwf>& g, int i, int j, 
     }
 }
 
-// Whether the block's cells (64 k x 8 j) and their neighbours have unit decays.
-__device__ __forceinline__ bool pair_block_unit(const DiffPtrs<dwf>& g, int i) {
-    const int j0 = blockIdx.y * 8, k0 = blockIdx.x * 64;
-    const int j1 = min(j0 + 8, g.ny) - 1, k1 = min(k0 + 64, g.nz) - 1;
-    return i >= g.unit_lo[0] && i < g.unit_hi[0] && j0 >= g.unit_lo[1] && j1 < g.unit_hi[1] &&
-           k0 >= g.unit_lo[2] && k1 < g.unit_hi[2];
-}
-
 template <bool ALIGNED>
-__global__ void __launch_bounds__(256, 5)
+__global__ void __launch_bounds__(256, 4)
     k_dfwd_pair(DiffPtrs<dwf> g, const dwf* __restrict__ p, const dwf* __restrict__ vx,
                 const dwf* __restrict__ vy, const dwf* __restrict__ vz, dwf* __restrict__ po,
                 dwf* __restrict__ vxo, dwf* __restrict__ vyo, dwf* __restrict__ vzo, long long src_cell,
@@ -396,12 +410,16 @@ __global__ void __launch_bounds__(256, 5)
     const int i = reverse ? (int)(gridDim.z - 1 - blockIdx.z) : (int)blockIdx.z;
     await_previous(p, vx, vy, vz, po, vxo, vyo, vzo, src_val, p_store, probe_cells, trace_row);
     if (k >= g.nz || j >= g.ny) return;
-    if (pair_block_unit(g, i))
-        dfwd_pair<true, ALIGNED>(g, i, j, k, p, vx, vy, vz, po, vxo, vyo, vzo, src_cell, src_val, p_store,
+    const int decays = pair_decays(g, i, j);
+    if (decays == kDecayK)
+        dfwd_pair<kDecayK, ALIGNED>(g, i, j, k, p, vx, vy, vz, po, vxo, vyo, vzo, src_cell, src_val, p_store,
+                                 probe_cells, n_fused, trace_row);
+    else if (decays == kDecayNone)
+        dfwd_pair<kDecayNone, ALIGNED>(g, i, j, k, p, vx, vy, vz, po, vxo, vyo, vzo, src_cell, src_val, p_store,
                                  probe_cells, n_fused, trace_row);
     else
-        dfwd_pair<false, ALIGNED>(g, i, j, k, p, vx, vy, vz, po, vxo, vyo, vzo, src_cell, src_val, p_store,
-                                  probe_cells, n_fused, trace_row);
+        dfwd_pair<kDecayAll, ALIGNED>(g, i, j, k, p, vx, vy, vz, po, vxo, vyo, vzo, src_cell, src_val, p_store,
+                                 probe_cells, n_fused, trace_row);
 }
 
 // What the adjoint of a step adds to the lambda_p it writes: the loss gradient
@@ -439,7 +457,7 @@ __device__ __forceinline__ void grad2(double* g, int c, bool two, bool c0, bool 
     st2<ALIGNED>(f, c, two, pick(c0, c1, sf_dw::add(x, a * b), x));
 }
 
-template <bool UNIT, bool ALIGNED>
+template <int DECAY, bool ALIGNED>
 __device__ __forceinline__ void dadj_pair(const DiffPtrs<dwf>& g, int i, int j, int k, const dwf* __restrict__ lp,
                                           const dwf* __restrict__ lx, const dwf* __restrict__ ly,
                                           const dwf* __restrict__ lz, dwf* __restrict__ lpo,
@@ -453,65 +471,66 @@ __device__ __forceinline__ void dadj_pair(const DiffPtrs<dwf>& g, int i, int j, 
     const bool two = ALIGNED || k + 1 < nz;
     const bool z0 = k < nz - 1, z1 = k + 1 < nz - 1;  // the cells' high z faces exist
     const dw2 cp = both(g.cp);
-    const dw2 dk = UNIT ? zero2() : join(g.dz[k], two ? g.dz[k + 1] : dwf(0));
-    auto mup2 = [&](int ii, int jj, int q) -> dw2 {
-        const dw2 v = ld2<ALIGNED>(lp, q, two);
-        if constexpr (UNIT) return v;
+    const dw2 dk = DECAY == kDecayNone ? zero2() : join(g.dz[k], two ? g.dz[k + 1] : dwf(0));
+    // past the grid: the cell itself, dropped below (no branch between the loads)
+    const bool hx = i < nx - 1, hy = j < ny - 1;
+    const int cxp = hx ? c + plane : c, cyp = hy ? c + nz : c, czp = z1 ? c + 2 : c;
+    const int cxm = i > 0 ? c - plane : c, cym = j > 0 ? c - nz : c, czm = k > 0 ? c - 1 : c;
+    const int ip = hx ? i + 1 : i, jp = hy ? j + 1 : j, im = i > 0 ? i - 1 : i, jm = j > 0 ? j - 1 : j;
+    const int km = k > 0 ? k - 1 : k, kp = z1 ? k + 2 : k;
+    auto mup2 = [&](int ii, int jj, dw2 v) -> dw2 {
+        if constexpr (DECAY == kDecayNone) return v;
+        else if constexpr (DECAY == kDecayK) return dk * v;
         else return both(g.dx[ii] * g.dy[jj]) * dk * v;
     };
-    auto mup1 = [&](int kk, int q) -> dwf {
-        if constexpr (UNIT) return lp[q];
-        else return g.dx[i] * g.dy[j] * g.dz[kk] * lp[q];
+    auto mup1 = [&](int kk, dwf v) -> dwf {
+        if constexpr (DECAY == kDecayNone) return v;
+        else if constexpr (DECAY == kDecayK) return g.dz[kk] * v;
+        else return g.dx[i] * g.dy[j] * g.dz[kk] * v;
     };
-    auto dec = [&](dw2 v, const dwf& d) -> dw2 {
-        if constexpr (UNIT) return v;
-        else return both(d) * v;
+    auto dec = [&](dw2 v, const dwf* d) -> dw2 {
+        if constexpr (DECAY != kDecayAll) return v;
+        else return both(*d) * v;
     };
-    const dw2 m0 = mup2(i, j, c);
-    const dw2 mxp = i < nx - 1 ? mup2(i + 1, j, c + plane) : zero2();
-    const dw2 myp = j < ny - 1 ? mup2(i, j + 1, c + nz) : zero2();
-    const dw2 mzp = join(z0 ? second(m0) : dwf(0), z1 ? mup1(k + 2, c + 2) : dwf(0));
-    const dw2 vx_hi = dec(ld2<ALIGNED>(lx, c, two), g.dx[i]) + cp * (m0 - mxp);
-    const dw2 vy_hi = dec(ld2<ALIGNED>(ly, c, two), g.dy[j]) + cp * (m0 - myp);
-    dw2 zl = ld2<ALIGNED>(lz, c, two);
-    if constexpr (!UNIT) zl = dk * zl;
+    const dw2 l0 = ld2<ALIGNED>(lp, c, two), lxp = ld2<ALIGNED>(lp, cxp, two), lyp = ld2<ALIGNED>(lp, cyp, two);
+    const dwf lzp = lp[czp];
+    const dw2 lx0 = ld2<ALIGNED>(lx, c, two), ly0 = ld2<ALIGNED>(ly, c, two), lz0 = ld2<ALIGNED>(lz, c, two);
+    const dw2 m0 = mup2(i, j, l0);
+    const dw2 mxp = pick(hx, hx, mup2(ip, j, lxp), zero2()), myp = pick(hy, hy, mup2(i, jp, lyp), zero2());
+    const dw2 mzp = join(z0 ? second(m0) : dwf(0), z1 ? mup1(kp, lzp) : dwf(0));
+    const dw2 vx_hi = dec(lx0, g.dx + i) + cp * (m0 - mxp);
+    const dw2 vy_hi = dec(ly0, g.dy + j) + cp * (m0 - myp);
+    dw2 zl = lz0;
+    if constexpr (DECAY != kDecayNone) zl = dk * zl;
     const dw2 vz_hi = zl + cp * (m0 - mzp);
     st2<ALIGNED>(lxo, c, two, vx_hi);
     st2<ALIGNED>(lyo, c, two, vy_hi);
     st2<ALIGNED>(lzo, c, two, vz_hi);
+    const dw2 lxm = ld2<ALIGNED>(lp, cxm, two), vxm = ld2<ALIGNED>(lx, cxm, two), axm = ld2<ALIGNED>(g.cvx, cxm, two);
+    const dw2 lym = ld2<ALIGNED>(lp, cym, two), vym = ld2<ALIGNED>(ly, cym, two), aym = ld2<ALIGNED>(g.cvy, cym, two);
     dw2 acc = m0;
-    if (i > 0) {
-        const dw2 v = dec(ld2<ALIGNED>(lx, c - plane, two), UNIT ? dwf(1) : g.dx[i - 1]) +
-                      cp * (mup2(i - 1, j, c - plane) - m0);
-        acc = acc + ld2<ALIGNED>(g.cvx, c - plane, two) * v;
-    }
-    if (j > 0) {
-        const dw2 v = dec(ld2<ALIGNED>(ly, c - nz, two), UNIT ? dwf(1) : g.dy[j - 1]) +
-                      cp * (mup2(i, j - 1, c - nz) - m0);
-        acc = acc + ld2<ALIGNED>(g.cvy, c - nz, two) * v;
-    }
-    const dw2 cz = ld2<ALIGNED>(g.cvz, c, two);
+    acc = pick(i > 0, i > 0, acc + axm * (dec(vxm, g.dx + im) + cp * (mup2(im, j, lxm) - m0)), acc);
+    acc = pick(j > 0, j > 0, acc + aym * (dec(vym, g.dy + jm) + cp * (mup2(i, jm, lym) - m0)), acc);
+    const dwf lzm = lp[czm], vzm = lz[czm], azm = g.cvz[czm];
+    const dw2 ax = ld2<ALIGNED>(g.cvx, c, two), ay = ld2<ALIGNED>(g.cvy, c, two), az = ld2<ALIGNED>(g.cvz, c, two);
     {
-        dwf v(0), w(0);
-        if (k > 0) {
-            dwf l = lz[c - 1];
-            if constexpr (!UNIT) l = g.dz[k - 1] * l;
-            v = l + g.cp * (mup1(k - 1, c - 1) - first(m0));
-            w = g.cvz[c - 1];
-        }
-        acc = pick(k > 0, true, acc + join(w, first(cz)) * join(v, first(vz_hi)), acc);
+        dwf l = vzm;
+        if constexpr (DECAY != kDecayNone) l = g.dz[km] * l;
+        const dwf v = l + g.cp * (mup1(km, lzm) - first(m0));
+        acc = pick(k > 0, true, acc + join(azm, first(az)) * join(v, first(vz_hi)), acc);
     }
-    acc = acc - (ld2<ALIGNED>(g.cvx, c, two) * vx_hi + ld2<ALIGNED>(g.cvy, c, two) * vy_hi + cz * vz_hi);
+    acc = acc - (ax * vx_hi + ay * vy_hi + az * vz_hi);
     for (int q = 0; q < inj.n; ++q)  // (rare)
         if (inj.cells[q] == c || inj.cells[q] == c + 1) {
             acc = join(inj.at(c, first(acc)), inj.at(c + 1, second(acc)));
             break;
         }
     st2<ALIGNED>(lpo, c, two, acc);
-    const dw2 p0 = ld2<ALIGNED>(pst, c, two);
-    if (i < nx - 1) grad2<ALIGNED>(gx, c, two, true, true, vx_hi, ld2<ALIGNED>(pst, c + plane, two) - p0);
-    if (j < ny - 1) grad2<ALIGNED>(gy, c, two, true, true, vy_hi, ld2<ALIGNED>(pst, c + nz, two) - p0);
-    if (z0) grad2<ALIGNED>(gz, c, two, true, z1, vz_hi, join(second(p0), z1 ? pst[c + 2] : dwf(0)) - p0);
+    const dw2 p0 = ld2<ALIGNED>(pst, c, two), pxp = ld2<ALIGNED>(pst, cxp, two), pyp = ld2<ALIGNED>(pst, cyp, two);
+    const dwf pzp = pst[czp];
+    if (hx) grad2<ALIGNED>(gx, c, two, true, true, vx_hi, pxp - p0);
+    if (hy) grad2<ALIGNED>(gy, c, two, true, true, vy_hi, pyp - p0);
+    if (z0) grad2<ALIGNED>(gz, c, two, true, z1, vz_hi, join(second(p0), z1 ? pzp : dwf(0)) - p0);
 }
 
 template <bool ALIGNED>
@@ -526,10 +545,13 @@ __global__ void __launch_bounds__(256, 4)
     const int i = reverse ? (int)(gridDim.z - 1 - blockIdx.z) : (int)blockIdx.z;
     await_previous(lp, lx, ly, lz, lpo, lxo, lyo, lzo, pst, gx, gy, gz);
     if (k >= g.nz || j >= g.ny) return;
-    if (pair_block_unit(g, i))
-        dadj_pair<true, ALIGNED>(g, i, j, k, lp, lx, ly, lz, lpo, lxo, lyo, lzo, pst, gx, gy, gz, inj);
+    const int decays = pair_decays(g, i, j);
+    if (decays == kDecayK)
+        dadj_pair<kDecayK, ALIGNED>(g, i, j, k, lp, lx, ly, lz, lpo, lxo, lyo, lzo, pst, gx, gy, gz, inj);
+    else if (decays == kDecayNone)
+        dadj_pair<kDecayNone, ALIGNED>(g, i, j, k, lp, lx, ly, lz, lpo, lxo, lyo, lzo, pst, gx, gy, gz, inj);
     else
-        dadj_pair<false, ALIGNED>(g, i, j, k, lp, lx, ly, lz, lpo, lxo, lyo, lzo, pst, gx, gy, gz, inj);
+        dadj_pair<kDecayAll, ALIGNED>(g, i, j, k, lp, lx, ly, lz, lpo, lxo, lyo, lzo, pst, gx, gy, gz, inj);
 }
 
 template <typename T, typename E = typename Ext<T>::E>

@@ -8,7 +8,8 @@ pytestmark = pytest.mark.gpu
 import strata_fdtd_gb300 as S  # noqa: E402
 
 
-@pytest.mark.parametrize("shape", [(6, 5, 4), (9, 8, 33), (12, 17, 66), (11, 9, 127), (5, 9, 1), (7, 3, 64)])
+@pytest.mark.parametrize("shape", [(6, 5, 4), (9, 8, 33), (12, 17, 66), (11, 9, 127), (5, 9, 1), (7, 3, 64),
+                                   (8, 11, 201), (8, 11, 200)])
 def test_double_word_pairs_match_fp64_on_odd_rows(shape):
     """Two cells per thread, whole and half pairs, 16-byte and 8-byte rows: the
     double-word trace, loss and both gradients against the FP64 kernels."""
