@@ -12,7 +12,10 @@ Gradients come from hand-written reverse-time adjoint kernels
 ``torch.autograd.Function``.  The forward keeps a state checkpoint every K
 steps; the backward recomputes each K-step segment from its checkpoint
 (storing that segment's pressures) and runs the adjoint back through it, so
-memory is O(N * (steps/K + K)) instead of O(N * steps).
+memory is O(N * (steps/K + K)) instead of O(N * steps).  The last segment's
+pressures are stored by the forward pass itself, which saves their
+recomputation: a gradient of 200 steps at 128^3 in segments of 100, 24.0 ms
+against 27.7.
 """
 from __future__ import annotations
 
@@ -217,6 +220,31 @@ class DifferentiableSolver:
     def forward(self, theta, n_steps, keep_checkpoints=True, occupancy=None):
         """Run n_steps from rest.  Returns (trace [n, n_probe], checkpoints,
         face coefficients, source values)."""
+        return self._forward(theta, n_steps, keep_checkpoints, occupancy, None)
+
+    # Largest buffer kept from a forward pass to its backward pass: a sixteenth
+    # of the device memory, as several losses may be waiting for theirs.
+    _STORE_FRACTION = 1 / 16
+
+    def _segment_store(self):
+        """Room for the pressures of one segment."""
+        return self.torch.empty((self.K,) + self.shape, dtype=self.dtype, device=self.dev)
+
+    def _last_segment_store(self):
+        """Room for the last segment's pressures, which a forward pass that has a
+        backward pass to come writes as it goes: the adjoint starts from them
+        without recomputing that segment and then uses it for the others.  None
+        where it would be too large to keep."""
+        total = self.torch.cuda.get_device_properties(self.dev).total_memory
+        if self.K * self.n * self.dtype.itemsize > self._STORE_FRACTION * total:
+            return None
+        try:
+            return self._segment_store()
+        except self.torch.cuda.OutOfMemoryError:
+            return None
+
+    def _forward(self, theta, n_steps, keep_checkpoints, occupancy, store):
+        """forward(); the last segment's pressures go to ``store``, if given."""
         torch = self.torch
         theta = theta.to(self.ext_dtype).contiguous()
         cv = self.coefficients(theta, occupancy)
@@ -233,8 +261,9 @@ class DifferentiableSolver:
                 ckpts.append([t.clone() for t in sets[cur]])
             _native.check(self.lib.sf_diff_forward(
                 ctypes.byref(desc), _ptrs(cv), _ptrs(sets[0]), _ptrs(sets[1]), cur, n,
-                src[s0:].data_ptr(), trace[s0:].data_ptr(), None, self._stream()),
-                "sf_diff_forward")
+                src[s0:].data_ptr(), trace[s0:].data_ptr(),
+                store.data_ptr() if store is not None and s0 + n == n_steps else None,
+                self._stream()), "sf_diff_forward")
             cur = (cur + n) & 1
         return trace[:, :len(self.probe_pos)], ckpts, cv, src
 
@@ -242,6 +271,11 @@ class DifferentiableSolver:
         """dL/dtheta of L = weight * sum((trace - target)^2) by checkpointed
         recomputation and the reverse-time adjoint; with an occupancy field,
         (dL/dtheta, dL/dphi)."""
+        return self._gradient(theta, trace, target, ckpts, cv, src, weight, occupancy, None)
+
+    def _gradient(self, theta, trace, target, ckpts, cv, src, weight, occupancy, last):
+        """gradient(); ``last``: the last segment's pressures, if the forward pass
+        kept them (overwritten: the earlier segments' come after them)."""
         torch = self.torch
         n_steps = trace.shape[0]
         theta = theta.to(self.ext_dtype).contiguous()
@@ -256,15 +290,16 @@ class DifferentiableSolver:
         # or for an FP32 or double-word solve a double-word float pair), zero-filled
         grad_cv = [torch.zeros(self.shape, dtype=torch.float64, device=self.dev) for _ in range(3)]
         desc = self._desc()
-        store = torch.empty((self.K,) + self.shape, dtype=self.dtype, device=self.dev)
+        store = self._segment_store() if last is None else last
         seg_starts = list(range(0, n_steps, self.K))
         for si in reversed(range(len(seg_starts))):
             s0 = seg_starts[si]
             n = min(self.K, n_steps - s0)
-            work = [[t.clone() for t in ckpts[si]], self._zeros4()]
-            _native.check(self.lib.sf_diff_forward(
-                ctypes.byref(desc), _ptrs(cv), _ptrs(work[0]), _ptrs(work[1]), 0, n,
-                src[s0:].data_ptr(), None, store.data_ptr(), self._stream()), "sf_diff_forward")
+            if last is None or s0 + n < n_steps:
+                work = [[t.clone() for t in ckpts[si]], self._zeros4()]
+                _native.check(self.lib.sf_diff_forward(
+                    ctypes.byref(desc), _ptrs(cv), _ptrs(work[0]), _ptrs(work[1]), 0, n,
+                    src[s0:].data_ptr(), None, store.data_ptr(), self._stream()), "sf_diff_forward")
             _native.check(self.lib.sf_diff_adjoint(
                 ctypes.byref(desc), _ptrs(cv), _ptrs(lam[0]), _ptrs(lam[1]), lcur, n,
                 store.data_ptr(), full[s0:].data_ptr(), tgt[s0:].data_ptr(), float(weight),
@@ -292,12 +327,14 @@ def _make_function():
         """loss = sum((trace(theta) - target)^2); backward via the adjoint."""
 
         @staticmethod
-        def forward(ctx, theta, target, solver, n_steps, occupancy=None):
+        def forward(ctx, theta, target, solver, n_steps, occupancy, keep):
             occ = None if occupancy is None else occupancy.detach()
-            trace, ckpts, cv, src = solver.forward(theta.detach(), n_steps, occupancy=occ)
+            last = solver._last_segment_store() if keep and any(ctx.needs_input_grad) else None
+            trace, ckpts, cv, src = solver._forward(theta.detach(), n_steps, True, occ, last)
             loss = ((trace - target.to(trace.dtype)) ** 2).sum()
             ctx.solver = solver
             ctx.saved = (trace, ckpts, cv, src)
+            ctx.last = last
             ctx.save_for_backward(theta, target, occupancy)
             return loss.to(theta.dtype)
 
@@ -305,12 +342,13 @@ def _make_function():
         def backward(ctx, grad_out):
             theta, target, occupancy = ctx.saved_tensors
             trace, ckpts, cv, src = ctx.saved
-            g = ctx.solver.gradient(theta.detach(), trace, target, ckpts, cv, src,
-                                    weight=float(grad_out),
-                                    occupancy=None if occupancy is None else occupancy.detach())
+            last, ctx.last = ctx.last, None  # for one backward pass; another recomputes
+            g = ctx.solver._gradient(theta.detach(), trace, target, ckpts, cv, src,
+                                     float(grad_out),
+                                     None if occupancy is None else occupancy.detach(), last)
             if occupancy is None:
-                return g.to(theta.dtype), None, None, None, None
-            return g[0].to(theta.dtype), None, None, None, g[1].to(occupancy.dtype)
+                return g.to(theta.dtype), None, None, None, None, None
+            return g[0].to(theta.dtype), None, None, None, g[1].to(occupancy.dtype), None
 
     return ProbeLossFn
 
@@ -319,10 +357,11 @@ class _Lazy:
     fn = None
 
     @classmethod
-    def apply(cls, *a):
+    def apply(cls, theta, target, solver, n_steps, occupancy=None):
         if cls.fn is None:
             cls.fn = _make_function()
-        return cls.fn.apply(*a)
+        keep = n_steps > 0 and solver.torch.is_grad_enabled()  # a backward pass may come
+        return cls.fn.apply(theta, target, solver, n_steps, occupancy, keep)
 
 
 ProbeLoss = _Lazy
