@@ -57,6 +57,13 @@ namespace {
 constexpr int VX_DSTACK = 32;
 constexpr int VX_PSTACK = 12;
 
+// A marker before a child of a union, intersection or difference (mark_program):
+// op kSkip, n nodes to pass over, the child's bit in a[0], the value that stands
+// for it in s0.
+constexpr int kSkip = 30;
+constexpr int kMaxParts = 64;
+constexpr int kSuperMin = 2048;  // super-blocks from which on they are looked at first
+
 __device__ __forceinline__ double norm3(double a, double b, double c) {
     return __dsqrt_rn(d_add(d_add(d_mul(a, a), d_mul(b, b)), d_mul(c, c)));
 }
@@ -113,8 +120,9 @@ __device__ double path_distance(const sf_sdf_node* __restrict__ d, int m, int di
     return d_sub(best, radius);
 }
 
+template <bool MARKED = false>
 __device__ double eval_sdf(const sf_sdf_node* __restrict__ prog, int n, double x, double y,
-                           double z, int* err) {
+                           double z, int* err, unsigned long long skip = 0) {
     double ds[VX_DSTACK];
     double px[VX_PSTACK], py[VX_PSTACK], pz[VX_PSTACK];
     int dtop = 0, ptop = 0;
@@ -298,6 +306,13 @@ __device__ double eval_sdf(const sf_sdf_node* __restrict__ prog, int n, double x
                 ds[dtop - 1] = -ds[dtop - 1];
                 break;
             default:
+                if (MARKED && N.op == kSkip) {
+                    if (skip >> (int)N.a[0] & 1) {
+                        ds[dtop++] = N.s0;
+                        q += N.n;
+                    }
+                    break;
+                }
                 *err = 4;
                 return 1.0;
         }
@@ -309,7 +324,8 @@ __device__ double eval_sdf(const sf_sdf_node* __restrict__ prog, int n, double x
 // ---- FP32 intervals ---------------------------------------------------------
 
 // A node's constants as intervals: the floats at or below / at or above each
-// double (rounded on the host).
+// double (rounded on the host).  A marker has its bit, and a union, intersection
+// or difference its first child's bit (-1: not marked), in a[0].x as an integer.
 struct IvNode {
     int op, n;
     float2 a[3], b[3], s0, s1;
@@ -442,8 +458,14 @@ __device__ float2 iv_path_distance(const IvNode* __restrict__ d, int m, int dims
 }
 
 // eval_sdf over a box, operation for operation.  The program has passed
-// check_program, so the stacks need no checks here.
-__device__ float2 eval_iv(const IvNode* __restrict__ prog, int n, float2 x, float2 y, float2 z) {
+// check_program, so the stacks need no checks here.  Children whose bit is set in
+// `skip` are passed over: their markers push a value that cannot win.  RECORD
+// sets in *lost the bits of the children that lose to another everywhere in the
+// box: whatever box inside it is looked at next, the result does not depend on
+// them.  (A NaN bound loses to nothing and nothing loses to it.)
+template <bool RECORD>
+__device__ float2 eval_iv(const IvNode* __restrict__ prog, int n, float2 x, float2 y, float2 z,
+                          unsigned long long skip, unsigned long long* lost) {
     float2 ds[VX_DSTACK];
     float2 px[VX_PSTACK], py[VX_PSTACK], pz[VX_PSTACK];
     int dtop = 0, ptop = 0;
@@ -556,6 +578,11 @@ __device__ float2 eval_iv(const IvNode* __restrict__ prog, int n, float2 x, floa
                 float2 r = ds[base];
                 for (int c = 1; c < N.n; ++c)
                     r = (N.op == 10) ? iv_min(r, ds[base + c]) : iv_max(r, ds[base + c]);
+                const int bit = __float_as_int(N.a[0].x);
+                if (RECORD && bit >= 0)
+                    for (int c = 0; c < N.n; ++c)
+                        if (N.op == 10 ? ds[base + c].x > r.y : ds[base + c].y < r.x)
+                            *lost |= 1ull << (bit + c);
                 dtop = base;
                 ds[dtop++] = r;
                 break;
@@ -564,6 +591,10 @@ __device__ float2 eval_iv(const IvNode* __restrict__ prog, int n, float2 x, floa
                 const int base = dtop - N.n;
                 float2 r = ds[base];
                 for (int c = 1; c < N.n; ++c) r = iv_max(r, iv_neg(ds[base + c]));
+                const int bit = __float_as_int(N.a[0].x);
+                if (RECORD && bit >= 0)
+                    for (int c = 0; c < N.n; ++c)
+                        if ((c == 0 ? ds[base].y : -ds[base + c].x) < r.x) *lost |= 1ull << (bit + c);
                 dtop = base;
                 ds[dtop++] = r;
                 break;
@@ -598,6 +629,12 @@ __device__ float2 eval_iv(const IvNode* __restrict__ prog, int n, float2 x, floa
             case 24:
                 ds[dtop - 1] = iv_neg(ds[dtop - 1]);
                 break;
+            case kSkip:
+                if (skip >> __float_as_int(N.a[0].x) & 1) {
+                    ds[dtop++] = N.s0;
+                    q += N.n;
+                }
+                break;
         }
     }
     return ds[0];
@@ -617,6 +654,9 @@ struct VxGrid {
     float2* axis;          // the same centres as intervals (k_vx_axes)
     unsigned* count;       // queued blocks
     unsigned* queue;
+    int si, sj, sk;               // super-blocks of 16 x 16 x 32 cells per axis
+    unsigned long long* lost;     // per queue entry, in front of them one per super-block: the
+    unsigned char* side;          // parts that do not matter there; per super-block its side + 1
     uint8_t* out;
 };
 
@@ -630,40 +670,74 @@ __global__ void k_vx_axes(VxGrid g) {
     g.axis[t] = iv(__double2float_rd(c), __double2float_ru(c));
 }
 
-__device__ __forceinline__ float2 axis_hull(const float2* __restrict__ a, int i0, int n) {
+__device__ __forceinline__ float2 axis_hull(const float2* __restrict__ a, int i0, int cells, int n) {
     float2 h = a[i0];
-    for (int e = 1; e < 4; ++e)
+    for (int e = 1; e < cells; ++e)
         if (i0 + e < n) h = iv_hull(h, a[i0 + e]);
     return h;
 }
 
-// One thread per 4 x 4 x 4 block of cells, blocks numbered with k fastest, so
-// a warp's 32 threads write 128 consecutive bytes of a row.  A decided block is
-// filled, any other is queued.  Bound by instruction issue of the interval
-// program; the block edge is the smallest whose row fits one 32-bit store.
-// Measured on GB300, whole sf_voxelize calls: 400^3 enclosure (4 nodes)
-// 16.3 ms -> 0.15 ms, 180 x 240 x 157 with 16 resonators 18.2 ms -> 0.5 ms
-// (there k_vx_blocks 53 us, k_vx_cells 365 us).
-__global__ void __launch_bounds__(128) k_vx_blocks(VxGrid g, const IvNode* __restrict__ prog, int n) {
-    const int bj_n = (g.ny + 3) / 4, bk_n = (g.nz + 3) / 4;
-    const long long total = (long long)((g.nx + 3) / 4) * bj_n * bk_n;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool real = t < total;
-    int i0 = 0, j0 = 0, k0 = 0, side = 0;
-    if (real) {
-        k0 = 4 * (int)(t % bk_n);
-        j0 = 4 * (int)(t / bk_n % bj_n);
-        i0 = 4 * (int)(t / bk_n / bj_n);
-        side = iv_side(eval_iv(prog, n, axis_hull(g.axis, i0, g.nx), axis_hull(g.axis + g.nx, j0, g.ny),
-                               axis_hull(g.axis + g.nx + g.ny, k0, g.nz)));
+// A program of up to kStaged nodes is read from shared memory: a thread that walks
+// it alone otherwise waits for each node in turn (16 resonators: TSUP).
+constexpr int kStaged = 256;
+__device__ __forceinline__ const IvNode* stage(IvNode* to, const IvNode* __restrict__ prog, int n) {
+    if (n > kStaged) return prog;
+    float2* d = reinterpret_cast<float2*>(to);
+    const float2* f = reinterpret_cast<const float2*>(prog);
+    for (int e = threadIdx.x; e < n * (int)(sizeof(IvNode) / sizeof(float2)); e += blockDim.x) d[e] = f[e];
+    __syncthreads();
+    return to;
+}
+
+// One thread per super-block of 16 x 16 x 32 cells: its side, and the parts of the
+// program that matter nowhere in it.
+__global__ void __launch_bounds__(32) k_vx_super(VxGrid g, const IvNode* __restrict__ program, int n) {
+    __shared__ IvNode staged[kStaged];
+    const IvNode* prog = stage(staged, program, n);
+    const int t = blockIdx.x * 32 + threadIdx.x;
+    if (t >= g.si * g.sj * g.sk) return;
+    const int k0 = 32 * (t % g.sk), j0 = 16 * (t / g.sk % g.sj), i0 = 16 * (t / g.sk / g.sj);
+    unsigned long long lost = 0;
+    const float2 d = eval_iv<true>(prog, n, axis_hull(g.axis, i0, 16, g.nx),
+                                   axis_hull(g.axis + g.nx, j0, 16, g.ny),
+                                   axis_hull(g.axis + g.nx + g.ny, k0, 32, g.nz), 0, &lost);
+    g.lost[t] = lost;
+    g.side[t] = (unsigned char)(iv_side(d) + 1);
+}
+
+// One thread block per super-block, one thread per 4 x 4 x 4 block of cells, with
+// k fastest, so that 8 threads write 32 consecutive bytes of a row.  A decided
+// block is filled, any other is queued with the parts that do not matter in it.
+// Bound by instruction issue of the interval program; the block edge is the
+// smallest whose row fits one 32-bit store.
+__global__ void __launch_bounds__(128) k_vx_blocks(VxGrid g, const IvNode* __restrict__ program, int n, int supers) {
+    __shared__ IvNode staged[kStaged];
+    const int sb = blockIdx.x, t = threadIdx.x;
+    const int k0 = 32 * (sb % g.sk) + 4 * (t & 7), j0 = 16 * (sb / g.sk % g.sj) + 4 * (t >> 3 & 3),
+              i0 = 16 * (sb / g.sk / g.sj) + 4 * (t >> 5);
+    const bool real = k0 < g.nz && j0 < g.ny && i0 < g.nx;
+    int side = supers ? (int)g.side[sb] - 1 : -1;  // (else the super-blocks were not looked at)
+    const bool open = side < 0;
+    const IvNode* prog = open ? stage(staged, program, n) : program;  // (the whole block is open or not)
+    unsigned long long lost = 0;
+    if (!real) side = 0;
+    if (real && open) {
+        const unsigned long long skip = supers ? g.lost[sb] : 0;
+        lost = skip;
+        side = iv_side(eval_iv<true>(prog, n, axis_hull(g.axis, i0, 4, g.nx),
+                                     axis_hull(g.axis + g.nx, j0, 4, g.ny),
+                                     axis_hull(g.axis + g.nx + g.ny, k0, 4, g.nz), skip, &lost));
     }
-    const int lane = threadIdx.x & 31;
+    const int lane = t & 31;
     const unsigned m = __ballot_sync(0xffffffffu, side < 0);
     if (m) {  // one atomic per warp
         unsigned at = 0;
         if (lane == 0) at = atomicAdd(g.count, (unsigned)__popc(m));
-        at = __shfl_sync(0xffffffffu, at, 0);
-        if (side < 0) g.queue[at + __popc(m & ((1u << lane) - 1))] = (unsigned)t;
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1));
+        if (side < 0) {
+            g.queue[at] = (unsigned)(((long long)(i0 / 4) * ((g.ny + 3) / 4) + j0 / 4) * ((g.nz + 3) / 4) + k0 / 4);
+            g.lost[(size_t)g.si * g.sj * g.sk + at] = lost;
+        }
     }
     if (!real || side < 0) return;
     const uint8_t v = (uint8_t)((side == 1) != (g.invert != 0));
@@ -678,30 +752,60 @@ __global__ void __launch_bounds__(128) k_vx_blocks(VxGrid g, const IvNode* __res
         }
 }
 
-// The queued blocks' cells, one thread each: the cell's own interval, and the
-// FP64 evaluation where that straddles zero.
-__global__ void __launch_bounds__(128) k_vx_cells(VxGrid g, const IvNode* __restrict__ ivp,
-                                                  const sf_sdf_node* __restrict__ prog, int n) {
+// The cell of thread t of the queued blocks.
+__device__ __forceinline__ bool queued_cell(const VxGrid& g, unsigned long long t, int& i, int& j, int& k) {
     const int bj_n = (g.ny + 3) / 4, bk_n = (g.nz + 3) / 4;
+    const unsigned b = g.queue[t >> 6];
+    const int e = (int)(t & 63);
+    k = 4 * (int)(b % bk_n) + (e & 3);
+    j = 4 * (int)(b / bk_n % bj_n) + (e >> 2 & 3);
+    i = 4 * (int)(b / bk_n / bj_n) + (e >> 4);
+    return i < g.nx && j < g.ny && k < g.nz;
+}
+
+// The queued blocks' cells, one thread each: the cell's own interval, and the
+// FP64 evaluation where that straddles zero.  Straddling cells lie in planes (a
+// face through cell centres), a few to a warp, and the FP64 pipe takes as long for
+// a few lanes as for 32: a thread block collects them and evaluates them side by
+// side (TCELL).
+__global__ void __launch_bounds__(128) k_vx_cells(VxGrid g, const IvNode* __restrict__ program,
+                                                  const sf_sdf_node* __restrict__ prog, int n) {
+    __shared__ IvNode staged[kStaged];
+    __shared__ unsigned long long open[256];
+    __shared__ int n_open;
     const unsigned long long cells = (unsigned long long)*g.count * 64;
-    for (unsigned long long t = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; t < cells;
-         t += (unsigned long long)gridDim.x * blockDim.x) {
-        const unsigned b = g.queue[t >> 6];
-        const int e = (int)(t & 63);
-        const int k = 4 * (int)(b % bk_n) + (e & 3), j = 4 * (int)(b / bk_n % bj_n) + (e >> 2 & 3),
-                  i = 4 * (int)(b / bk_n / bj_n) + (e >> 4);
-        if (i >= g.nx || j >= g.ny || k >= g.nz) continue;
-        const int side = iv_side(
-            eval_iv(ivp, n, g.axis[i], g.axis[g.nx + j], g.axis[g.nx + g.ny + k]));
-        bool inside = side == 1;
-        if (side < 0) {
-            int err = 0;  // the program has passed check_program
-            inside = eval_sdf(prog, n, cell_centre(g.coords, 0, i, g.res),
-                              cell_centre(g.coords, g.nx, j, g.res),
-                              cell_centre(g.coords, g.nx + g.ny, k, g.res), &err) <= 0.0;
-        }
+    const unsigned long long* lost = g.lost + (size_t)g.si * g.sj * g.sk;
+    if (threadIdx.x == 0) n_open = 0;
+    const IvNode* ivp = stage(staged, program, n);
+    auto put = [&](int i, int j, int k, bool inside) {
         g.out[((long long)i * g.ny + j) * g.nz + k] = (uint8_t)(inside != (g.invert != 0));
+    };
+    auto exact = [&](unsigned long long t) {
+        int i, j, k, err = 0;  // the program has passed check_program
+        queued_cell(g, t, i, j, k);
+        put(i, j, k,
+            eval_sdf<true>(prog, n, cell_centre(g.coords, 0, i, g.res), cell_centre(g.coords, g.nx, j, g.res),
+                           cell_centre(g.coords, g.nx + g.ny, k, g.res), &err, lost[t >> 6]) <= 0.0);
+    };
+    __syncthreads();
+    for (unsigned long long first = (unsigned long long)blockIdx.x * 128; first < cells;
+         first += (unsigned long long)gridDim.x * 128) {
+        const unsigned long long t = first + threadIdx.x;
+        int i, j, k;
+        if (t < cells && queued_cell(g, t, i, j, k)) {
+            const int side = iv_side(eval_iv<false>(ivp, n, g.axis[i], g.axis[g.nx + j],
+                                                    g.axis[g.nx + g.ny + k], lost[t >> 6], nullptr));
+            if (side < 0) open[atomicAdd(&n_open, 1)] = t;  // at most 127 + 128
+            else put(i, j, k, side == 1);
+        }
+        __syncthreads();
+        const int have = n_open;
+        if (have >= 128) exact(open[have - 128 + threadIdx.x]);
+        __syncthreads();
+        if (have >= 128 && threadIdx.x == 0) n_open = have - 128;
+        __syncthreads();
     }
+    if ((int)threadIdx.x < n_open) exact(open[threadIdx.x]);
 }
 
 // MaterializedGeometry.voxelize_with_materials (geometry/
@@ -851,10 +955,117 @@ float2 bounds_of(double v) {
     return r;
 }
 
+IvNode interval_node(const sf_sdf_node& N) {
+    IvNode v;
+    v.op = N.op;
+    v.n = N.n;
+    for (int e = 0; e < 3; ++e) {
+        v.a[e] = bounds_of(N.a[e]);
+        v.b[e] = bounds_of(N.b[e]);
+    }
+    v.s0 = bounds_of(N.s0);
+    v.s1 = bounds_of(N.s1);
+    return v;
+}
+
+// A checked program with a skip marker before each child of its unions, intersections and differences: the outer ones first, up to kMaxParts
+// children (an operation whose children do not fit has none).  A child is the run
+// of nodes that leaves its value, from the transforms it opens with to the last of
+// those it closes with; where a transform encloses anything but one value, no
+// child of the program is marked.
+std::vector<sf_sdf_node> mark_program(const sf_sdf_node* nodes, int n, std::vector<int>& first_bit) {
+    struct Child {
+        int op, index, start, end;  // its operation's node, its place there, its nodes
+    };
+    struct Open {
+        int node;
+        size_t values;
+    };
+    std::vector<Child> children;
+    std::vector<int> value;  // first node of each value on the stack
+    std::vector<Open> open;
+    auto inside = [&] { return open.empty() ? 0 : open.back().values; };  // values below the transform
+    bool clean = true;
+    for (int q = 0; q < n; ++q) {
+        const sf_sdf_node& N = nodes[q];
+        const int at = q;
+        switch (N.op) {
+            case 4: case 5: ++q; value.push_back(at); break;
+            case 6: case 7: q += N.n; value.push_back(at); break;
+            case 13: case 14: case 15:
+                value.pop_back();
+                clean = clean && value.size() > inside();
+                break;
+            case 10: case 11: case 12: {
+                if (N.n == 0) {
+                    value.push_back(at);
+                    break;
+                }
+                const size_t base = value.size() - N.n;
+                clean = clean && base >= inside();
+                for (int c = 0; c < N.n; ++c)
+                    children.push_back({at, c, value[base + c], c + 1 < N.n ? value[base + c + 1] : at});
+                value.resize(base + 1);
+                break;
+            }
+            case 20: case 21: open.push_back({at, value.size()}); break;
+            case 25: ++q; open.push_back({at, value.size()}); break;
+            case 22:
+                if (value.size() == open.back().values + 1) value.back() = open.back().node;
+                else clean = false;
+                open.pop_back();
+                break;
+            case 23: case 24: clean = clean && value.size() > inside(); break;
+            default: value.push_back(at); break;  // 1, 2, 3
+        }
+    }
+    std::vector<int> bit(n, -1), last(n, -1), before(children.size(), -1);
+    int used = 0;
+    for (size_t c = children.size(); clean && c-- > 0;) {  // an outer operation stands after its children's
+        const int op = children[c].op, k = nodes[op].n;
+        if (children[c].index != 0 || k < 2 || used + k > kMaxParts) continue;
+        bit[op] = used;
+        used += k;
+    }
+    for (size_t c = 0; c < children.size(); ++c) {  // children by first node, the outermost first
+        before[c] = last[children[c].start];
+        last[children[c].start] = (int)c;
+    }
+    std::vector<sf_sdf_node> out;
+    first_bit.clear();
+    auto put = [&](const sf_sdf_node& N, int b) {
+        out.push_back(N);
+        first_bit.push_back(b);
+    };
+    std::vector<int> place(n + 1);
+    std::vector<std::pair<int, int>> jumps;  // marker, the node it passes over to
+    for (int q = 0; q < n; ++q) {
+        place[q] = (int)out.size();
+        for (int c = last[q]; c >= 0; c = before[c]) {
+            const Child& C = children[c];
+            if (bit[C.op] < 0) continue;
+            sf_sdf_node m{};
+            const int op = nodes[C.op].op;
+            const bool high = op == 10 || (op == 12 && C.index > 0);  // what never wins there
+            m.op = kSkip;
+            m.a[0] = bit[C.op] + C.index;
+            m.s0 = high ? INFINITY : -INFINITY;
+            jumps.push_back({(int)out.size(), C.end});
+            put(m, bit[C.op] + C.index);
+        }
+        const int op = nodes[q].op;
+        put(nodes[q], bit[q]);
+        const int data = op == 4 || op == 5 || op == 25 ? 1 : (op == 6 || op == 7 ? nodes[q].n : 0);
+        for (int e = 0; e < data; ++e) put(nodes[++q], -1);
+    }
+    for (const auto& j : jumps) out[j.first].n = place[j.second] - j.first - 1;
+    return out;
+}
+
 // Device memory of a voxelisation, kept between calls (one block per device
 // of at most kKeepBytes, lent to one call at a time; released with the
 // deferred frees): a call's allocation took longer than its kernels.
-constexpr size_t kKeepBytes = size_t(24) << 20;
+constexpr size_t kKeepBytes = size_t(72) << 20;  // 500^3 cells: 26 MB
 constexpr int kKeepDevices = 64;
 struct Kept {
     char* p = nullptr;
@@ -931,26 +1142,26 @@ int sf_launch_voxelize(const sf_sdf_node* nodes, int n_nodes, int nx, int ny, in
                        const double* const* coords, int invert, uint8_t* out, cudaStream_t st) {
     if (!check_program(nodes, n_nodes))
         return sf_fail("sf_voxelize: malformed SDF program (stack error)");
+    const int si = (nx + 15) / 16, sj = (ny + 15) / 16, sk = (nz + 31) / 32;
+    const long long supers = (long long)si * sj * sk;
     const long long blocks =
         (long long)((nx + 3) / 4) * ((ny + 3) / 4) * ((nz + 3) / 4);
     if (blocks > 0xffffffffLL) return sf_fail("sf_voxelize: grid too large");
+    std::vector<int> first_bit;
+    const std::vector<sf_sdf_node> marked = mark_program(nodes, n_nodes, first_bit);
+    const int n_marked = (int)marked.size();
     const size_t n_axis = (size_t)nx + ny + nz;
-    const size_t off_iv = up16(sizeof(sf_sdf_node) * n_nodes);
-    const size_t off_co = off_iv + up16(sizeof(IvNode) * n_nodes);
+    const size_t off_iv = up16(sizeof(sf_sdf_node) * n_marked);
+    const size_t off_co = off_iv + up16(sizeof(IvNode) * n_marked);
     const size_t sent = off_co + (coords ? up16(sizeof(double) * n_axis) : 0);
-    const size_t off_ax = sent, off_ct = off_ax + up16(sizeof(float2) * n_axis), off_q = off_ct + 16;
+    const size_t off_ax = sent, off_ct = off_ax + up16(sizeof(float2) * n_axis), off_sd = off_ct + 16,
+                 off_l = off_sd + up16((size_t)supers), off_q = off_l + 8 * (size_t)(supers + blocks);
     std::vector<char> host(sent);
-    std::memcpy(host.data(), nodes, sizeof(sf_sdf_node) * n_nodes);
-    for (int q = 0; q < n_nodes; ++q) {
-        IvNode v;
-        v.op = nodes[q].op;
-        v.n = nodes[q].n;
-        for (int e = 0; e < 3; ++e) {
-            v.a[e] = bounds_of(nodes[q].a[e]);
-            v.b[e] = bounds_of(nodes[q].b[e]);
-        }
-        v.s0 = bounds_of(nodes[q].s0);
-        v.s1 = bounds_of(nodes[q].s1);
+    std::memcpy(host.data(), marked.data(), sizeof(sf_sdf_node) * n_marked);
+    for (int q = 0; q < n_marked; ++q) {
+        const int op = marked[q].op;
+        IvNode v = interval_node(marked[q]);
+        if (op == kSkip || op == 10 || op == 11 || op == 12) std::memcpy(&v.a[0].x, &first_bit[q], 4);
         std::memcpy(host.data() + off_iv + sizeof(IvNode) * q, &v, sizeof(v));
     }
     if (coords) {
@@ -968,12 +1179,18 @@ int sf_launch_voxelize(const sf_sdf_node* nodes, int n_nodes, int nx, int ny, in
         return sf_fail("sf_voxelize: upload failed");
     const VxGrid g{nx, ny, nz, invert, res, coords ? reinterpret_cast<const double*>(b + off_co) : nullptr,
                    reinterpret_cast<float2*>(b + off_ax), reinterpret_cast<unsigned*>(b + off_ct),
-                   reinterpret_cast<unsigned*>(b + off_q), out};
+                   reinterpret_cast<unsigned*>(b + off_q), si, sj, sk,
+                   reinterpret_cast<unsigned long long*>(b + off_l),
+                   reinterpret_cast<unsigned char*>(b + off_sd), out};
     const sf_sdf_node* prog = reinterpret_cast<const sf_sdf_node*>(b);
     const IvNode* ivp = reinterpret_cast<const IvNode*>(b + off_iv);
     k_vx_axes<<<(unsigned)((n_axis + 127) / 128), 128, 0, st>>>(g);
-    k_vx_blocks<<<(unsigned)((blocks + 127) / 128), 128, 0, st>>>(g, ivp, n_nodes);
-    k_vx_cells<<<152 * 16, 128, 0, st>>>(g, ivp, prog, n_nodes);
+    // One thread walks the whole program for a super-block, so that takes its
+    // latency however few there are: TSUPER.
+    const bool look = supers >= kSuperMin;
+    if (look) k_vx_super<<<(unsigned)((supers + 31) / 32), 32, 0, st>>>(g, ivp, n_marked);
+    k_vx_blocks<<<(unsigned)supers, 128, 0, st>>>(g, ivp, n_marked, look);
+    k_vx_cells<<<152 * 16, 128, 0, st>>>(g, ivp, prog, n_marked);
     if (cudaGetLastError() != cudaSuccess) return sf_fail("k_voxelize launch failed");
     if (cudaStreamSynchronize(st) != cudaSuccess) return sf_fail("sf_voxelize: kernel failed");
     return 0;
