@@ -40,9 +40,12 @@
 // FP64 evaluator computes from any point of the box, roundings included: an
 // interval wholly at or below zero, or wholly above, decides every cell in
 // the box exactly as the FP64 evaluation would.  Blocks of 4 x 4 x 4 cells
-// are decided (or queued) by k_vx_blocks, the queued blocks' cells one at a
+// are decided (or queued) by k_vx_blocks (on large grids super-blocks of 16 x 16 x
+// 32 before them, by k_vx_super), the queued blocks' cells one at a
 // time by k_vx_cells, and only a cell whose own interval straddles zero is
-// evaluated in FP64.
+// evaluated in FP64.  Solids of many parts are mostly decided by a few of them:
+// a part of a union, intersection or difference that loses to another everywhere in
+// a block is left out inside it.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -678,7 +681,8 @@ __device__ __forceinline__ float2 axis_hull(const float2* __restrict__ a, int i0
 }
 
 // A program of up to kStaged nodes is read from shared memory: a thread that walks
-// it alone otherwise waits for each node in turn (16 resonators: TSUP).
+// it alone otherwise waits for each node in turn (k_vx_super on 900 super-blocks,
+// a program of 16 resonators: 69 -> 43 us).
 constexpr int kStaged = 256;
 __device__ __forceinline__ const IvNode* stage(IvNode* to, const IvNode* __restrict__ prog, int n) {
     if (n > kStaged) return prog;
@@ -709,7 +713,10 @@ __global__ void __launch_bounds__(32) k_vx_super(VxGrid g, const IvNode* __restr
 // k fastest, so that 8 threads write 32 consecutive bytes of a row.  A decided
 // block is filled, any other is queued with the parts that do not matter in it.
 // Bound by instruction issue of the interval program; the block edge is the
-// smallest whose row fits one 32-bit store.
+// smallest whose row fits one 32-bit store.  Measured on GB300, whole sf_voxelize
+// calls: 400^3 enclosure (4 nodes) 16.3 ms with one FP64 evaluation per cell, 0.154
+// with blocks and cells over the whole program, 0.12 now; 180 x 240 x 157 with 16
+// resonators 18.2, 0.53 and 0.27 (of which 0.17 is the host's).
 __global__ void __launch_bounds__(128) k_vx_blocks(VxGrid g, const IvNode* __restrict__ program, int n, int supers) {
     __shared__ IvNode staged[kStaged];
     const int sb = blockIdx.x, t = threadIdx.x;
@@ -767,7 +774,10 @@ __device__ __forceinline__ bool queued_cell(const VxGrid& g, unsigned long long 
 // FP64 evaluation where that straddles zero.  Straddling cells lie in planes (a
 // face through cell centres), a few to a warp, and the FP64 pipe takes as long for
 // a few lanes as for 32: a thread block collects them and evaluates them side by
-// side (TCELL).
+// side (180 x 240 x 157 with 32 resonators: 289 -> 243 us; with 16, where the
+// interval program bounds it, 30 -> 32).  Both evaluators pass over the parts that
+// do not matter in the block: 365 -> 332 us for 16 with the intervals alone, then 47
+// with the FP64 program too.
 __global__ void __launch_bounds__(128) k_vx_cells(VxGrid g, const IvNode* __restrict__ program,
                                                   const sf_sdf_node* __restrict__ prog, int n) {
     __shared__ IvNode staged[kStaged];
@@ -968,11 +978,13 @@ IvNode interval_node(const sf_sdf_node& N) {
     return v;
 }
 
-// A checked program with a skip marker before each child of its unions, intersections and differences: the outer ones first, up to kMaxParts
-// children (an operation whose children do not fit has none).  A child is the run
-// of nodes that leaves its value, from the transforms it opens with to the last of
-// those it closes with; where a transform encloses anything but one value, no
-// child of the program is marked.
+// A checked program with a skip marker before each child of its unions,
+// intersections and differences: the outer ones first, up to kMaxParts children
+// (an operation whose children do not fit has none).  first_bit[q] is the bit of
+// the marker at node q of the result, or of the first child of the operation there,
+// or -1.  A child is the run of nodes that leaves its value, from the transforms it
+// opens with to the last of those it closes with; where a transform encloses
+// anything but one value made inside it, no child of the program is marked.
 std::vector<sf_sdf_node> mark_program(const sf_sdf_node* nodes, int n, std::vector<int>& first_bit) {
     struct Child {
         int op, index, start, end;  // its operation's node, its place there, its nodes
@@ -1186,7 +1198,10 @@ int sf_launch_voxelize(const sf_sdf_node* nodes, int n_nodes, int nx, int ny, in
     const IvNode* ivp = reinterpret_cast<const IvNode*>(b + off_iv);
     k_vx_axes<<<(unsigned)((n_axis + 127) / 128), 128, 0, st>>>(g);
     // One thread walks the whole program for a super-block, so that takes its
-    // latency however few there are: TSUPER.
+    // latency however few there are, and pays where they fill the chip.  Calls with
+    // and without (16 resonators): 180 x 240 x 157 (900 super-blocks) 293 and 273
+    // us, 300^3 (3610) 313 and 481, 400^3 313 and 747; enclosure 200^3 (1183) 129
+    // and 112 to 131, 400^3 (8125) 138 and 172.
     const bool look = supers >= kSuperMin;
     if (look) k_vx_super<<<(unsigned)((supers + 31) / 32), 32, 0, st>>>(g, ivp, n_marked);
     k_vx_blocks<<<(unsigned)supers, 128, 0, st>>>(g, ivp, n_marked, look);

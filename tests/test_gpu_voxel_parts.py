@@ -60,3 +60,13 @@ def test_mask_equals_point_evaluation(name, shape):
     want = solid.contains(pts.reshape(-1, 3)).reshape(shape)
     assert np.array_equal(solid.voxelize(grid), want)
     assert np.array_equal(solid.voxelize_device(grid, invert=True).cpu().numpy().astype(bool), ~want)
+
+
+@pytest.mark.parametrize("name", list(SHAPES))
+def test_grid_of_many_super_blocks_equals_point_evaluation(name):
+    """Thin, but with more super-blocks than are needed to look at those first."""
+    solid = SHAPES[name]().translate((-30 * R, -29 * R, 0))
+    grid = S.UniformGrid((17, 20, 16400), R / 256)
+    pts = np.stack(np.meshgrid(grid.x_coords, grid.y_coords, grid.z_coords, indexing="ij"), -1)
+    want = solid.contains(pts.reshape(-1, 3)).reshape(grid.shape)
+    assert np.array_equal(solid.voxelize(grid), want)
