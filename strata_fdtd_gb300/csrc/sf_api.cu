@@ -1011,6 +1011,9 @@ bool resident_extra(const sf_plan* P, bool mics, SfResExtra& x) {
     x.n_plane = P->n_plane;
     for (int q = 0; q < P->n_plane; ++q) {
         x.ops[q] = P->plane_ops[q];
+        const double c = x.ops[q].coeff;
+        if (std::fabs(c) > 0x1p-20 && std::fabs(c) < 0x1p20)
+            x.coeff[q] = make_float2((float)c, (float)(c - (double)(float)c));
         for (int side = 0; side < 2; ++side) x.prev[q][side] = P->plane_prev + P->plane_off[q][side];
     }
     for (int q = 0; q < P->src.n; ++q) {

@@ -111,12 +111,14 @@ struct SfResLayout {
     int wlist;           // weighted sources: (cell in P, source, weight) entries
     int mic;             // microphone corners (int4)
     int end;
+    int plist;           // cells of the absorbing planes
 };
 // What acts between the steps: pressure-plane boundaries, weighted sources on
 // the pressure, microphone corners.
 struct SfResExtra {
     int n_plane;
     sf_plane_bc ops[SF_MAX_PLANE_OPS];
+    float2 coeff[SF_MAX_PLANE_OPS];  // ops[].coeff as a sum of two floats (0, 0: not taken apart)
     float* prev[SF_MAX_PLANE_OPS][2];
     const long long* wcells[SF_MAX_SOURCES];  // by source
     const double* ww[SF_MAX_SOURCES];

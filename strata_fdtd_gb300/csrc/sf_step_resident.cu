@@ -41,6 +41,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 
 #include "sf_common.cuh"
 #include "sf_kernels.h"
@@ -181,6 +182,10 @@ inline Layout layout(int L, int nci, int nj, int nq, int n_probe, bool nu, const
         for (int side = 0; side < 2; ++side)
             l.prev[q][side] =
                 x && q < x->n_plane ? take(plane_cells(x->ops[q].axis, planes, nj, nq * 4)) : 0;
+    int listed = 0;
+    for (int q = 0; x && q < x->n_plane; ++q)
+        listed += (x->ops[q].kind == 0 ? 2 : 1) * plane_cells(x->ops[q].axis, planes, nj, nq * 4);
+    l.plist = take((listed + 1) / 2);  // two to a word
     long long wcap = 0;  // entries a block can have: its overlap with the sources' box
     if (x && x->w_slots > 0) {
         const int dims[3] = {planes, nj, nq * 4};
@@ -415,46 +420,76 @@ __device__ __forceinline__ void phase_p(const SfStepArgs& a, const Layout& S, co
 
 // ---- between the steps --------------------------------------------------------
 
-// One plane boundary over the block's share of its planes (k_plane_bc's
-// arithmetic: the low end, then the high one).
-__device__ __forceinline__ void plane_op(const SfStepArgs& a, const Layout& S, const Place& g,
-                                         const sf_plane_bc& op, const int (&prev)[2]) {
-    const int ax = op.axis;
-    const bool lo = !g.b.lo[ax] && (op.kind == 0 || op.side == 0);
-    const bool hi = !g.b.hi[ax] && (op.kind == 0 || op.side == 1);
-    if (!lo && !hi) return;
-    const int cnt = plane_cells(ax, g.planes, g.b.nj, g.row);
-    const int n = ax == 0 ? a.nx - g.gi0 : (ax == 1 ? g.b.nj : a.nz - g.gk0);  // cells up to the grid's end
-    const int stride = ax == 0 ? g.plane : (ax == 1 ? g.row : 1);
-    for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
-        int base;  // the plane's cell at position 0 along the axis
-        if (ax == 0) {
-            if (g.gk0 + t % g.row >= a.nz) continue;
-            base = t;
-        } else if (ax == 1) {
-            const int i = t / g.row;
-            if (g.gi0 + i >= a.nx || g.gk0 + t % g.row >= a.nz) continue;
-            base = i * g.plane + t % g.row;
-        } else {
-            const int i = t / g.b.nj;
-            if (g.gi0 + i >= a.nx) continue;
-            base = i * g.plane + t % g.b.nj * g.row;
-        }
-#pragma unroll
+// float(double(was) + coeff * double(d)), the two FP64 operations rounded, with
+// coeff = c.x + c.y to 2^-47 (c.x = 0: no such split).  In FP32 x = zh + zl is was
+// + coeff d to 2^-44 (|c.x d| + |s|), and the FP64 result differs from it by less;
+// where everything within 2^-43 of that scale rounds to zh, zh is the answer.
+// Elsewhere (one in 2^17, and below 2^-70, where a product's low part could be
+// lost) the FP64 pipe decides: it has 2 lanes a clock, and took 0.5 us of a step
+// for a corner block's 1344 plane cells (112 x 96 x 120, three absorbing axes).
+__device__ __forceinline__ float plane_value(float was, double coeff, float2 c, float d) {
+    const float ph = f_mul(c.x, d);
+    if (d == 0.0f && c.x != 0.0f) return f_add(was, ph);  // exact, the sign of zero too
+    const float pl = __fmaf_rn(c.y, d, __fmaf_rn(c.x, d, -ph));
+    const float s = f_add(was, ph), bv = f_sub(s, was);
+    const float t = f_add(f_add(f_sub(was, f_sub(s, bv)), f_sub(ph, bv)), pl);
+    const float zh = f_add(s, t), tv = f_sub(zh, s);
+    const float zl = f_add(f_sub(s, f_sub(zh, tv)), f_sub(t, tv));
+    const float err = f_mul(f_add(fabsf(ph), fabsf(s)), 0x1p-43f);
+    if (fabsf(ph) >= 0x1p-70f && f_add(zh, f_add(zl, err)) == zh && f_add(zh, f_sub(zl, err)) == zh)
+        return zh;
+    return __double2float_rn(d_add((double)was, d_mul(coeff, (double)d)));
+}
+
+// The places in shared memory of the block's cells in the grid's absorbing planes,
+// by operation and end, each list as long as its stored plane (kNoCell: past the
+// grid).  Built once: with the places worked out at each step an operation took
+// 0.65 us of a step, of two cells a thread (112 x 96 x 120, three operations, two
+// sources and two microphones: 7.84 us a step, 7.16 with the lists; 9.56 with four
+// cells' loads before their stores, which spilled).
+constexpr unsigned short kNoCell = 0xffff;
+__device__ __forceinline__ bool has_plane(const Place& g, const sf_plane_bc& op, int side) {
+    return !(side ? g.b.hi[op.axis] : g.b.lo[op.axis]) && (op.kind == 0 || op.side == side);
+}
+__device__ __forceinline__ void list_planes(const SfStepArgs& a, const SfResExtra& x, const Layout& S,
+                                            const Place& g) {
+    unsigned short* list = reinterpret_cast<unsigned short*>(smem + S.plist);
+    for (int q = 0; q < x.n_plane; ++q) {
+        const sf_plane_bc& op = x.ops[q];
+        const int ax = op.axis, cnt = plane_cells(ax, g.planes, g.b.nj, g.row);
+        const int n = ax == 0 ? a.nx - g.gi0 : (ax == 1 ? g.b.nj : a.nz - g.gk0);  // cells up to the grid's end
+        const int stride = ax == 0 ? g.plane : (ax == 1 ? g.row : 1);
         for (int side = 0; side < 2; ++side) {
-            if (!(side ? hi : lo)) continue;
-            float& pb = smem[S.P + base + (side ? n - 1 : 0) * stride];
-            const float pi = smem[S.P + base + (side ? n - 2 : 1) * stride];
-            float& was = smem[prev[side] + t];
-            const double abc = d_add((double)was, d_mul(op.coeff, (double)f_sub(pi, pb)));
-            if (op.kind == 0) {
-                pb = __double2float_rn(abc);
-            } else {
-                const float rig = f_mul(__double2float_rn(op.reflection), pi);
-                pb = __double2float_rn(d_add((double)rig, d_mul(d_sub(1.0, op.reflection), abc)));
+            if (!has_plane(g, op, side)) continue;
+            for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
+                const int per = ax == 2 ? g.b.nj : g.row, u = t / per, v = t % per;
+                const bool live = (ax == 0 || g.gi0 + u < a.nx) && (ax == 2 || g.gk0 + v < a.nz);
+                const int cell = u * (ax == 0 ? g.row : g.plane) + v * (ax == 2 ? g.row : 1);
+                list[t] = live ? (unsigned short)(S.P + cell + (side ? n - 1 : 0) * stride) : kNoCell;
             }
-            was = pi;
+            list += cnt;
         }
+    }
+}
+
+// One plane boundary over one end's list (k_plane_bc's arithmetic): its inner
+// neighbours lie at `inner`, its stored values at `prev`.
+__device__ __forceinline__ void plane_op(const sf_plane_bc& op, float2 coeff, const unsigned short* list,
+                                         int cnt, int inner, int prev) {
+    for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
+        const unsigned cell = list[t];
+        if (cell == kNoCell) continue;
+        float& pb = smem[cell];
+        const float pi = smem[(int)cell + inner];
+        float& was = smem[prev + t];
+        if (op.kind == 0) {
+            pb = plane_value(was, op.coeff, coeff, f_sub(pi, pb));
+        } else {
+            const double abc = d_add((double)was, d_mul(op.coeff, (double)f_sub(pi, pb)));
+            const float rig = f_mul(__double2float_rn(op.reflection), pi);
+            pb = __double2float_rn(d_add((double)rig, d_mul(d_sub(1.0, op.reflection), abc)));
+        }
+        was = pi;
     }
 }
 
@@ -723,10 +758,13 @@ __global__ void __launch_bounds__(MAXT, 1) k_resident(const __grid_constant__ Sf
     const SfResExtra& x = A.x;
     // microphone corners: (number, value, its decay, -1) in shared memory, or
     // (number, field << 8 | plane << 2 | cell, its decay, thread) in a thread's registers
+    // (walked as lists: every owner passing over the 40 corners of two microphones, one
+    // a cardioid, took 1.5 us a step)
     int4* mics = reinterpret_cast<int4*>(smem + S.mic);
     int4* wlist = reinterpret_cast<int4*>(smem + S.wlist);  // (place in P, source, weight)
     if (EXTRA) {
         move_prev(a, x, S, g, false);
+        list_planes(a, x, S, g);
         for (int q = 0; q < src.n; ++q)
             if (src.s[q].kind == 2)
                 for (int t = tid; t < x.wn[q]; t += nthreads) {
@@ -825,8 +863,13 @@ __global__ void __launch_bounds__(MAXT, 1) k_resident(const __grid_constant__ Sf
     const int probes = ctl[1];
     const bool has_units = U[0].d != 0;
     const int n_w = EXTRA ? ctl[0] : 0, n_mics = EXTRA ? ctl[3] : 0;
-    bool my_mics = false;
-    for (int t = 0; t < n_mics; ++t) my_mics = my_mics || mics[t].w == tid;
+    // a thread's own corners as a list (the next one + 1 in bits 16 up of .y)
+    int my_mics = -1;
+    for (int t = n_mics - 1; t >= 0; --t)
+        if (mics[t].w == tid) {
+            mics[t].y |= (my_mics + 1) << 16;
+            my_mics = t;
+        }
     // the state's values at the microphone corners after step s
     auto record_mics = [&](int s) {
         float* out = x.corners + (size_t)s * x.n_mic * 8;
@@ -835,15 +878,14 @@ __global__ void __launch_bounds__(MAXT, 1) k_resident(const __grid_constant__ Sf
             if (m.w >= 0) continue;
             out[m.x] = m.z < 0 ? smem[m.y] : f_mul(smem[m.y], smem[m.z]);
         }
-        if (!my_mics) return;
-        for (int t = 0; t < n_mics; ++t) {
+        for (int t = my_mics; t >= 0;) {
             const int4 m = mics[t];
-            if (m.w != tid) continue;
+            t = (m.y >> 16) - 1;
             float v = 0.0f;
 #pragma unroll
             for (int l = 0; l < L; ++l) {
                 if (l != (m.y >> 2 & 63)) continue;
-                const Quad f = m.y >> 8 == 1 ? o.vx[l] : o.vz[z_shared(L) ? 0 : l];
+                const Quad f = (m.y >> 8 & 255) == 1 ? o.vx[l] : o.vz[z_shared(L) ? 0 : l];
                 const int e = m.y & 3;
                 v = e == 0 ? f[0] : (e == 1 ? f[1] : (e == 2 ? f[2] : f[3]));
             }
@@ -928,8 +970,16 @@ __global__ void __launch_bounds__(MAXT, 1) k_resident(const __grid_constant__ Sf
         }
         __syncthreads();
         if (EXTRA) {
+            const unsigned short* list = reinterpret_cast<const unsigned short*>(smem + S.plist);
             for (int q = 0; q < x.n_plane; ++q) {
-                plane_op(a, S, g, x.ops[q], S.prev[q]);
+                const sf_plane_bc& op = x.ops[q];
+                const int ax = op.axis, cnt = plane_cells(ax, planes, b.nj, row);
+                const int stride = ax == 0 ? plane : (ax == 1 ? row : 1);
+                for (int side = 0; side < 2; ++side) {  // (an axis has 4 cells or more: no common ones)
+                    if (!has_plane(g, op, side)) continue;
+                    plane_op(op, x.coeff[q], list, cnt, side ? -stride : stride, S.prev[q][side]);
+                    list += cnt;
+                }
                 __syncthreads();
             }
             for (int q = 0; q < src.n; ++q) {

@@ -210,3 +210,29 @@ def test_what_acts_between_the_steps_against_single_steps(shape, boundary):
         for name in ("omni", "card", "edge"):
             np.testing.assert_array_equal(a.microphones[name].get_waveform(),
                                           b.microphones[name].get_waveform(), err_msg=name)
+
+
+@pytest.mark.parametrize("scale", [1e-2, 1e-20, 1e-36, 1e36])
+@pytest.mark.parametrize("courant", [0.6, 0.31])
+def test_absorbing_planes_round_as_in_fp64(scale, courant):
+    """The planes' FP64 operations in FP32 pairs, from magnitudes near both ends of
+    the range (overflow included) and over zeros: the bits of the per-step kernel."""
+    shape = (40, 37, 44)
+    rng = np.random.default_rng(8)
+    p0 = (rng.standard_normal(shape) * np.exp2(rng.integers(-20, 1, shape)) * scale).astype(np.float32)
+    p0[rng.random(shape) < 0.3] = 0.0
+    p0[:, :, 22:] *= rng.random() < 0.5
+    out = []
+    for kernel in (None, "tile1_r2_w8"):
+        s = S.FDTDSolver(shape=shape, resolution=1e-3, c=343.0, rho=1.2, courant=courant)
+        s.add_boundary(S.ABCFirstOrder())
+        if kernel:
+            s.set_kernel(kernel)
+        else:
+            assert _resident(s, 40)
+        s.p = p0.copy()
+        for n in (40, 9):
+            s.run_steps(n)
+        out.append(s)
+    with np.errstate(all="ignore"):
+        _check(*out, (scale, courant))
