@@ -672,6 +672,7 @@ int default_single(const SfStepArgs& a) {
 }
 bool pipe_fits(sf_plan* P, int cfg, const SfStepArgs& a);
 int chunk_for(const sf_plan* P, int cfg);
+int tbq_chunk(const sf_plan* P, const SfTbConfig& c, double* share);
 
 int effective_config(const sf_plan* P, const SfStepArgs& a) {
     int cfg;
@@ -693,6 +694,34 @@ int effective_config(const sf_plan* P, const SfStepArgs& a) {
     else if (P->poles.n > 0 && !tile_ok)
         cfg = SF_CFG_CELL;
     return cfg;
+}
+
+// The two-step configuration that the automatic choice takes for pairs of steps of
+// this plan, or -1.  It reads and writes the state once per two steps, but computes
+// its windows' overlaps twice, so it is taken where the share of its threads' cells
+// that are output is high enough.  Steps in us, pairs and the default single step, 20
+// rows without walls (96 registers), 16 with them (their masks spill at 96):
+//   walls   400^3 (share 0.83) 280 and 332, 300^3 (0.87) 124 and 148, 350 x 210 x 164
+//           (0.87) 55 and 72, 64 x 400 x 400 (0.76) 54.8 and 57.2, 128 x 128 x 400 (0.72)
+//           35.5 and 37.7, 203 x 167 x 184 (0.717) 37.0 and 37.1, 176 x 152 x 144 (0.696)
+//           24.1 and 23.3
+//   none    400^3 (0.87) 236 and 318, 256^3 (0.81) 67 and 84, 130 x 140 x 148 (0.72) 13.6
+//           and 14.9, 203 x 167 x 184 (0.65) 32.8 and 34.8
+// A plane source along y or z acts in every plane of the blocks it crosses, which
+// the others then wait for: those plans keep single steps.
+int default_pair(const sf_plan* P, const SfStepArgs& a) {
+    if (P->variant != SF_CFG_AUTO || P->tuned > 0 || P->i_chunk > 0 || !tb_fits(P, a) || !sf_tile_supported(a, 4))
+        return -1;
+    for (int q = 0; q < P->src.n; ++q)
+        if (P->src.s[q].kind != 0 && P->src.s[q].a != 0) return -1;
+    const bool walls = a.flags != nullptr;
+    for (int q = 0; q < kSfTbConfigCount; ++q) {
+        double share = 0.0;
+        if (kSfTbConfigs[q].quads == 0 || kSfTbConfigs[q].rows != (walls ? 16 : 20)) continue;
+        tbq_chunk(P, kSfTbConfigs[q], &share);
+        return share >= (walls ? 0.718 : 0.62) ? SF_CFG_TB_FIRST + q : -1;
+    }
+    return -1;
 }
 
 // The cells an ADE step gives to the per-cell kernel when warp-tile
@@ -728,6 +757,28 @@ void ade_region(const sf_plan* P, int cfg, int ich, int lo[3], int hi[3]) {
 // for the chunk's prologue), among those that fill one wave.  Against
 // auto_chunk alone (4 planes for these): 203 x 167 x 184 with walls 40.8 -> 39.9
 // us a step, 176 x 152 x 144 27.2 -> 26.3, free 300 x 90 x 120 20.5 -> 18.7.
+int tile_chunk(const sf_plan* P, const SfTileConfig& t);
+// Planes per block of a window configuration of the two-step kernel: the number of
+// chunks with the best product of (blocks / whole waves) and (planes / planes + 2
+// for the overlap and the lag).  *share: of the threads' cells, those that are
+// output and in the grid, over all blocks of the waves.
+int tbq_chunk(const sf_plan* P, const SfTbConfig& c, double* share) {
+    const int w = 4 * c.quads - 8, h = c.rows - 4;
+    const long long ck = (P->d.nz + w - 1) / w, cj = (P->d.ny + h - 1) / h, wave = (long long)c.minb * P->sms;
+    int best = P->d.nx;
+    double best_eff = 0.0;
+    for (int chunks = 1; chunks <= 64 && chunks <= P->d.nx; ++chunks) {
+        const int ich = (P->d.nx + chunks - 1) / chunks;
+        const long long blocks = ck * cj * ((P->d.nx + ich - 1) / ich), waves = (blocks + wave - 1) / wave;
+        const double eff = (double)blocks / (double)(waves * wave) * ich / (ich + 2.0);
+        if (eff > best_eff) {
+            best_eff = eff;
+            best = ich;
+        }
+    }
+    if (share) *share = best_eff * P->d.nz / (double)(ck * w) * P->d.ny / (double)(cj * h);
+    return best;
+}
 int tile_chunk(const sf_plan* P, const SfTileConfig& t) {
     const int jspan = 4 * t.rows * t.warps;
     const long long cols = (long long)((P->d.nz + 31) / 32) * ((P->d.ny + jspan - 1) / jspan);
@@ -755,6 +806,7 @@ int chunk_for(const sf_plan* P, int cfg) {
         return kSfPipeConfigs[cfg - SF_CFG_PIPE_FIRST].stream ? 4 : 2;
     if (is_tb(cfg)) {  // about four waves of blocks, chunks of at least 4 planes
         const SfTbConfig& c = kSfTbConfigs[cfg - SF_CFG_TB_FIRST];
+        if (c.quads > 0) return tbq_chunk(P, c, nullptr);
         int sms = 152;
         int dev = 0;
         if (cudaGetDevice(&dev) == cudaSuccess)
@@ -1186,8 +1238,13 @@ int sf_plan_step_ex(sf_plan* P, int64_t n_steps, const double* src_values, float
     const int levels = pipe ? kSfPipeConfigs[cfg0 - SF_CFG_PIPE_FIRST].levels : 1;
     const int pipe_S = pipe ? chunk_for(P, cfg0) : 0;
     // a two-step configuration runs pairs of steps under the same conditions
-    const bool tb = is_tb(cfg0) && !deferred && !mics;
-    const int tb_ich = tb ? chunk_for(P, cfg0) : 0;
+    const int pair = !deferred && !mics && n_steps >= 2 ? default_pair(P, a) : -1;
+    // an even number of pairs, so that the current set after n steps is the one after n
+    // single steps (a captured graph of an even number of steps ends where it began)
+    const int64_t pair_steps = n_steps & ~int64_t(3);
+    const int tb_cfg = pair >= 0 ? pair : cfg0;
+    const bool tb = is_tb(tb_cfg) && !deferred && !mics;
+    const int tb_ich = tb ? chunk_for(P, tb_cfg) : 0;
     const int cfg = (is_pipe(cfg0) || is_tb(cfg0)) ? SF_CFG_TILE_DEFAULT : cfg0;
     const int ich = chunk_for(P, cfg);
     SideBranch branch;  // (its events are host work: only where a graph keeps the edges)
@@ -1212,13 +1269,13 @@ int sf_plan_step_ex(sf_plan* P, int64_t n_steps, const double* src_values, float
             s += levels;
             continue;
         }
-        if (tb && n_steps - s >= 2) {
+        if (tb && (pair >= 0 ? s < pair_steps : n_steps - s >= 2)) {
             set_io(P, a, P->cur);
             a.src_val = P->src.n > 0 ? src_values + s * P->src.n : nullptr;
             a.trace_prev = (a.n_probe > 0 && s > 0) ? trace + (s - 1) * P->n_probe : nullptr;
             a.reverse = (int)((P->steps_done >> 1) & 1);
             float* t1 = a.n_probe > 0 ? trace + s * P->n_probe : nullptr;
-            if (int rc = sf_launch_step_tb(a, P->src, P->flags != nullptr, cfg0 - SF_CFG_TB_FIRST,
+            if (int rc = sf_launch_step_tb(a, P->src, P->flags != nullptr, tb_cfg - SF_CFG_TB_FIRST,
                                            tb_ich, t1, st))
                 return rc;
             P->cur = 1 - P->cur;

@@ -89,10 +89,13 @@ int sf_launch_step_stream(const SfPipeArgs& P, const SfSources& src, bool geom, 
 struct SfTbConfig {
     int rows, warps, minb;
     const char* name;
+    int quads;  // 0: warp tiles; else windows of `rows` x `quads` (k_step_tbq)
 };
 extern const SfTbConfig kSfTbConfigs[];
 extern const int kSfTbConfigCount;
 bool sf_tb_supported(const SfStepArgs& a);
+int sf_launch_step_tbq(const SfStepArgs& a, const SfSources& src, bool geom, int rows, int ich, float* trace1,
+                       cudaStream_t st);
 int sf_launch_step_tb(const SfStepArgs& a, const SfSources& src, bool geom, int cfg, int ich,
                       float* trace1, cudaStream_t st);
 

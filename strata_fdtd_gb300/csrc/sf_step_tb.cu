@@ -72,12 +72,16 @@ int launch_tb(const SfStepArgs& a, const SfSources& src, bool geom, int ich, flo
 
 }  // namespace
 
-// Two-step configurations: output rows per warp, warps per block, min blocks.
+// Two-step configurations: output rows per warp, warps per block, min blocks; and the
+// windows of k_step_tbq (rows, warps, blocks per SM, name, quads), which need aligned
+// rows and are replaced by the first configuration where they are not.
 const SfTbConfig kSfTbConfigs[] = {
     {4, 4, 3, "tb2_r4_w4"},
     {6, 4, 2, "tb2_r6_w4"},
     {4, 8, 1, "tb2_r4_w8"},
     {2, 8, 2, "tb2_r2_w8"},
+    {16, 8, 2, "tb2q_r16", 16},
+    {20, 10, 2, "tb2q_r20", 16},
 };
 const int kSfTbConfigCount = sizeof(kSfTbConfigs) / sizeof(kSfTbConfigs[0]);
 
@@ -89,6 +93,11 @@ bool sf_tb_supported(const SfStepArgs& a) {
 int sf_launch_step_tb(const SfStepArgs& a, const SfSources& src, bool geom, int cfg, int ich,
                       float* trace1, cudaStream_t st) {
     if (ich < 1) ich = 1;
+    if (kSfTbConfigs[cfg].quads > 0) {
+        if (sf_tile_supported(a, 4))
+            return sf_launch_step_tbq(a, src, geom, kSfTbConfigs[cfg].rows, ich, trace1, st);
+        cfg = 0;
+    }
     switch (cfg) {
         case 0: return launch_tb<4, 4, 3>(a, src, geom, ich, trace1, st);
         case 1: return launch_tb<6, 4, 2>(a, src, geom, ich, trace1, st);
