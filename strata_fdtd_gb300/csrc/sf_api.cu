@@ -1269,7 +1269,7 @@ int sf_plan_step_ex(sf_plan* P, int64_t n_steps, const double* src_values, float
             s += levels;
             continue;
         }
-        if (tb && (pair >= 0 ? s < pair_steps : n_steps - s >= 2)) {
+        if (tb && s < pair_steps) {
             set_io(P, a, P->cur);
             a.src_val = P->src.n > 0 ? src_values + s * P->src.n : nullptr;
             a.trace_prev = (a.n_probe > 0 && s > 0) ? trace + (s - 1) * P->n_probe : nullptr;
