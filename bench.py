@@ -16,7 +16,7 @@ the same metric through the public API with host-resident (pinned) fields
 uploaded and the pressure field and probe traces read back every bench step.
 ``roofline`` relates the fused step kernel to HBM bandwidth (33 algorithmic
 bytes per cell-update: 16 read + 16 written for p, vx, vy, vz, plus the 1-byte
-cell-flag read); ``cpu_baseline`` is the CPU oracle (the bit-exact C
+cell-flag read; half of that where a launch advances two steps); ``cpu_baseline`` is the CPU oracle (the bit-exact C
 restatement of the reference native kernels, OpenMP) on a bounded sample.
 
 --impl reference times that CPU implementation alone (all host threads) on
@@ -111,9 +111,9 @@ def replica_rate(world: int, cell_updates_per_rank: int, seconds: float) -> floa
     return world * cell_updates_per_rank / seconds / 1e9
 
 
-def profiled_traffic():
+def profiled_traffic(name):
     """DRAM bytes per launch of the step kernel from the committed ncu summary."""
-    path = os.path.join(ROOT, "profiles", "k_step_enclosure_400.md")
+    path = os.path.join(ROOT, "profiles", name)
     try:
         for line in open(path):
             if line.startswith("traffic_bytes_per_launch_400:"):
@@ -329,12 +329,16 @@ def run_gpu(args):
     # per bench step: the step kernels, and one probe gather per sf_plan_step
     # call or captured block of steps (run_steps replays 50-step graphs)
     G = S.FDTDSolver._GRAPH_STEPS if s._kernel_auto else inner + 1
-    launches = K * (inner + inner // G + (1 if inner % G else 0))
+    # (a two-step configuration takes an even number of pairs per call, then single steps)
+    pairs = (inner & ~3) // 2 if chosen.startswith("tb2") else 0
+    launches = K * (inner - pairs + inner // G + (1 if inner % G else 0))
     value = replica_rate(world, cells * inner * K, ms / 1e3)
     kernel_ms = ms / (K * inner)  # every timed launch attributed to the step kernel
     hbm, peak_kind = peaks()
-    achieved = BYTES_PER_CELL * cells / (kernel_ms / 1e3) / 1e9
-    traffic = profiled_traffic()
+    # a pass of two steps reads and writes the state once
+    bytes_per_cell = BYTES_PER_CELL * (1 - pairs / inner)
+    achieved = bytes_per_cell * cells / (kernel_ms / 1e3) / 1e9
+    traffic = profiled_traffic("k_step_tbq_enclosure.md" if pairs else "k_step_enclosure_400.md")
     s._mark_device_newer()
     s._step_count += (W + K) * inner
 
@@ -452,7 +456,7 @@ def run_gpu(args):
             "kernel": {"name": chosen, "i_chunk": args.ichunk, "autotune_ms_per_step": tune},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                          "frac": achieved / hbm, "traffic": traffic, "peak_kind": peak_kind,
-                         "bytes_per_cell": BYTES_PER_CELL,
+                         "bytes_per_cell": bytes_per_cell,
                          "kernel": f"fused step kernel, configuration {chosen}"},
             "cpu_baseline": cpu, "e2e": e2e, "gpu_launches": launches, "clocks": clk,
             "device": torch.cuda.get_device_name(local),
