@@ -756,9 +756,11 @@ int forward(const sf_diff_desc* d, const void* const* cv, void* const* set0, voi
     for (int64_t s = 0; s < n; ++s) {
         void* const* in = cur ? set1 : set0;
         void* const* out = cur ? set0 : set1;
-        auto kernel = narrow ? k_dfwd<T, int> : k_dfwd<T, long long>;
+        auto kernel = k_dfwd<T, long long>;
         dim3 grid = grid_of(d);
-        if constexpr (std::is_same<T, dwf>::value) {
+        if constexpr (!std::is_same<T, dwf>::value) {
+            if (narrow) kernel = k_dfwd<T, int>;
+        } else {
             if (narrow) {  // two cells per thread (32-bit cell indices)
                 grid = pair_grid(d);
                 kernel = pairs_aligned(d, {in[0], in[1], in[2], in[3], out[0], out[1], out[2], out[3], g.cvx,
@@ -805,9 +807,11 @@ int adjoint(const sf_diff_desc* d, const void* const* cv, void* const* lam0, voi
             inj.trace = tr + (s - 1) * d->n_probe;
             inj.target = tg + (s - 1) * d->n_probe;
         }
-        auto kernel = narrow ? k_dadj<T, int> : k_dadj<T, long long>;
+        auto kernel = k_dadj<T, long long>;
         dim3 grid = grid_of(d);
-        if constexpr (std::is_same<T, dwf>::value) {
+        if constexpr (!std::is_same<T, dwf>::value) {
+            if (narrow) kernel = k_dadj<T, int>;
+        } else {
             if (narrow) {
                 grid = pair_grid(d);
                 kernel = pairs_aligned(d, {in[0], in[1], in[2], in[3], out[0], out[1], out[2], out[3], g.cvx,

@@ -699,8 +699,10 @@ int effective_config(const sf_plan* P, const SfStepArgs& a) {
 // The two-step configuration that the automatic choice takes for pairs of steps of
 // this plan, or -1.  It reads and writes the state once per two steps, but computes
 // its windows' overlaps twice, so it is taken where the share of its threads' cells
-// that are output is high enough.  Steps in us, pairs and the default single step, 20
-// rows without walls (96 registers), 16 with them (their masks spill at 96):
+// that are output is high enough.  20 rows without walls (96 registers), 16 with
+// them (their masks spill at 96) unless 20 have 1.05 times the share (64 x 400 x 400
+// 52.3 against 55.5 us a step, 160 x 400 x 220 63.5 and 66.2; at 1.047 times, 400^3,
+// 293 and 279).  Pairs and the default single step:
 //   walls   400^3 (share 0.83) 280 and 332, 300^3 (0.87) 124 and 148, 350 x 210 x 164
 //           (0.87) 55 and 72, 64 x 400 x 400 (0.76) 54.8 and 57.2, 128 x 128 x 400 (0.72)
 //           35.5 and 37.7, 203 x 167 x 184 (0.717) 37.0 and 37.1, 176 x 152 x 144 (0.696)
@@ -715,13 +717,18 @@ int default_pair(const sf_plan* P, const SfStepArgs& a) {
     for (int q = 0; q < P->src.n; ++q)
         if (P->src.s[q].kind != 0 && P->src.s[q].a != 0) return -1;
     const bool walls = a.flags != nullptr;
+    int best = -1;
+    double best_share = 0.0;
     for (int q = 0; q < kSfTbConfigCount; ++q) {
+        if (kSfTbConfigs[q].quads == 0 || (!walls && kSfTbConfigs[q].rows != 20)) continue;
         double share = 0.0;
-        if (kSfTbConfigs[q].quads == 0 || kSfTbConfigs[q].rows != (walls ? 16 : 20)) continue;
         tbq_chunk(P, kSfTbConfigs[q], &share);
-        return share >= (walls ? 0.718 : 0.62) ? SF_CFG_TB_FIRST + q : -1;
+        if (best < 0 || share > 1.05 * best_share) {
+            best = q;
+            best_share = share;
+        }
     }
-    return -1;
+    return best >= 0 && best_share >= (walls ? 0.718 : 0.62) ? SF_CFG_TB_FIRST + best : -1;
 }
 
 // The cells an ADE step gives to the per-cell kernel when warp-tile
