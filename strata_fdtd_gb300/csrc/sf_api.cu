@@ -702,11 +702,10 @@ int effective_config(const sf_plan* P, const SfStepArgs& a) {
 // that are output is high enough.  20 rows without walls (96 registers), 16 with
 // them (their masks spill at 96) unless 20 have 1.05 times the share (64 x 400 x 400
 // 52.3 against 55.5 us a step, 160 x 400 x 220 63.5 and 66.2; at 1.047 times, 400^3,
-// 293 and 279).  Pairs and the default single step:
-//   walls   400^3 (share 0.83) 280 and 332, 300^3 (0.87) 124 and 148, 350 x 210 x 164
-//           (0.87) 55 and 72, 64 x 400 x 400 (0.76) 54.8 and 57.2, 128 x 128 x 400 (0.72)
-//           35.5 and 37.7, 203 x 167 x 184 (0.717) 37.0 and 37.1, 176 x 152 x 144 (0.696)
-//           24.1 and 23.3
+// 285 and 270).  Pairs and the default single step:
+//   walls   400^3 (share 0.83) 270 and 332, 300^3 (0.87) 115 and 148, 350 x 210 x 164
+//           (0.87) 50 and 72, 203 x 167 x 184 (0.717) 35.8 and 36.9, 150 x 150 x 152
+//           (0.716) 20.5 and 21.1, 176 x 152 x 144 (0.696) 23.7 and 23.4
 //   none    400^3 (0.87) 236 and 318, 256^3 (0.81) 67 and 84, 130 x 140 x 148 (0.72) 13.6
 //           and 14.9, 203 x 167 x 184 (0.65) 32.8 and 34.8
 // A plane source along y or z acts in every plane of the blocks it crosses, which
@@ -728,7 +727,7 @@ int default_pair(const sf_plan* P, const SfStepArgs& a) {
             best_share = share;
         }
     }
-    return best >= 0 && best_share >= (walls ? 0.718 : 0.62) ? SF_CFG_TB_FIRST + best : -1;
+    return best >= 0 && best_share >= (walls ? 0.71 : 0.62) ? SF_CFG_TB_FIRST + best : -1;
 }
 
 // The cells an ADE step gives to the per-cell kernel when warp-tile

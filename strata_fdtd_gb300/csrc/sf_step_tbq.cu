@@ -24,8 +24,9 @@
 // 400^3 with walls, us a step: 420 with loads in registers one plane ahead (one block
 // of 40 rows per SM), 368 in packed FP32, 333 and 320 (two blocks of 16 rows) with
 // the thread's own values kept in shared memory, 327 and 304 (24 rows) with the rings,
-// 277 with two blocks of 16 rows, own values in registers and the decays read ahead;
-// the single-step kernel takes 332.  Three and four blocks of 16 rows 312 to 448, 32
+// 277 with two blocks of 16 rows, own values in registers and the decays read ahead,
+// 270 with the next plane's velocities read behind the barrier before it; the
+// single-step kernel takes 332.  Three and four blocks of 16 rows 312 to 448, 32
 // to 64 rows 310 to 436, 32 quads 353 to 414.
 //
 // The per-cell operations are those of tile4_run (sf_tile.cuh), in the same order.
@@ -254,6 +255,9 @@ __global__ void __launch_bounds__(NQ* NR, MINB) k_step_tbq(SfStepArgs a, SfSourc
     copies_wait<2>();
     __syncthreads();
     Q4 P = lds4(r_p);
+    // with registers to spare, a plane's velocities are read behind the barrier before it
+    constexpr bool AHEAD = NT * MINB <= 512;
+    Q4 nx1 = lds4(r_v), ny1 = lds4(r_v + NT), nz1 = lds4(r_v + 2 * NT);
 
     for (int t = ts; t <= i1; ++t, c += plane) {
         const bool first = t < nx;
@@ -265,14 +269,14 @@ __global__ void __launch_bounds__(NQ* NR, MINB) k_step_tbq(SfStepArgs a, SfSourc
         if (first) {
             const float4* const s_p0 = r_p + sp * NT;
             const float4* const s_v = r_v + 3 * sv * NT;
-            x1 = lds4(s_v);
+            x1 = AHEAD ? nx1 : lds4(s_v);
             if (t < nx - 1) {
                 Pn = lds4(r_p + (sp + 1 & 3) * NT);
                 x1 = face(x1, Pn, P);
             }
-            y1 = lds4(s_v + NT);
+            y1 = AHEAD ? ny1 : lds4(s_v + NT);
             if (jf) y1 = face(y1, lds4(s_p0 + NQ), P);
-            z1 = zface(lds4(s_v + 2 * NT), P);
+            z1 = zface(AHEAD ? nz1 : lds4(s_v + 2 * NT), P);
             if (GEOM) Ft = r_f[sv * NT] | kept | (t == nx - 1 ? 0x01010101u * SF_OPX : 0u);
             walls = GEOM && __any_sync(kAll, Ft != kOpen4);
             if (walls) {
@@ -290,6 +294,7 @@ __global__ void __launch_bounds__(NQ* NR, MINB) k_step_tbq(SfStepArgs a, SfSourc
             if (walls) p1 = close4(p1, Ft, SF_AIR);
             p1 = dk * (dj * (pr(d_t, d_t) * p1));
             if (hot == t || hot == kEvery) p1 = inject(p1, val1, t, Ft);
+            sts4(s_p1, p1);
             for (unsigned m = pmask; m != 0; m &= m - 1) {
                 const int s = __ffs(m) - 1, w = (int)a.probe_cells[s] - c;
                 if (w >= 0 && w < 4) trace1[s] = p1.at(w);
@@ -314,13 +319,19 @@ __global__ void __launch_bounds__(NQ* NR, MINB) k_step_tbq(SfStepArgs a, SfSourc
             }
             u2x = x2;
         }
-        if (first) {
-            sts4(s_p1, p1);
-        }
         fetch_p(t, 4, sp);
         copies_commit();
         __syncthreads();
         // ---- 3
+        copies_wait<2>();
+        sp = sp + 1 & 3;
+        sv = sv == 2 ? 0 : sv + 1;
+        if (AHEAD) {
+            const float4* const s_v = r_v + 3 * sv * NT;
+            nx1 = lds4(s_v);
+            ny1 = lds4(s_v + NT);
+            nz1 = lds4(s_v + 2 * NT);
+        }
         if (first) {
             u2y = dj * y1;
             if (jf) u2y = face(u2y, lds4(s_p1 + NQ), p1);
@@ -338,9 +349,6 @@ __global__ void __launch_bounds__(NQ* NR, MINB) k_step_tbq(SfStepArgs a, SfSourc
         }
         d_prev = d_t;
         d_t = d_next;
-        sp = sp + 1 & 3;
-        sv = sv == 2 ? 0 : sv + 1;
-        copies_wait<2>();
     }
 }
 
