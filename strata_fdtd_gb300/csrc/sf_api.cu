@@ -128,7 +128,6 @@ extern "C" int sf_release_deferred(void) {
 // host-mapped error words, one per plan.
 namespace {
 constexpr int kResDevices = 64, kResSlots = 4096;
-constexpr size_t kResMailMax = size_t(64) << 20;
 constexpr int kResChunk = 4096;        // steps per launch
 constexpr int kResMinSteps = 8;        // shorter calls step launch by launch
 constexpr long long kResPolls = 1LL << 23;  // polls (about 0.5 us each) before a wait gives up
@@ -1126,8 +1125,7 @@ int step_resident(sf_plan* P, const SfStepArgs& a0, int64_t n_steps, const doubl
     const SfResCut& c = P->res_cut;
     SfResExtra x{};
     if (c.extra) resident_extra(P, mic_trace != nullptr, x);
-    const size_t mail = (size_t)2 * c.bi * c.bj * c.bk * 6 * c.side_max * 4 * sizeof(unsigned long long);
-    if (mail > kResMailMax) return sf_fail("k_resident: mailboxes too large");
+    const size_t mail = sf_resident_mail_bytes(c.bi * c.bj * c.bk, c.side_max);
     std::lock_guard<std::mutex> lock(g_res_mu);
     ResDevice& D = g_res[P->device];
     SF_CUDA_OK(cudaStreamWaitEvent(st, D.done, 0));

@@ -139,7 +139,7 @@ struct SfResCut {
     int bi, bj, bk;    // blocks along x, y, z
     int chunks, quads; // chunks of planes and quads of k cells in the grid
     int threads;
-    int side_max;      // message units of the largest block side
+    int side_max;      // message units of the largest block side that a cut crosses
     int units;         // message units of a block at most
     SfResLayout lay;
     size_t smem;
@@ -156,6 +156,11 @@ struct SfResArgs {
     int hold;          // expiry test hook: block 0 waits for tags nothing sends
     SfResExtra x;
 };
+// Both sets of mailboxes of a launch, and the most that a cut may need.
+constexpr size_t kSfResMailMax = size_t(64) << 20;
+inline size_t sf_resident_mail_bytes(int blocks, int side_max) {
+    return (size_t)2 * blocks * 6 * side_max * 4 * sizeof(unsigned long long);
+}
 SfResCut sf_resident_cut(int nx, int ny, int nz, int n_probe, bool nu, int sms, const SfResExtra* x);
 int sf_launch_resident_mics(const float* corners, const float* w, int n_mic, long long n_steps,
                             float* mic_trace, cudaStream_t st);

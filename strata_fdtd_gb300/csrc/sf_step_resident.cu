@@ -1112,13 +1112,17 @@ SfResCut sf_resident_cut(int nx, int ny, int nz, int n_probe, bool nu, int sms, 
                     if (x && !planes_fit(*x, nx, ny, nz, K.L, chunks, quads, bi, bj, bk)) continue;
                     const long long tiles = (long long)nci * nj * nq;
                     if (tiles > K.threads) continue;
-                    int units = 0, side = 0;
+                    // (only sides that a cut crosses have messages: 1000 x 1 x 1000 would
+                    // need 93 MB of mailboxes for its y sides, which nothing is sent over)
+                    int units = 0, side = 1;
                     const int split[3] = {bi, bj, bk};
                     for (int s = 0; s < 6; ++s) {
+                        if (split[s >> 1] == 1) continue;
                         const int n = side_units(s, nci * K.L, nj, nq);
-                        if (n > side) side = n;
-                        if (split[s >> 1] > 1) units += n;
+                        side = std::max(side, n);
+                        units += n;
                     }
+                    if (sf_resident_mail_bytes(bi * bj * bk, side) > kSfResMailMax) continue;
                     // the phases' cells, and the messages
                     const long long cost = (tiles + 31) / 32 * 32 * K.L + units;
                     if (best.kind >= 0 && cost >= best_cost) continue;

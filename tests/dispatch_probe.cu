@@ -1,0 +1,63 @@
+// Prints what the host-side dispatch of sf_api.cu decides, one line per line of
+// standard input, for the tests that need no GPU.  Plans are made here, for a
+// device of 152 SMs, with field pointers that nothing dereferences.
+#include "sf_api.cu"
+
+#include <cstdio>
+#include <iostream>
+#include <sstream>
+
+namespace {
+
+constexpr int kSms = 152;
+
+sf_plan plan_of(int nx, int ny, int nz, bool walls) {
+    sf_plan P;
+    P.d.nx = nx;
+    P.d.ny = ny;
+    P.d.nz = nz;
+    P.n = (long long)nx * ny * nz;
+    P.sms = kSms;
+    for (auto& set : P.f)
+        for (auto& f : set) f = reinterpret_cast<float*>(uintptr_t(4096));
+    if (walls) P.flags = reinterpret_cast<uint8_t*>(uintptr_t(4096));
+    return P;
+}
+
+void cut(std::istringstream& in) {  // nx ny nz probes nu planes: the state-on-chip cut
+    int nx, ny, nz, probes, nu, planes;
+    in >> nx >> ny >> nz >> probes >> nu >> planes;
+    SfResExtra x{};
+    x.n_plane = planes;
+    for (int q = 0; q < planes; ++q) x.ops[q].axis = q % 3;
+    const SfResCut c = sf_resident_cut(nx, ny, nz, probes, nu != 0, kSms, planes ? &x : nullptr);
+    std::printf("%d %d %d %d %d %d\n", c.kind, c.bi, c.bj, c.bk, c.side_max, c.threads);
+}
+
+void pair(std::istringstream& in) {  // nx ny nz walls plane_axis: the two-step choice
+    int nx, ny, nz, walls, axis;
+    in >> nx >> ny >> nz >> walls >> axis;
+    sf_plan P = plan_of(nx, ny, nz, walls != 0);
+    P.src.n = 1;
+    P.src.s[0].kind = axis >= 0;
+    P.src.s[0].a = axis >= 0 ? axis : 1;
+    SfStepArgs a;
+    fill_args(&P, a, false);
+    set_io(&P, a, 0);
+    const int c = default_pair(&P, a);
+    std::printf("%s\n", c < 0 ? "-" : sf_kernel_config_name(c));
+}
+
+}  // namespace
+
+int main() {
+    std::string line, what;
+    while (std::getline(std::cin, line)) {
+        std::istringstream in(line);
+        in >> what;
+        if (what == "cut") cut(in);
+        else if (what == "pair") pair(in);
+        else return 2;
+    }
+    return 0;
+}

@@ -1,0 +1,63 @@
+"""The dispatch rules on the host: which grids the state-on-chip kernel takes and
+how it cuts them, and where pairs of steps run.  The rules are compiled into a
+small program (dispatch_probe.cu) that answers for a device of 152 SMs; no GPU is
+used."""
+import os
+import random
+import subprocess
+
+import pytest
+
+from conftest import ROOT
+from strata_fdtd_gb300 import _native
+
+MAIL_MAX = 64 << 20  # bytes of mailboxes a launch may use
+
+
+@pytest.fixture(scope="session")
+def ask(tmp_path_factory):
+    lib = _native.build()
+    exe = str(tmp_path_factory.mktemp("dispatch") / "probe")
+    csrc = os.path.join(_native.PKG, "csrc")
+    subprocess.run([_native._nvcc(), _native.ARCH, "-O1", "-std=c++17", f"-I{csrc}",
+                    f"-I{os.path.join(ROOT, 'include')}",
+                    os.path.join(ROOT, "tests", "dispatch_probe.cu"), lib,
+                    "-Xlinker", f"-rpath={os.path.dirname(lib)}", "-o", exe],
+                   check=True, capture_output=True, text=True)
+
+    def run(lines):
+        out = subprocess.run([exe], input="\n".join(lines) + "\n", check=True,
+                             capture_output=True, text=True).stdout.splitlines()
+        assert len(out) == len(lines)
+        return [r.split() for r in out]
+
+    return run
+
+
+def _cuts(ask, shapes):
+    """(kind, mailbox bytes) per (nx, ny, nz, probes, nu, planes)."""
+    rows = ask(["cut %d %d %d %d %d %d" % s for s in shapes])
+    out = []
+    for r in rows:
+        kind, bi, bj, bk, side_max, _ = map(int, r)
+        out.append((kind, 2 * bi * bj * bk * 6 * side_max * 4 * 8))
+    return out
+
+
+def test_cuts_keep_their_mailboxes_within_the_limit(ask):
+    """Thin grids (a side that no cut crosses used to size the mailboxes) and
+    thick ones, uniform and stretched, with and without absorbing planes."""
+    rng = random.Random(4)
+    shapes = [(1000, 1, 1000), (1200, 1, 1200), (3000, 1, 400), (800, 2, 1000), (1, 1000, 1000),
+              (1000, 1000, 1), (2, 2, 200000), (65535, 3, 4), (1, 1, 4), (65535, 1, 30)]
+    for _ in range(150):
+        thin = rng.choice((1, 1, 2, 3))
+        a, b = (int(2 ** rng.uniform(2, 12)) for _ in range(2))
+        shapes.append(tuple(rng.sample((thin, a, b), 3)))
+    for _ in range(150):
+        shapes.append(tuple(int(2 ** rng.uniform(2, 9.2)) for _ in range(3)))
+    for extra in ((1, 0, 0), (1, 1, 0), (1, 0, 3)):
+        cuts = _cuts(ask, [s + extra for s in shapes])
+        assert sum(k >= 0 for k, _ in cuts) > 50
+        for s, (kind, mail) in zip(shapes, cuts):
+            assert kind < 0 or 0 < mail <= MAIL_MAX, (s, extra, mail)

@@ -1,0 +1,42 @@
+"""The state-on-chip kernel (k_resident) at the limits of what it takes."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+import strata_fdtd_gb300 as S  # noqa: E402
+from strata_fdtd_gb300 import _native  # noqa: E402
+
+from test_gpu_pipe import _check  # noqa: E402
+from test_gpu_resident import _fill, _resident  # noqa: E402
+
+
+@pytest.mark.parametrize("stretched", [False, True])
+@pytest.mark.parametrize("shape", [(1000, 1, 1000), (1200, 1, 1200), (3000, 1, 400), (800, 2, 1000),
+                                   (1, 900, 1100), (1000, 1000, 1)])
+def test_thin_grids_equal_single_steps(shape, stretched):
+    """Grids of one or two cells along an axis, up to 1.4 million cells: whole blocks
+    have no neighbour along it."""
+    out = []
+    rng = np.random.default_rng(shape[0])
+    coords = [np.cumsum(rng.uniform(0.7, 1.4, n)) * 1e-3 for n in shape]
+    for single in (False, True):
+        if stretched:
+            s = S.FDTDSolver(grid=S.NonuniformGrid(*coords), c=343.0, rho=1.2, courant=0.6)
+        else:
+            s = S.FDTDSolver(shape=shape, resolution=1e-3, c=343.0, rho=1.2, courant=0.6)
+        mask = np.ones(shape, bool)
+        mask[tuple(slice(n // 3, n // 3 + 40) if n > 2 else slice(0, 1) for n in shape)] = False
+        s.set_geometry(mask)
+        s.add_source(S.GaussianPulse(position=tuple(n // 2 for n in shape), frequency=20000.0))
+        s.add_probe("a", tuple(n - 1 for n in shape))
+        if single:
+            s.set_kernel("tile1_r2_w8")
+        out.append(s)
+    _fill(*out, 3)
+    assert _resident(out[0], 9)
+    for n in (9, 14):
+        for s in out:
+            s.run_steps(n)
+    _check(*out, shape)
