@@ -12,12 +12,15 @@ from test_gpu_pipe import _check  # noqa: E402
 from test_gpu_resident import _fill, _resident  # noqa: E402
 
 
-@pytest.mark.parametrize("stretched", [False, True])
-@pytest.mark.parametrize("shape", [(1000, 1, 1000), (1200, 1, 1200), (3000, 1, 400), (800, 2, 1000),
-                                   (1, 900, 1100), (1000, 1000, 1)])
-def test_thin_grids_equal_single_steps(shape, stretched):
+@pytest.mark.parametrize("shape,stretched,on_chip", [
+    ((1000, 1, 1000), False, True), ((1200, 1, 1200), False, True), ((3000, 1, 400), False, True),
+    ((800, 2, 1000), False, True), ((1, 900, 1100), False, False), ((1000, 1000, 1), False, False),
+    ((1, 250, 1100), False, True), ((900, 500, 1), False, True), ((800, 2, 1000), True, True),
+    ((2, 700, 900), True, False)])
+def test_thin_grids_equal_single_steps(shape, stretched, on_chip):
     """Grids of one or two cells along an axis, up to 1.4 million cells: whole blocks
-    have no neighbour along it."""
+    have no neighbour along it.  (One cell along x leaves a thread one plane, one along z
+    a quarter of its cells: fewer fit on the chip.)"""
     out = []
     rng = np.random.default_rng(shape[0])
     coords = [np.cumsum(rng.uniform(0.7, 1.4, n)) * 1e-3 for n in shape]
@@ -35,7 +38,7 @@ def test_thin_grids_equal_single_steps(shape, stretched):
             s.set_kernel("tile1_r2_w8")
         out.append(s)
     _fill(*out, 3)
-    assert _resident(out[0], 9)
+    assert _resident(out[0], 9) == on_chip
     for n in (9, 14):
         for s in out:
             s.run_steps(n)
