@@ -389,6 +389,18 @@ int sf_plan_set_nonuniform(sf_plan* P, const float* const* cv_face, const float*
     return 0;
 }
 
+namespace {
+// Whether a cell list names a cell twice (lists come sorted as a rule).
+bool lists_repeat(const int64_t* cells, int64_t n) {
+    int64_t q = 1;
+    while (q < n && cells[q - 1] < cells[q]) ++q;
+    if (q >= n) return false;
+    std::vector<int64_t> sorted(cells, cells + n);
+    std::sort(sorted.begin(), sorted.end());
+    return std::adjacent_find(sorted.begin(), sorted.end()) != sorted.end();
+}
+}  // namespace
+
 int sf_plan_set_weighted_source(sf_plan* P, int slot, int64_t n, const int64_t* cells,
                                 const double* weights) {
     if (!P) return sf_fail("sf_plan_set_weighted_source: NULL plan");
@@ -398,6 +410,7 @@ int sf_plan_set_weighted_source(sf_plan* P, int slot, int64_t n, const int64_t* 
         if (cells[q] < 0 || cells[q] >= P->n)
             return sf_fail("sf_plan_set_weighted_source: cell outside the grid");
     ++P->tables;
+    P->wsrc_repeats[slot] = lists_repeat(cells, n);
     int* box = P->wsrc_box[slot];
     for (int64_t q = 0; q < n; ++q) {
         const long long plane = (long long)P->d.ny * P->d.nz, r = cells[q] % plane;
@@ -1062,7 +1075,8 @@ int pipe_check(sf_plan* P, cudaStream_t st) {
 }
 
 // What acts between this plan's steps, for the state-on-chip kernel; false when
-// that kernel cannot do it (a source weighted on a velocity, too many rows).
+// that kernel cannot do it (a source weighted on a velocity, a list with a cell
+// twice, too many rows).
 bool resident_extra(const sf_plan* P, bool mics, SfResExtra& x) {
     x = SfResExtra{};
     x.n_plane = P->n_plane;
@@ -1076,7 +1090,8 @@ bool resident_extra(const sf_plan* P, bool mics, SfResExtra& x) {
     for (int q = 0; q < P->src.n; ++q) {
         const sf_source& S = P->src.s[q];
         if (S.kind != 2) continue;
-        if (S.b != 0 || P->wsrc_n[S.a] > INT_MAX) return false;
+        // (a block's list has room for each of its cells once per source)
+        if (S.b != 0 || P->wsrc_n[S.a] > INT_MAX || P->wsrc_repeats[S.a]) return false;
         x.wcells[q] = P->wsrc_cells[S.a];
         x.ww[q] = P->wsrc_w[S.a];
         x.wn[q] = (int)P->wsrc_n[S.a];

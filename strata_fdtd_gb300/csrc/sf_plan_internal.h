@@ -60,6 +60,7 @@ struct sf_plan {
     double* wsrc_w[SF_MAX_SOURCES] = {nullptr};
     long long wsrc_n[SF_MAX_SOURCES] = {0};
     int wsrc_box[SF_MAX_SOURCES][6];    // cells lo, hi (exclusive) per axis
+    bool wsrc_repeats[SF_MAX_SOURCES] = {false};  // some cell is listed twice
     long long tables = 0;               // bumped by the setters the state-on-chip cut depends on
     // multi-step pipeline (sf_step_pipe.cu)
     float* pipe_ring = nullptr;  // owned: rings of planes between levels

@@ -48,6 +48,21 @@ void pair(std::istringstream& in) {  // nx ny nz walls plane_axis: the two-step 
     std::printf("%s\n", c < 0 ? "-" : sf_kernel_config_name(c));
 }
 
+void weighted(std::istringstream& in) {  // nx ny nz, cells: whether the plan may stay on the chip
+    int nx, ny, nz;
+    in >> nx >> ny >> nz;
+    sf_plan P = plan_of(nx, ny, nz, false);
+    std::vector<int64_t> cells;
+    for (int64_t c; in >> c;) cells.push_back(c);
+    const std::vector<double> w(cells.size(), 1.0);
+    sf_plan_set_weighted_source(&P, 0, (int64_t)cells.size(), cells.data(), w.data());
+    P.wsrc_n[0] = (long long)cells.size();  // (without a device the tables' copies fail)
+    P.src.n = 1;
+    P.src.s[0].kind = 2;
+    SfResExtra x;
+    std::printf("%d\n", resident_extra(&P, false, x) ? 1 : 0);
+}
+
 }  // namespace
 
 int main() {
@@ -57,6 +72,7 @@ int main() {
         in >> what;
         if (what == "cut") cut(in);
         else if (what == "pair") pair(in);
+        else if (what == "weighted") weighted(in);
         else return 2;
     }
     return 0;

@@ -61,3 +61,11 @@ def test_cuts_keep_their_mailboxes_within_the_limit(ask):
         assert sum(k >= 0 for k, _ in cuts) > 50
         for s, (kind, mail) in zip(shapes, cuts):
             assert kind < 0 or 0 < mail <= MAIL_MAX, (s, extra, mail)
+
+
+def test_a_weighted_list_with_a_cell_twice_stays_off_the_chip(ask):
+    """A block's list has room for each of its cells once; a sorted list without
+    repeats, an unsorted one, and lists with a repeat in either."""
+    lists = ([5, 6, 7, 300], [300, 7, 5, 6], [5, 6, 6, 300], [300, 6, 5, 6], [9] * 1000, [4])
+    got = ask(["weighted 20 20 20 " + " ".join(map(str, c)) for c in lists])
+    assert [int(g[0]) for g in got] == [1, 1, 0, 0, 0, 1]
