@@ -300,13 +300,13 @@ class FDTDSolver:
         return int(self._lib.sf_plan_current(self._plan))
 
     def _field(self, name):
+        self._host_untouched[name] = False  # from here on, also where the read fails
         if not self._host_fresh[name]:
             src = self._dev[self._cur()][_FIELDS.index(name)]
             self._torch.from_numpy(self._host[name]).copy_(src)
             self._check_status()
             self._host_fresh[name] = True
         self._host_exposed[name] = True
-        self._host_untouched[name] = False
         self._vz_seen = self._vz_seen or name == "vz"
         return self._host[name]
 

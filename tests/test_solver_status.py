@@ -1,0 +1,55 @@
+"""What a solver does with a run that failed on the device (a bounded wait of the
+state-on-chip kernel that ran out), on a solver whose device is the CPU: fields are
+CPU tensors and the library's status is scripted."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+import strata_fdtd_gb300 as S  # noqa: E402
+from strata_fdtd_gb300 import _native  # noqa: E402
+
+FIELDS = ("p", "vx", "vy", "vz")
+SHAPE = (4, 3, 5)
+
+
+class _Lib:
+    """sf_plan_status answers from `status`, one value per call, then 0."""
+
+    def __init__(self, *status):
+        self.status = list(status)
+
+    def sf_plan_status(self, plan):
+        return self.status.pop(0) if self.status else 0
+
+    def sf_plan_current(self, plan):
+        return 0
+
+
+def _solver(*status):
+    """A solver behind a run that left 7 everywhere."""
+    s = S.FDTDSolver.__new__(S.FDTDSolver)
+    s._lib, s._torch, s._plan = _Lib(*status), torch, None
+    s._grid = S.UniformGrid(SHAPE, 1e-3)
+    s._dev = [[torch.full(SHAPE, 7.0) for _ in FIELDS] for _ in range(2)]
+    s._host = {f: np.zeros(SHAPE, dtype=np.float32) for f in FIELDS}
+    s._host_fresh = {f: False for f in FIELDS}
+    s._host_exposed = {f: False for f in FIELDS}
+    s._host_untouched = {f: True for f in FIELDS}
+    s._vz_seen = False
+    s._pending_traces, s._pending_mics = [], []
+    s._probes, s._microphones = {}, {}
+    s._boundaries, s._ade_debye, s._ade_lorentz = [], [], []
+    s._snap_staged, s._snap_inflight, s._snapshots = [], [], []
+    s._velocity_snapshots, s._energy_history = [], []
+    return s
+
+
+def test_a_read_that_failed_leaves_nothing_behind_a_reset():
+    s = _solver(1)
+    with pytest.raises(_native.NativeError):
+        s.p
+    s.reset()
+    for f in FIELDS:
+        assert not s._dev[0][FIELDS.index(f)].any()
+        np.testing.assert_array_equal(getattr(s, f), np.zeros(SHAPE, np.float32), err_msg=f)
