@@ -310,11 +310,40 @@ class FDTDSolver:
         self._vz_seen = self._vz_seen or name == "vz"
         return self._host[name]
 
-    def _check_status(self):
-        """Raise when an earlier asynchronous run of this solver failed."""
+    # A state-on-chip run whose wait ran out is reported once by the library, after
+    # the call that queued it has returned.  From then on the fields it left are void
+    # until reset() or until the host has given each of them again, and so are the
+    # traces and microphone rows not yet read, which are dropped.
+    _void = frozenset()  # those fields
+    _failures = 0        # failed runs seen so far (results under way compare it)
+    _failure = ""        # the last one's message
+
+    def _checked(self, rc: int, what: str, status: bool = False):
+        """Raise for a nonzero result of the library; that of a state-on-chip run
+        (any ``status``, else told by its message) is noted."""
+        try:
+            _native.check(rc, what)
+        except _native.NativeError as e:
+            if status or "k_resident: a dependency wait expired" in str(e):
+                self._failure = str(e)
+                self._failures += 1
+                self._void = {f for f in _FIELDS if not self._host_fresh[f]}
+                self._pending_traces.clear()
+                self._pending_mics = []
+            raise
+
+    def _check_status(self, since: int | None = None):
+        """Raise when an earlier asynchronous run of this solver failed and some of
+        its state is still in place, or when a run failed after ``since`` of them."""
         twin = getattr(self, "_pad_twin", None)
         for plan in (self._plan,) if twin is None else (self._plan, twin.plan):
-            _native.check(self._lib.sf_plan_status(plan), "sf_plan_step")
+            self._checked(self._lib.sf_plan_status(plan), "sf_plan_step", status=True)
+        if self._void or (since is not None and since != self._failures):
+            raise _native.NativeError(self._failure)
+
+    def _given(self, name):
+        """The host has given this field's state."""
+        self._void = self._void - {name}
 
     def _set_field(self, name, value):
         arr = np.asarray(value)
@@ -327,6 +356,7 @@ class FDTDSolver:
         self._host_exposed[name] = True
         self._host_untouched[name] = False
         self._vz_seen = self._vz_seen or name == "vz"
+        self._given(name)
 
     p = property(lambda s: s._field("p"), lambda s, v: s._set_field("p", v))
     vx = property(lambda s: s._field("vx"), lambda s, v: s._set_field("vx", v))
@@ -335,6 +365,7 @@ class FDTDSolver:
 
     def device_fields(self) -> dict:
         """The current state as CUDA tensors (no copy); valid until the next step."""
+        self._check_status()
         self._vz_seen = True  # the caller may write vz through the tensor
         self._upload_exposed()
         cur = self._cur()
@@ -363,6 +394,7 @@ class FDTDSolver:
             self._host_fresh[name] = False
             self._host_exposed[name] = False
             self._vz_seen = self._vz_seen or name == "vz"
+            self._given(name)
 
     def fields_async(self, names=_FIELDS, out: dict | None = None):
         """Start copying the named fields of the current state to pinned host
@@ -372,8 +404,9 @@ class FDTDSolver:
         shape per name to copy into (no allocation); the arrays must not be
         read before the function returns."""
         torch = self._torch
+        self._check_status()
         self._upload_exposed()
-        cur = self._cur()
+        cur, failures = self._cur(), self._failures
         dst = {}
         for name in names:
             src = self._dev[cur][_FIELDS.index(name)]
@@ -392,7 +425,7 @@ class FDTDSolver:
 
         def result() -> dict:
             done.synchronize()
-            self._check_status()
+            self._check_status(failures)
             return {n: t.numpy() for n, t in dst.items()}
 
         return result
@@ -921,7 +954,7 @@ class FDTDSolver:
                 plan, n - n_graph, None if src_dev is None else src_dev[n_graph:].data_ptr(),
                 None if trace is None else trace[n_graph:].data_ptr(),
                 None if mic_trace is None else mic_trace.data_ptr(), self._stream())
-            _native.check(rc, "sf_plan_step")
+            self._checked(rc, "sf_plan_step")
         if twin is not None:
             twin.copy_out(self)
         if trace is not None:
@@ -936,21 +969,25 @@ class FDTDSolver:
         self._step_count += n
 
     def _flush_traces(self):
-        for trace, names in self._pending_traces:
+        self._check_status()
+        while self._pending_traces:  # off the list as they are appended
+            trace, names = self._pending_traces[0]
             host = trace.cpu().numpy()
             self._check_status()
+            del self._pending_traces[0]
             for q, name in enumerate(names):
                 if name in self._probes:
                     self._probes[name]._samples.extend(host[:, q].tolist())
-        self._pending_traces.clear()
-        for trace, layout, times in getattr(self, "_pending_mics", []):
+        while self._pending_mics:
+            trace, layout, times = self._pending_mics[0]
             host = trace.cpu().numpy()
+            self._check_status()
+            del self._pending_mics[0]
             q = 0
             for name, n_rows in layout:
                 if name in self._microphones:
                     self._microphones[name]._append(host[:, q:q + n_rows], times)
                 q += n_rows
-        self._pending_mics = []
 
     def step(self) -> None:
         """Advance one time step (core/solver.py:2003-2077)."""
@@ -1142,7 +1179,9 @@ class FDTDSolver:
         return a function that waits for those copies only (not for work
         queued later on the stream) and returns get_probe_data()'s dict."""
         torch = self._torch
+        self._check_status()
         copies = []
+        failures = self._failures
         stream = torch.cuda.current_stream(self._device)
         for trace, names in self._pending_traces:
             host = torch.empty(trace.shape, dtype=trace.dtype, pin_memory=True)
@@ -1157,7 +1196,7 @@ class FDTDSolver:
 
         def result() -> dict:
             done.synchronize()
-            self._check_status()
+            self._check_status(failures)
             for host, names in copies:
                 arr = host.numpy()
                 for q, name in enumerate(names):
@@ -1178,10 +1217,12 @@ class FDTDSolver:
 
     def get_snapshots(self):
         self._snap_collect()
+        self._check_status()
         return self._snapshots
 
     def get_velocity_snapshots(self):
         self._snap_collect()
+        self._check_status()
         return self._velocity_snapshots
 
     def compute_energy(self) -> float:
@@ -1193,9 +1234,10 @@ class FDTDSolver:
         if self._energy_scratch is None or self._energy_scratch.numel() < need:
             self._energy_scratch = torch.empty(need, dtype=torch.float64, device=self._device)
         out = ctypes.c_double()  # without a geometry every cell counts as air
-        _native.check(self._lib.sf_plan_energy(self._plan, float(self.rho), float(self.c),
+        self._checked(self._lib.sf_plan_energy(self._plan, float(self.rho), float(self.c),
                                                float(self.dx), self._energy_scratch.data_ptr(),
                                                ctypes.byref(out), self._stream()), "sf_plan_energy")
+        self._check_status()
         return float(out.value)
 
     def get_energy_history(self):
@@ -1215,6 +1257,10 @@ class FDTDSolver:
 
     def reset(self) -> None:
         """core/solver.py:2781-2800."""
+        try:
+            self._check_status()  # a failed run ends here
+        except _native.NativeError:
+            pass
         for s in self._dev:
             for t in s:
                 t.zero_()
@@ -1225,6 +1271,7 @@ class FDTDSolver:
                 self._host[f].fill(0)
             self._host_fresh[f] = True
             self._host_exposed[f] = False
+            self._given(f)
         self._step_count = 0
         self._time = 0.0
         self._src_cache = None

@@ -43,3 +43,32 @@ def test_thin_grids_equal_single_steps(shape, stretched, on_chip):
         for s in out:
             s.run_steps(n)
     _check(*out, shape)
+
+
+@pytest.mark.parametrize("read", ["microphone", "field", "async", "energy"])
+def test_an_expired_wait_is_seen_by_every_read(read):
+    """The bounded wait's test hook on a solver with a microphone and no probe: what is
+    read first raises, so does what is read after it, and a run from a reset is exact."""
+    def build():
+        s = S.FDTDSolver(shape=(40, 41, 44), resolution=1e-3, c=343.0, rho=1.2, courant=0.6)
+        s.add_source(S.GaussianPulse(position=(20, 20, 20), frequency=20000.0))
+        s.add_microphone(position=(0.021, 0.019, 0.022), name="m")
+        return s
+
+    reads = {"microphone": lambda s: s.microphones["m"].get_waveform(), "field": lambda s: s.p,
+             "async": lambda s: s.fields_async(("p",))(), "energy": lambda s: s.compute_energy()}
+    s, ref = build(), build()
+    lib = _native.load()
+    _native.check(lib.sf_plan_set_wait_limit(s._plan, 2000, 1), "sf_plan_set_wait_limit")
+    s.run_steps(10)
+    for q in [read] + sorted(reads):
+        with pytest.raises(_native.NativeError, match="dependency wait expired"):
+            reads[q](s)
+    _native.check(lib.sf_plan_set_wait_limit(s._plan, 0, 0), "sf_plan_set_wait_limit")
+    s.reset()
+    for q in ("p", "vx", "vy", "vz"):
+        assert not getattr(s, q).any()
+    s.run_steps(10)
+    ref.run_steps(10)
+    _check(s, ref, read)
+    np.testing.assert_array_equal(reads["microphone"](s), reads["microphone"](ref))
