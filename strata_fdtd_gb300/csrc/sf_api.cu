@@ -122,7 +122,7 @@ extern "C" int sf_release_deferred(void) {
 // ---- state-on-chip launches (sf_step_resident.cu) ---------------------------
 //
 // Per device: the mailboxes every launch uses (grown on demand, released with
-// the deferred frees when idle), the next message tag, an event that orders the
+// the deferred frees), the next message tag, an event that orders the
 // launches of all streams and threads one after another (each takes every SM
 // its cut names, so two at once could wait for each other's SMs), and a page of
 // host-mapped error words, one per plan.
@@ -197,8 +197,9 @@ void resident_release() {
     std::lock_guard<std::mutex> lock(g_res_mu);
     for (int d = 0; d < kResDevices; ++d) {
         ResDevice& D = g_res[d];
-        if (!D.mail || cudaEventQuery(D.done) != cudaSuccess) continue;
+        if (!D.mail && !D.corners) continue;
         DeviceGuard g(d);
+        cudaEventSynchronize(D.done);  // the launches that use them
         cudaFree(D.mail);
         D.mail = nullptr;
         D.bytes = 0;

@@ -72,3 +72,35 @@ def test_an_expired_wait_is_seen_by_every_read(read):
     ref.run_steps(10)
     _check(s, ref, read)
     np.testing.assert_array_equal(reads["microphone"](s), reads["microphone"](ref))
+
+
+def test_buffers_are_released_behind_a_run_in_flight():
+    """sf_release_deferred() while the state-on-chip kernel runs: it waits for the run,
+    and leaves no error behind for the next launch."""
+    lib = _native.load()
+
+    def build(kernel=None):
+        s = S.FDTDSolver(shape=(96, 92, 100), resolution=1e-3, c=343.0, rho=1.2, courant=0.6)
+        s.add_source(S.GaussianPulse(position=(40, 41, 42), frequency=20000.0))
+        s.add_probe("a", (50, 50, 50))
+        if kernel:
+            s.set_kernel(kernel)
+        return s
+
+    a, b, c, ref = build(), build("col4"), build(), build("col4")
+    assert _resident(a, 40000)
+    for s in (b, ref):
+        s.run_steps(1)
+    a.run_steps(9)
+    torch.cuda.synchronize()
+    _native.check(lib.sf_release_deferred())  # (nothing else is queued for release)
+    a.run_steps(9)
+    a.run_steps(40000)  # about 0.16 s
+    _native.check(lib.sf_release_deferred())
+    assert torch.cuda.current_stream().query()
+    b.run_steps(8)
+    ref.run_steps(8)
+    c.run_steps(9)  # new mailboxes
+    _check(b, ref, "behind the release")
+    _check(c, ref, "new mailboxes")
+    a.synchronize()
