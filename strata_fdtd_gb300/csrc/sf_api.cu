@@ -1145,6 +1145,16 @@ int step_resident(sf_plan* P, const SfStepArgs& a0, int64_t n_steps, const doubl
     std::lock_guard<std::mutex> lock(g_res_mu);
     ResDevice& D = g_res[P->device];
     SF_CUDA_OK(cudaStreamWaitEvent(st, D.done, 0));
+    struct Behind {  // the event moves behind what is queued here, also when a later launch fails
+        cudaEvent_t done;
+        cudaStream_t st;
+        cudaError_t record() {
+            const cudaError_t e = done ? cudaEventRecord(done, st) : cudaSuccess;
+            done = nullptr;
+            return e;
+        }
+        ~Behind() { (void)record(); }
+    } behind{D.done, st};
     if (D.bytes < mail) {
         cudaFree(D.mail);  // waits for the launches that use it
         D.mail = nullptr;
@@ -1196,7 +1206,7 @@ int step_resident(sf_plan* P, const SfStepArgs& a0, int64_t n_steps, const doubl
         P->steps_done += n;
         s += n;
     }
-    SF_CUDA_OK(cudaEventRecord(D.done, st));
+    SF_CUDA_OK(behind.record());
     return 0;
 }
 

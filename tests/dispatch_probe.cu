@@ -1,11 +1,45 @@
 // Prints what the host-side dispatch of sf_api.cu decides, one line per line of
 // standard input, for the tests that need no GPU.  Plans are made here, for a
 // device of 152 SMs, with field pointers that nothing dereferences.
-#include "sf_api.cu"
+//
+// The state-on-chip launches run here too, against calls that are only listed.
+#include <cuda_runtime.h>
 
+#include <cstdint>
 #include <cstdio>
 #include <iostream>
 #include <sstream>
+#include <string>
+
+namespace probe {
+
+std::string calls;        // what was called, in order
+int launches_left = 1000;  // launches that succeed
+
+cudaError_t note(const char* what) {
+    calls += what;
+    calls += ' ';
+    return cudaSuccess;
+}
+template <class T>
+cudaError_t malloc(T** p, size_t) {
+    *p = reinterpret_cast<T*>(uintptr_t(1) << 20);
+    return note("malloc");
+}
+
+}  // namespace probe
+
+#define cudaStreamWaitEvent(...) probe::note("wait")
+#define cudaEventRecord(...) probe::note("record")
+#define cudaMalloc(...) probe::malloc(__VA_ARGS__)
+#define cudaFree(...) probe::note("free")
+#define cudaMemsetAsync(...) probe::note("clear")
+#include "sf_api.cu"
+
+int sf_launch_resident(SfResArgs&, const SfSources&, const SfResCut&, cudaStream_t) {
+    probe::note("launch");
+    return --probe::launches_left >= 0 ? 0 : sf_fail("launch failed");
+}
 
 namespace {
 
@@ -63,6 +97,20 @@ void weighted(std::istringstream& in) {  // nx ny nz, cells: whether the plan ma
     std::printf("%d\n", resident_extra(&P, false, x) ? 1 : 0);
 }
 
+void steps(std::istringstream& in) {  // nx ny nz, steps, launches that succeed: the calls made
+    int nx, ny, nz, n;
+    in >> nx >> ny >> nz >> n >> probe::launches_left;
+    sf_plan P = plan_of(nx, ny, nz, false);
+    SfStepArgs a;
+    fill_args(&P, a, false);
+    P.res_cut = sf_resident_cut(nx, ny, nz, 0, false, kSms, nullptr);
+    g_res[0] = ResDevice{};
+    g_res[0].done = reinterpret_cast<cudaEvent_t>(uintptr_t(4096));
+    probe::calls.clear();
+    const int rc = step_resident(&P, a, n, nullptr, nullptr, nullptr, nullptr);
+    std::printf("%s%d\n", probe::calls.c_str(), rc);
+}
+
 }  // namespace
 
 int main() {
@@ -73,6 +121,7 @@ int main() {
         if (what == "cut") cut(in);
         else if (what == "pair") pair(in);
         else if (what == "weighted") weighted(in);
+        else if (what == "steps") steps(in);
         else return 2;
     }
     return 0;

@@ -69,3 +69,12 @@ def test_a_weighted_list_with_a_cell_twice_stays_off_the_chip(ask):
     lists = ([5, 6, 7, 300], [300, 7, 5, 6], [5, 6, 6, 300], [300, 6, 5, 6], [9] * 1000, [4])
     got = ask(["weighted 20 20 20 " + " ".join(map(str, c)) for c in lists])
     assert [int(g[0]) for g in got] == [1, 1, 0, 0, 0, 1]
+
+
+@pytest.mark.parametrize("succeed", [3, 2, 1])
+def test_launches_are_ordered_behind_one_that_was_queued_before_a_failure(ask, succeed):
+    """The event that orders the launches of all streams, and that the mailboxes' release
+    waits for, is recorded behind what was queued, also where a later launch fails."""
+    (calls,) = ask(["steps 40 40 40 9000 %d" % succeed])
+    assert calls[0] == "wait" and calls.count("launch") == min(3, succeed + 1)
+    assert calls[-2] == "record" and int(calls[-1]) == (0 if succeed == 3 else 1)
