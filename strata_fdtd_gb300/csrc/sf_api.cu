@@ -152,6 +152,7 @@ bool resident_slot(sf_plan* P) {
     std::lock_guard<std::mutex> lock(g_res_mu);
     ResDevice& D = g_res[P->device];
     if (!D.err_host) {
+        SfRelaxedCapture relaxed;
         void* h = nullptr;
         if (cudaHostAlloc(&h, sizeof(int) * kResSlots, cudaHostAllocMapped | cudaHostAllocPortable) !=
             cudaSuccess) {
@@ -1155,8 +1156,11 @@ int step_resident(sf_plan* P, const SfStepArgs& a0, int64_t n_steps, const doubl
         }
         ~Behind() { (void)record(); }
     } behind{D.done, st};
+    // (outgrown buffers are queued for release: launches in flight use them, and
+    // cudaFree would wait for everything on the device)
     if (D.bytes < mail) {
-        cudaFree(D.mail);  // waits for the launches that use it
+        SfRelaxedCapture relaxed;
+        sf_defer_free(D.mail, D.bytes);
         D.mail = nullptr;
         D.bytes = 0;
         SF_CUDA_OK(cudaMalloc(&D.mail, mail));
@@ -1166,7 +1170,8 @@ int step_resident(sf_plan* P, const SfStepArgs& a0, int64_t n_steps, const doubl
     if (x.n_mic > 0) {
         const size_t need = sizeof(float) * 8 * x.n_mic * (size_t)std::min<int64_t>(kResChunk, n_steps);
         if (D.corner_bytes < need) {
-            cudaFree(D.corners);
+            SfRelaxedCapture relaxed;
+            sf_defer_free(D.corners, D.corner_bytes);
             D.corners = nullptr;
             D.corner_bytes = 0;
             SF_CUDA_OK(cudaMalloc(&D.corners, need));

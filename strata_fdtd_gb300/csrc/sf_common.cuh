@@ -71,6 +71,17 @@ struct SfStepArgs {
     const float* nu_inv[3];           // nonuniform grid: cell inverse spacings per axis
 };
 
+// While it lives, this thread may allocate, free and wait although another thread is
+// capturing a graph in the global mode (which forbids such calls in every thread, and
+// drops the other's capture when one is made).
+struct SfRelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    SfRelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~SfRelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+    SfRelaxedCapture(const SfRelaxedCapture&) = delete;
+    SfRelaxedCapture& operator=(const SfRelaxedCapture&) = delete;
+};
+
 // Programmatic dependent launch: a kernel launched with launch_dependent may be
 // set up while the kernel before it on the stream drains, and calls
 // await_previous() before it touches anything that kernel wrote (or reads).  Every

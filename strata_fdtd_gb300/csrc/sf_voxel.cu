@@ -54,6 +54,7 @@
 #include <vector>
 
 #include "sf_common.cuh"
+#include "sf_plan_internal.h"
 
 namespace {
 
@@ -1097,11 +1098,11 @@ class Scratch {
             std::lock_guard<std::mutex> lock(g_keep_mu);
             Kept& k = g_keep[dev_];
             if (!k.lent) {
-                if (k.bytes < bytes) {  // at least doubled: cudaFree waits for the device
+                if (k.bytes < bytes) {  // at least doubled; the old one is queued for release
                     size_t grown = 2 * k.bytes < (size_t(1) << 20) ? size_t(1) << 20 : 2 * k.bytes;
                     if (grown < bytes) grown = bytes;
                     if (grown > kKeepBytes) grown = kKeepBytes;
-                    if (k.p) cudaFree(k.p);
+                    sf_defer_free(k.p, k.bytes);
                     k = Kept{};
                     if (cudaMalloc(&k.p, grown) == cudaSuccess) k.bytes = grown;
                     else (void)cudaGetLastError();
@@ -1184,6 +1185,7 @@ int sf_launch_voxelize(const sf_sdf_node* nodes, int n_nodes, int nx, int ny, in
             o += sizeof(double) * n3[a];
         }
     }
+    SfRelaxedCapture relaxed;  // (the call allocates and waits)
     Scratch scratch;
     if (int rc = scratch.take(off_q + sizeof(unsigned) * (size_t)blocks, st)) return rc;
     char* b = scratch.p;

@@ -34,6 +34,7 @@ cudaError_t malloc(T** p, size_t) {
 #define cudaMalloc(...) probe::malloc(__VA_ARGS__)
 #define cudaFree(...) probe::note("free")
 #define cudaMemsetAsync(...) probe::note("clear")
+#define cudaThreadExchangeStreamCaptureMode(...) probe::note("mode")
 #include "sf_api.cu"
 
 int sf_launch_resident(SfResArgs&, const SfSources&, const SfResCut&, cudaStream_t) {
@@ -104,7 +105,6 @@ void steps(std::istringstream& in) {  // nx ny nz, steps, launches that succeed:
     SfStepArgs a;
     fill_args(&P, a, false);
     P.res_cut = sf_resident_cut(nx, ny, nz, 0, false, kSms, nullptr);
-    g_res[0] = ResDevice{};
     g_res[0].done = reinterpret_cast<cudaEvent_t>(uintptr_t(4096));
     probe::calls.clear();
     const int rc = step_resident(&P, a, n, nullptr, nullptr, nullptr, nullptr);

@@ -78,3 +78,13 @@ def test_launches_are_ordered_behind_one_that_was_queued_before_a_failure(ask, s
     (calls,) = ask(["steps 40 40 40 9000 %d" % succeed])
     assert calls[0] == "wait" and calls.count("launch") == min(3, succeed + 1)
     assert calls[-2] == "record" and int(calls[-1]) == (0 if succeed == 3 else 1)
+
+
+def test_outgrown_mailboxes_are_queued_for_release(ask):
+    """Mailboxes grow without cudaFree, which would wait for the device, and are
+    allocated in the relaxed capture mode."""
+    small, large, again = ask(["steps 20 20 20 9 1000", "steps 100 100 100 9 1000",
+                               "steps 20 20 20 9 1000"])
+    for calls in (small, large):
+        assert calls == "wait mode malloc mode clear launch record 0".split()
+    assert again == "wait launch record 0".split()
