@@ -402,32 +402,38 @@ int sf_launch_step(const SfStepArgs& a, const SfSources& src, const SfPoles& pol
     if (ex <= 0 || ey <= 0 || ez <= 0) return 0;
     dim3 blk(BX, BY, 1), grd((ez + BX - 1) / BX, (ey + BY - 1) / BY, ex);
     const bool ade = poles.n > 0;
+    // Behind the density pass this launch has that one predecessor; without it, on a
+    // branch (a.serial) it has the two that the branch forks from, and is plain.
+    bool dependent = !a.serial;
     if (ade && poles.n_density > 0) {
         const long long n = (long long)(a.ade_hi[0] - a.ade_lo[0]) * (a.ade_hi[1] - a.ade_lo[1]) *
                             (a.ade_hi[2] - a.ade_lo[2]);
         const int blocks = (int)((n + 255) / 256 < 152 * 16 ? (n + 255) / 256 : 152 * 16);
-        if (n > 0 && launch_kernel(!a.serial, k_ade_density, dim3(blocks), dim3(256), st, a, poles, n) != cudaSuccess)
-            return sf_fail("k_ade_density launch failed");
+        if (n > 0) {
+            if (launch_kernel(!a.serial, k_ade_density, dim3(blocks), dim3(256), st, a, poles, n) != cudaSuccess)
+                return sf_fail("k_ade_density launch failed");
+            dependent = true;
+        }
     }
     const bool nu = a.nu_cv[0] != nullptr;
     cudaError_t rc;
     if (nu) {
         if (geom)
-            ade ? rc = launch_dependent(k_step<true, true, true>, grd, blk, st, a, src, poles)
-                : rc = launch_dependent(k_step<true, false, true>, grd, blk, st, a, src, poles);
+            ade ? rc = launch_kernel(dependent, k_step<true, true, true>, grd, blk, st, a, src, poles)
+                : rc = launch_kernel(dependent, k_step<true, false, true>, grd, blk, st, a, src, poles);
         else
-            ade ? rc = launch_dependent(k_step<false, true, true>, grd, blk, st, a, src, poles)
-                : rc = launch_dependent(k_step<false, false, true>, grd, blk, st, a, src, poles);
+            ade ? rc = launch_kernel(dependent, k_step<false, true, true>, grd, blk, st, a, src, poles)
+                : rc = launch_kernel(dependent, k_step<false, false, true>, grd, blk, st, a, src, poles);
     } else if (geom) {
         if (ade)
-            rc = launch_dependent(k_step<true, true, false>, grd, blk, st, a, src, poles);
+            rc = launch_kernel(dependent, k_step<true, true, false>, grd, blk, st, a, src, poles);
         else
-            rc = launch_dependent(k_step<true, false, false>, grd, blk, st, a, src, poles);
+            rc = launch_kernel(dependent, k_step<true, false, false>, grd, blk, st, a, src, poles);
     } else {
         if (ade)
-            rc = launch_dependent(k_step<false, true, false>, grd, blk, st, a, src, poles);
+            rc = launch_kernel(dependent, k_step<false, true, false>, grd, blk, st, a, src, poles);
         else
-            rc = launch_dependent(k_step<false, false, false>, grd, blk, st, a, src, poles);
+            rc = launch_kernel(dependent, k_step<false, false, false>, grd, blk, st, a, src, poles);
     }
     return rc == cudaSuccess ? 0 : sf_fail("k_step launch failed");
 }

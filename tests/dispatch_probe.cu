@@ -27,6 +27,11 @@ cudaError_t malloc(T** p, size_t) {
     return note("malloc");
 }
 
+template <class... A>
+cudaError_t launch(const cudaLaunchConfig_t* cfg, A...) {
+    return note(cfg->numAttrs > 0 ? "dependent" : "plain");
+}
+
 }  // namespace probe
 
 #define cudaStreamWaitEvent(...) probe::note("wait")
@@ -35,7 +40,9 @@ cudaError_t malloc(T** p, size_t) {
 #define cudaFree(...) probe::note("free")
 #define cudaMemsetAsync(...) probe::note("clear")
 #define cudaThreadExchangeStreamCaptureMode(...) probe::note("mode")
+#define cudaLaunchKernelEx(...) probe::launch(__VA_ARGS__)
 #include "sf_api.cu"
+#include "sf_step.cu"
 
 int sf_launch_resident(SfResArgs&, const SfSources&, const SfResCut&, cudaStream_t) {
     probe::note("launch");
@@ -111,6 +118,21 @@ void steps(std::istringstream& in) {  // nx ny nz, steps, launches that succeed:
     std::printf("%s%d\n", probe::calls.c_str(), rc);
 }
 
+void ade(std::istringstream& in) {  // density poles, modulus poles, serial: the launches of a step
+    SfPoles poles{};
+    int serial;
+    in >> poles.n_density >> poles.n_modulus >> serial;
+    poles.n = poles.n_density + poles.n_modulus;
+    sf_plan P = plan_of(20, 20, 80, false);
+    for (int q = 0; q < 3; ++q) P.ade_hi[q] = 10;
+    SfStepArgs a;
+    fill_args(&P, a, false);
+    a.serial = serial;
+    probe::calls.clear();
+    const int rc = sf_launch_step(a, SfSources{}, poles, false, nullptr);
+    std::printf("%s%d\n", probe::calls.c_str(), rc);
+}
+
 }  // namespace
 
 int main() {
@@ -122,6 +144,7 @@ int main() {
         else if (what == "pair") pair(in);
         else if (what == "weighted") weighted(in);
         else if (what == "steps") steps(in);
+        else if (what == "ade") ade(in);
         else return 2;
     }
     return 0;

@@ -88,3 +88,11 @@ def test_outgrown_mailboxes_are_queued_for_release(ask):
     for calls in (small, large):
         assert calls == "wait mode malloc mode clear launch record 0".split()
     assert again == "wait launch record 0".split()
+
+
+def test_launches_behind_a_fork_are_plain(ask):
+    """On a branch (serial) the first launch of an ADE step has two predecessors and must
+    not be a dependent one; the step kernel behind the density pass may be."""
+    got = ask(["ade 1 1 1", "ade 0 2 1", "ade 2 0 1", "ade 1 1 0", "ade 0 2 0"])
+    assert [" ".join(g) for g in got] == ["plain dependent 0", "plain 0", "plain dependent 0",
+                                          "dependent dependent 0", "dependent 0"]

@@ -38,3 +38,21 @@ def test_captured_ade_steps_equal_single_steps(name):
     assert list(ta) == list(tb)
     for k in ta:
         np.testing.assert_array_equal(ta[k], tb[k])
+
+
+MODULUS_ONLY = dict(
+    shape=(40, 45, 140), res=1e-3, courant=0.5, pml=dict(depth=5),
+    materials=[dict(id=2, name="m2", rho=1.3, c=330.0, poles=[("debye", "modulus", 0.3, 4e-4)],
+                    box=((19, 31), (13, 27), (33, 47))),
+               dict(id=5, name="m5", rho=1.1, c=355.0,
+                    poles=[("lorentz", "modulus", 0.15, 2 * np.pi * 9000.0, 4000.0)],
+                    box=((30, 37), (20, 31), (45, 52)))],
+    sources=[("point", (20, 22, 38), 15000.0, 1.0), ("point", (10, 30, 60), 11000.0, 0.6)],
+    probes=[("mid", (25, 20, 40)), ("far", (30, 35, 20)), ("wide", (20, 22, 120))],
+    steps=100, store_fields=False)
+
+
+def test_captured_steps_of_modulus_poles_alone_equal_single_steps(monkeypatch):
+    """Without a density pass the per-cell kernel is the first launch of the branch."""
+    monkeypatch.setitem(C.ADE_CASES, "modulus_only", MODULUS_ONLY)
+    test_captured_ade_steps_equal_single_steps("modulus_only")
