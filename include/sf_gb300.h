@@ -320,7 +320,7 @@ int sf_plan_step_ex(sf_plan* plan, int64_t n_steps, const double* src_values_dev
 int sf_plan_resident(sf_plan* plan, int64_t n_steps, int with_mics, void* stream);
 /* Nonzero, once, when a bounded wait of an earlier state-on-chip launch of this
  * plan expired (that call's results are void).  The launch itself is
- * asynchronous; sf_plan_step_ex and sf_plan_energy report it too.  No
+ * asynchronous; sf_plan_step_ex and the energy readings report it too.  No
  * counterpart in the reference. */
 int sf_plan_status(sf_plan* plan);
 

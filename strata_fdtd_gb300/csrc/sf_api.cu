@@ -1720,6 +1720,7 @@ extern "C" int sf_plan_energy_noalloc(sf_plan* P, double rho, double c, double d
     double sums[2];
     SF_CUDA_OK(cudaMemcpyAsync(sums, scratch + 2 * nb, sizeof(sums), cudaMemcpyDeviceToHost, st));
     SF_CUDA_OK(cudaStreamSynchronize(st));
+    if (int rc = resident_status(P)) return rc;
     const double dV = dx * dx * dx;
     *out_host = 0.5 * sums[0] / (rho * c * c) * dV + 0.5 * rho * sums[1] * dV;
     return 0;

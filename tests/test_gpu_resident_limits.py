@@ -1,4 +1,6 @@
 """The state-on-chip kernel (k_resident) at the limits of what it takes."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -72,6 +74,23 @@ def test_an_expired_wait_is_seen_by_every_read(read):
     ref.run_steps(10)
     _check(s, ref, read)
     np.testing.assert_array_equal(reads["microphone"](s), reads["microphone"](ref))
+
+
+def test_an_expired_wait_is_seen_by_the_energy_reading_without_allocations():
+    s = S.FDTDSolver(shape=(40, 41, 44), resolution=1e-3, c=343.0, rho=1.2, courant=0.6)
+    s.add_source(S.GaussianPulse(position=(20, 20, 20), frequency=20000.0))
+    lib = _native.load()
+    out = ctypes.c_double()
+
+    def energy():
+        return lib.sf_plan_energy_noalloc(s._plan, s.rho, s.c, s.dx, ctypes.byref(out), s._stream())
+
+    s.run_steps(10)
+    assert energy() == 0 and out.value > 0
+    _native.check(lib.sf_plan_set_wait_limit(s._plan, 2000, 1), "sf_plan_set_wait_limit")
+    s.run_steps(10)
+    assert energy() != 0 and b"wait expired" in lib.sf_last_error()
+    assert energy() == 0  # (reported once)
 
 
 def test_buffers_are_released_behind_a_run_in_flight():
