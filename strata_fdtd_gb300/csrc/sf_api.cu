@@ -13,6 +13,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "sf_common.cuh"
@@ -1114,10 +1115,37 @@ bool resident_extra(const sf_plan* P, bool mics, SfResExtra& x) {
     return true;
 }
 
+// Room for the mailboxes of this plan's cut and the corners of one launch's
+// microphone rows; false when the device has none (the plan then steps launch by
+// launch, which needs no memory).  Outgrown buffers are queued for release:
+// launches in flight use them, and cudaFree would wait for everything on the device.
+// The caller holds g_res_mu.
+bool resident_buffers(ResDevice& D, const sf_plan* P, int n_mic, int64_t n_steps) {
+    auto grow = [](auto*& p, size_t& have, size_t need) {
+        if (have >= need) return true;
+        SfRelaxedCapture relaxed;
+        void* q = nullptr;
+        if (cudaMalloc(&q, need) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        sf_defer_free(p, have);
+        p = static_cast<std::remove_reference_t<decltype(p)>>(q);
+        have = need;
+        return true;
+    };
+    const SfResCut& c = P->res_cut;
+    const size_t had = D.bytes;
+    if (!grow(D.mail, D.bytes, sf_resident_mail_bytes(c.bi * c.bj * c.bk, c.side_max))) return false;
+    if (D.bytes != had) D.tag = 0xffffffffu;  // to be cleared
+    return grow(D.corners, D.corner_bytes,
+                sizeof(float) * 8 * n_mic * (size_t)std::min<int64_t>(kResChunk, n_steps));
+}
+
 // Whether n steps of this plan run on the state-on-chip path: automatic
 // kernel choice, no ADE poles, a grid whose blocks fit on the SMs, enough steps
-// to pay for loading the state, and no stream capture (a captured launch would
-// keep its message tags).
+// to pay for loading the state, room for its buffers, and no stream capture (a
+// captured launch would keep its message tags).
 bool resident_fits(sf_plan* P, const SfStepArgs& a, int64_t n_steps, bool deferred, bool mics,
                    cudaStream_t st) {
     if (P->variant != SF_CFG_AUTO || P->i_chunk != 0 || P->poles.n > 0 || n_steps < kResMinSteps ||
@@ -1133,18 +1161,23 @@ bool resident_fits(sf_plan* P, const SfStepArgs& a, int64_t n_steps, bool deferr
                                          extra ? &x : nullptr);
         P->res_key = key;
     }
-    return P->res_cut.kind >= 0 && resident_slot(P);
+    if (P->res_cut.kind < 0 || !resident_slot(P)) return false;
+    std::lock_guard<std::mutex> lock(g_res_mu);
+    return resident_buffers(g_res[P->device], P, mics ? P->n_mic : 0, n_steps);
 }
 
-// n steps of the plan from its current set, in launches of at most kResChunk.
+// n steps of the plan from its current set, in launches of at most kResChunk;
+// kResNoMemory, with nothing queued, when there is no room for the buffers.
+constexpr int kResNoMemory = -1;
 int step_resident(sf_plan* P, const SfStepArgs& a0, int64_t n_steps, const double* src_values,
                   float* trace, float* mic_trace, cudaStream_t st) {
     const SfResCut& c = P->res_cut;
     SfResExtra x{};
     if (c.extra) resident_extra(P, mic_trace != nullptr, x);
-    const size_t mail = sf_resident_mail_bytes(c.bi * c.bj * c.bk, c.side_max);
     std::lock_guard<std::mutex> lock(g_res_mu);
     ResDevice& D = g_res[P->device];
+    if (!resident_buffers(D, P, x.n_mic, n_steps)) return kResNoMemory;
+    x.corners = D.corners;
     SF_CUDA_OK(cudaStreamWaitEvent(st, D.done, 0));
     struct Behind {  // the event moves behind what is queued here, also when a later launch fails
         cudaEvent_t done;
@@ -1156,29 +1189,6 @@ int step_resident(sf_plan* P, const SfStepArgs& a0, int64_t n_steps, const doubl
         }
         ~Behind() { (void)record(); }
     } behind{D.done, st};
-    // (outgrown buffers are queued for release: launches in flight use them, and
-    // cudaFree would wait for everything on the device)
-    if (D.bytes < mail) {
-        SfRelaxedCapture relaxed;
-        sf_defer_free(D.mail, D.bytes);
-        D.mail = nullptr;
-        D.bytes = 0;
-        SF_CUDA_OK(cudaMalloc(&D.mail, mail));
-        D.bytes = mail;
-        D.tag = 0xffffffffu;  // cleared below
-    }
-    if (x.n_mic > 0) {
-        const size_t need = sizeof(float) * 8 * x.n_mic * (size_t)std::min<int64_t>(kResChunk, n_steps);
-        if (D.corner_bytes < need) {
-            SfRelaxedCapture relaxed;
-            sf_defer_free(D.corners, D.corner_bytes);
-            D.corners = nullptr;
-            D.corner_bytes = 0;
-            SF_CUDA_OK(cudaMalloc(&D.corners, need));
-            D.corner_bytes = need;
-        }
-        x.corners = D.corners;
-    }
     for (int64_t s = 0; s < n_steps;) {
         const int n = (int)std::min<int64_t>(kResChunk, n_steps - s);
         if (D.tag > 0xffffffffu - kResChunk) {  // new mailboxes, or the tags wrapped
@@ -1262,8 +1272,10 @@ int sf_plan_step_ex(sf_plan* P, int64_t n_steps, const double* src_values, float
     const bool mics = mic_trace != nullptr && P->n_mic > 0;
     // plane boundaries or weighted sources: sources move after the fused kernel
     const bool deferred = defers(P);
-    if (resident_fits(P, a, n_steps, deferred, mics, st))
-        return step_resident(P, a, n_steps, src_values, trace, mics ? mic_trace : nullptr, st);
+    if (resident_fits(P, a, n_steps, deferred, mics, st)) {
+        const int rc = step_resident(P, a, n_steps, src_values, trace, mics ? mic_trace : nullptr, st);
+        if (rc != kResNoMemory) return rc;
+    }
     const int cfg0 = effective_config(P, a);
     // A pipeline configuration runs whole groups of its steps per launch when
     // nothing has to happen between steps; remaining steps (and plans with

@@ -15,6 +15,7 @@ namespace probe {
 
 std::string calls;        // what was called, in order
 int launches_left = 1000;  // launches that succeed
+size_t room = size_t(1) << 30;  // largest allocation that succeeds
 
 cudaError_t note(const char* what) {
     calls += what;
@@ -22,7 +23,8 @@ cudaError_t note(const char* what) {
     return cudaSuccess;
 }
 template <class T>
-cudaError_t malloc(T** p, size_t) {
+cudaError_t malloc(T** p, size_t bytes) {
+    if (bytes > room) return cudaErrorMemoryAllocation;
     *p = reinterpret_cast<T*>(uintptr_t(1) << 20);
     return note("malloc");
 }
@@ -144,6 +146,7 @@ int main() {
         else if (what == "pair") pair(in);
         else if (what == "weighted") weighted(in);
         else if (what == "steps") steps(in);
+        else if (what == "room") in >> probe::room;
         else if (what == "ade") ade(in);
         else return 2;
     }

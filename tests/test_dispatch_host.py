@@ -28,7 +28,7 @@ def ask(tmp_path_factory):
     def run(lines):
         out = subprocess.run([exe], input="\n".join(lines) + "\n", check=True,
                              capture_output=True, text=True).stdout.splitlines()
-        assert len(out) == len(lines)
+        assert len(out) == sum(not q.startswith("room") for q in lines)
         return [r.split() for r in out]
 
     return run
@@ -76,7 +76,8 @@ def test_launches_are_ordered_behind_one_that_was_queued_before_a_failure(ask, s
     """The event that orders the launches of all streams, and that the mailboxes' release
     waits for, is recorded behind what was queued, also where a later launch fails."""
     (calls,) = ask(["steps 40 40 40 9000 %d" % succeed])
-    assert calls[0] == "wait" and calls.count("launch") == min(3, succeed + 1)
+    assert calls.index("wait") < calls.index("launch")
+    assert calls.count("launch") == min(3, succeed + 1)
     assert calls[-2] == "record" and int(calls[-1]) == (0 if succeed == 3 else 1)
 
 
@@ -86,7 +87,7 @@ def test_outgrown_mailboxes_are_queued_for_release(ask):
     small, large, again = ask(["steps 20 20 20 9 1000", "steps 100 100 100 9 1000",
                                "steps 20 20 20 9 1000"])
     for calls in (small, large):
-        assert calls == "wait mode malloc mode clear launch record 0".split()
+        assert calls == "mode malloc mode wait clear launch record 0".split()
     assert again == "wait launch record 0".split()
 
 
@@ -96,3 +97,12 @@ def test_launches_behind_a_fork_are_plain(ask):
     got = ask(["ade 1 1 1", "ade 0 2 1", "ade 2 0 1", "ade 1 1 0", "ade 0 2 0"])
     assert [" ".join(g) for g in got] == ["plain dependent 0", "plain 0", "plain dependent 0",
                                           "dependent dependent 0", "dependent 0"]
+
+
+def test_no_memory_for_mailboxes_queues_nothing_and_keeps_the_old_ones(ask):
+    """The caller then takes the single-step kernels; a smaller grid still has the
+    mailboxes that were there."""
+    small, large, again = ask(["steps 20 20 20 9 1000", "room 1000", "steps 100 100 100 9 1000",
+                               "steps 20 20 20 9 1000"])
+    assert large == "mode mode -1".split()
+    assert again == "wait launch record 0".split()
