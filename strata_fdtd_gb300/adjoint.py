@@ -226,9 +226,9 @@ class DifferentiableSolver:
     # of the device memory, as several losses may be waiting for theirs.
     _STORE_FRACTION = 1 / 16
 
-    def _segment_store(self):
-        """Room for the pressures of one segment."""
-        return self.torch.empty((self.K,) + self.shape, dtype=self.dtype, device=self.dev)
+    def _segment_store(self, steps):
+        """Room for the pressures of a segment of ``steps`` steps."""
+        return self.torch.empty((steps,) + self.shape, dtype=self.dtype, device=self.dev)
 
     def _last_segment_store(self):
         """Room for the last segment's pressures, which a forward pass that has a
@@ -239,7 +239,7 @@ class DifferentiableSolver:
         if self.K * self.n * self.dtype.itemsize > self._STORE_FRACTION * total:
             return None
         try:
-            return self._segment_store()
+            return self._segment_store(self.K)
         except self.torch.cuda.OutOfMemoryError:
             return None
 
@@ -271,11 +271,12 @@ class DifferentiableSolver:
         """dL/dtheta of L = weight * sum((trace - target)^2) by checkpointed
         recomputation and the reverse-time adjoint; with an occupancy field,
         (dL/dtheta, dL/dphi)."""
-        return self._gradient(theta, trace, target, ckpts, cv, src, weight, occupancy, None)
+        return self._gradient(theta, trace, target, ckpts, cv, src, weight, occupancy, self.K, None)
 
-    def _gradient(self, theta, trace, target, ckpts, cv, src, weight, occupancy, last):
-        """gradient(); ``last``: the last segment's pressures, if the forward pass
-        kept them (overwritten: the earlier segments' come after them)."""
+    def _gradient(self, theta, trace, target, ckpts, cv, src, weight, occupancy, every, last):
+        """gradient() of checkpoints ``every`` so many steps; ``last``: the last
+        segment's pressures, if the forward pass kept them (overwritten: the earlier
+        segments' come after them)."""
         torch = self.torch
         n_steps = trace.shape[0]
         theta = theta.to(self.ext_dtype).contiguous()
@@ -290,11 +291,11 @@ class DifferentiableSolver:
         # or for an FP32 or double-word solve a double-word float pair), zero-filled
         grad_cv = [torch.zeros(self.shape, dtype=torch.float64, device=self.dev) for _ in range(3)]
         desc = self._desc()
-        store = self._segment_store() if last is None else last
-        seg_starts = list(range(0, n_steps, self.K))
+        store = self._segment_store(every) if last is None else last
+        seg_starts = list(range(0, n_steps, every))
         for si in reversed(range(len(seg_starts))):
             s0 = seg_starts[si]
-            n = min(self.K, n_steps - s0)
+            n = min(every, n_steps - s0)
             if last is None or s0 + n < n_steps:
                 work = [[t.clone() for t in ckpts[si]], self._zeros4()]
                 _native.check(self.lib.sf_diff_forward(
@@ -334,6 +335,7 @@ def _make_function():
             loss = ((trace - target.to(trace.dtype)) ** 2).sum()
             ctx.solver = solver
             ctx.saved = (trace, ckpts, cv, src)
+            ctx.every = solver.K  # (may be set anew before the backward pass)
             ctx.last = last
             ctx.save_for_backward(theta, target, occupancy)
             return loss.to(theta.dtype)
@@ -345,7 +347,8 @@ def _make_function():
             last, ctx.last = ctx.last, None  # for one backward pass; another recomputes
             g = ctx.solver._gradient(theta.detach(), trace, target, ckpts, cv, src,
                                      float(grad_out),
-                                     None if occupancy is None else occupancy.detach(), last)
+                                     None if occupancy is None else occupancy.detach(),
+                                     ctx.every, last)
             if occupancy is None:
                 return g.to(theta.dtype), None, None, None, None, None
             return g[0].to(theta.dtype), None, None, None, g[1].to(occupancy.dtype), None
