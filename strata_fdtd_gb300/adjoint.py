@@ -20,6 +20,8 @@ against 27.7.
 from __future__ import annotations
 
 import ctypes
+import threading
+import weakref
 
 import numpy as np
 
@@ -27,6 +29,47 @@ from . import _native
 from .boundaries import PML
 from .grid import UniformGrid
 from .solver import GaussianPulse, step_coefficients
+
+
+class _Kept:
+    """The last segment's pressures of a loss that waits for its backward pass."""
+
+    lock = threading.Lock()
+    waiting: "weakref.WeakSet[_Kept]" = weakref.WeakSet()
+
+    def __init__(self, store):
+        self.store = store
+        self.device, self.bytes = store.device, store.numel() * store.element_size()
+
+    def take(self):
+        """The pressures, once; None when they were dropped."""
+        with _Kept.lock:
+            _Kept.waiting.discard(self)
+            store, self.store = self.store, None
+        return store
+
+    @classmethod
+    def keep(cls, store):
+        kept = cls(store)
+        with cls.lock:
+            cls.waiting.add(kept)
+        return kept
+
+    @classmethod
+    def held(cls, device) -> int:
+        with cls.lock:
+            return sum(k.bytes for k in cls.waiting if k.device == device)
+
+    @classmethod
+    def drop(cls, device) -> bool:
+        """Gives up every waiting loss's pressures (its backward pass recomputes them);
+        whether there were any."""
+        with cls.lock:
+            old = [k for k in cls.waiting if k.device == device]
+            for k in old:
+                k.store = None
+                cls.waiting.discard(k)
+        return bool(old)
 
 
 class _Desc(ctypes.Structure):
@@ -222,26 +265,41 @@ class DifferentiableSolver:
         face coefficients, source values)."""
         return self._forward(theta, n_steps, keep_checkpoints, occupancy, None)
 
-    # Largest buffer kept from a forward pass to its backward pass: a sixteenth
-    # of the device memory, as several losses may be waiting for theirs.
+    # Most that the losses of a process keep from their forward to their backward
+    # passes, all together: a sixteenth of the device memory.
     _STORE_FRACTION = 1 / 16
 
     def _segment_store(self, steps):
         """Room for the pressures of a segment of ``steps`` steps."""
         return self.torch.empty((steps,) + self.shape, dtype=self.dtype, device=self.dev)
 
+    def _device(self):
+        """The device as tensors on it name it (with its index)."""
+        return self.torch.empty(0, device=self.dev).device
+
     def _last_segment_store(self):
         """Room for the last segment's pressures, which a forward pass that has a
         backward pass to come writes as it goes: the adjoint starts from them
         without recomputing that segment and then uses it for the others.  None
-        where it would be too large to keep."""
+        where it would be too large to keep beside those of other waiting losses."""
         total = self.torch.cuda.get_device_properties(self.dev).total_memory
-        if self.K * self.n * self.dtype.itemsize > self._STORE_FRACTION * total:
+        bytes_ = self.K * self.n * self.dtype.itemsize
+        if _Kept.held(self._device()) + bytes_ > self._STORE_FRACTION * total:
             return None
         try:
-            return self._segment_store(self.K)
+            return _Kept.keep(self._segment_store(self.K))
         except self.torch.cuda.OutOfMemoryError:
             return None
+
+    def _with_room(self, work):
+        """work(), once more without the waiting losses' pressures if the device runs
+        out of memory: they are never what a solve fails for."""
+        try:
+            return work()
+        except self.torch.cuda.OutOfMemoryError:
+            if not _Kept.drop(self._device()):
+                raise
+        return work()
 
     def _forward(self, theta, n_steps, keep_checkpoints, occupancy, store):
         """forward(); the last segment's pressures go to ``store``, if given."""
@@ -331,7 +389,8 @@ def _make_function():
         def forward(ctx, theta, target, solver, n_steps, occupancy, keep):
             occ = None if occupancy is None else occupancy.detach()
             last = solver._last_segment_store() if keep and any(ctx.needs_input_grad) else None
-            trace, ckpts, cv, src = solver._forward(theta.detach(), n_steps, True, occ, last)
+            trace, ckpts, cv, src = solver._with_room(lambda: solver._forward(
+                theta.detach(), n_steps, True, occ, None if last is None else last.store))
             loss = ((trace - target.to(trace.dtype)) ** 2).sum()
             ctx.solver = solver
             ctx.saved = (trace, ckpts, cv, src)
@@ -344,11 +403,12 @@ def _make_function():
         def backward(ctx, grad_out):
             theta, target, occupancy = ctx.saved_tensors
             trace, ckpts, cv, src = ctx.saved
-            last, ctx.last = ctx.last, None  # for one backward pass; another recomputes
-            g = ctx.solver._gradient(theta.detach(), trace, target, ckpts, cv, src,
-                                     float(grad_out),
-                                     None if occupancy is None else occupancy.detach(),
-                                     ctx.every, last)
+            kept, ctx.last = ctx.last, None  # for one backward pass; another recomputes
+            last = [None if kept is None else kept.take()]
+            g = ctx.solver._with_room(lambda: ctx.solver._gradient(
+                theta.detach(), trace, target, ckpts, cv, src, float(grad_out),
+                None if occupancy is None else occupancy.detach(), ctx.every,
+                last.pop() if last else None))
             if occupancy is None:
                 return g.to(theta.dtype), None, None, None, None, None
             return g[0].to(theta.dtype), None, None, None, g[1].to(occupancy.dtype), None

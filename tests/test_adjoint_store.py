@@ -82,3 +82,53 @@ def test_a_backward_pass_keeps_the_segments_of_its_forward_pass(after):
     assert [c[:2] for c in s.lib.calls[3:]] == [("adjoint", 5), ("forward", 10), ("adjoint", 10),
                                                 ("forward", 10), ("adjoint", 10)]
     assert all(n <= s.stores[at] for _, n, at in s.lib.calls if at is not None)
+
+
+def test_losses_that_wait_share_one_bound():
+    """24000 bytes each, 60000 for all: the third loss keeps nothing, a loss that was
+    dropped or has had its backward pass makes room for the next."""
+    s = _solver(50)
+    kept = lambda: s.lib.calls[-1][2] is not None  # noqa: E731
+    losses = []
+    for expect in (True, True, False, False):
+        losses.append(_loss(s, 60))
+        assert kept() == expect
+    del losses[0]
+    losses.append(_loss(s, 60))
+    assert kept()
+    losses[0][0].backward()
+    assert losses[0][1].grad is not None
+    losses.append(_loss(s, 60))
+    assert kept()
+    losses.append(_loss(s, 60))
+    assert not kept()
+
+
+def test_a_solve_that_runs_out_of_memory_takes_the_waiting_pressures():
+    """Forward and backward passes run again without them, and the losses that lost
+    theirs recompute them."""
+    s = _solver(50)
+    waiting, _ = _loss(s, 60)
+    plain, left = s._zeros4, [1]
+
+    def short():
+        if left[0]:
+            left[0] -= 1
+            raise torch.cuda.OutOfMemoryError("no room")
+        return plain()
+
+    s._zeros4 = short
+    other, _ = _loss(s, 60)
+    assert s.lib.calls[-1][2] is None  # (its own were dropped too)
+    del s.lib.calls[:]
+    waiting.backward()
+    assert [c[:2] for c in s.lib.calls] == [("forward", 10), ("adjoint", 10), ("forward", 50),
+                                            ("adjoint", 50)]
+    again, _ = _loss(s, 60)
+    left[0] = 1
+    del s.lib.calls[:]
+    other.backward()
+    assert [c[0] for c in s.lib.calls] == ["forward", "adjoint"] * 2
+    with pytest.raises(torch.cuda.OutOfMemoryError):
+        left[0] = 2
+        _loss(s, 60)
