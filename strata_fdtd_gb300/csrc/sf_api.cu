@@ -1292,7 +1292,7 @@ int sf_plan_step_ex(sf_plan* P, int64_t n_steps, const double* src_values, float
     const int tb_cfg = pair >= 0 ? pair : cfg0;
     const bool tb = is_tb(tb_cfg) && !deferred && !mics;
     const int tb_ich = tb ? chunk_for(P, tb_cfg) : 0;
-    const int cfg = (is_pipe(cfg0) || is_tb(cfg0)) ? SF_CFG_TILE_DEFAULT : cfg0;
+    const int cfg = (is_pipe(cfg0) || is_tb(cfg0)) ? default_single(a) : cfg0;
     const int ich = chunk_for(P, cfg);
     SideBranch branch;  // (its events are host work: only where a graph keeps the edges)
     const SideBranch* br = nullptr;

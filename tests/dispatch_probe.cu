@@ -46,6 +46,14 @@ cudaError_t launch(const cudaLaunchConfig_t* cfg, A...) {
 #include "sf_api.cu"
 #include "sf_step.cu"
 
+int sf_launch_step_tile_cfg(const SfStepArgs&, const SfSources&, bool, int cfg, int, cudaStream_t) {
+    probe::note(kSfTileConfigs[cfg].name);
+    return 0;
+}
+int sf_launch_step_tb(const SfStepArgs&, const SfSources&, bool, int cfg, int, float*, cudaStream_t) {
+    probe::note(kSfTbConfigs[cfg].name);
+    return 0;
+}
 int sf_launch_resident(SfResArgs&, const SfSources&, const SfResCut&, cudaStream_t) {
     probe::note("launch");
     return --probe::launches_left >= 0 ? 0 : sf_fail("launch failed");
@@ -120,6 +128,29 @@ void steps(std::istringstream& in) {  // nx ny nz, steps, launches that succeed:
     std::printf("%s%d\n", probe::calls.c_str(), rc);
 }
 
+int config_named(const std::string& name) {
+    for (int q = 0; q < sf_kernel_config_count(); ++q)
+        if (name == sf_kernel_config_name(q)) return q;
+    return -1;
+}
+
+// nx ny nz walls plane_axis, the tuned configuration ("-": none), steps: their kernels
+void tuned(std::istringstream& in) {
+    int nx, ny, nz, walls, axis, n;
+    std::string name;
+    in >> nx >> ny >> nz >> walls >> axis >> name >> n;
+    sf_plan P = plan_of(nx, ny, nz, walls != 0);
+    P.bound = true;
+    P.tuned = name == "-" ? 0 : config_named(name);
+    P.src.n = 1;
+    P.src.s[0].kind = axis >= 0;
+    P.src.s[0].a = axis >= 0 ? axis : 1;
+    const double value = 0.0;
+    probe::calls.clear();
+    const int rc = sf_plan_step(&P, n, &value, nullptr, nullptr);
+    std::printf("%s%d\n", probe::calls.c_str(), rc);
+}
+
 void ade(std::istringstream& in) {  // density poles, modulus poles, serial: the launches of a step
     SfPoles poles{};
     int serial;
@@ -146,6 +177,7 @@ int main() {
         else if (what == "pair") pair(in);
         else if (what == "weighted") weighted(in);
         else if (what == "steps") steps(in);
+        else if (what == "tuned") tuned(in);
         else if (what == "room") in >> probe::room;
         else if (what == "ade") ade(in);
         else return 2;

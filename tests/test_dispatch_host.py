@@ -106,3 +106,13 @@ def test_no_memory_for_mailboxes_queues_nothing_and_keeps_the_old_ones(ask):
                                "steps 20 20 20 9 1000"])
     assert large == "mode mode -1".split()
     assert again == "wait launch record 0".split()
+
+
+def test_steps_beside_tuned_pairs_run_the_default_kernel(ask):
+    """The steps that a tuned two-step configuration leaves over: with walls the kernel
+    whose masks do not spill, as for a plan that was not tuned."""
+    walls, free, plain = ask(["tuned 300 300 300 1 -1 tb2q_r16 7", "tuned 300 300 300 0 -1 tb2q_r20 5",
+                              "tuned 300 300 300 1 -1 - 3"])
+    assert walls == ["tb2q_r16"] * 2 + ["tile_r1_w4_m6_wb"] * 3 + ["0"]
+    assert plain == ["tile_r1_w4_m6_wb"] * 3 + ["0"]
+    assert free[:2] == ["tb2q_r20"] * 2 and free[2:] == ["tile_r1_w4"] + ["0"]
