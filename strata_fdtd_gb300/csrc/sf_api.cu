@@ -674,6 +674,15 @@ bool is_tb(int cfg) { return cfg >= SF_CFG_TB_FIRST; }
 bool tb_fits(const sf_plan* P, const SfStepArgs& a) {
     return P->poles.n == 0 && P->nu == nullptr && sf_tb_supported(a);
 }
+// Whether the two-step kernel cfg should be chosen for this plan's sources: a plane
+// source along y or z acts in every plane of the windows it crosses, which the other
+// blocks then wait for.
+bool tb_suits(const sf_plan* P, int cfg) {
+    if (kSfTbConfigs[cfg - SF_CFG_TB_FIRST].quads == 0) return true;
+    for (int q = 0; q < P->src.n; ++q)
+        if (P->src.s[q].kind != 0 && P->src.s[q].a != 0) return false;
+    return true;
+}
 // float4 warp tiles of 8 blocks per SM (64 registers) without flag bytes, of 6
 // blocks (80) and write-back stores with them, whose masks spill at 64: GB300,
 // 400^3 enclosure 411 -> 336 us a step, 256^3 with a wall 102 -> 92, 120 x 300 x
@@ -699,7 +708,7 @@ int effective_config(const sf_plan* P, const SfStepArgs& a) {
         cfg = default_single(a);
     }
     if (is_tb(cfg)) {  // likewise for the two-step kernels
-        if (tb_fits(P, a)) return cfg;
+        if (tb_fits(P, a) && (P->variant != SF_CFG_AUTO || tb_suits(P, cfg))) return cfg;
         cfg = default_single(a);
     }
     const bool tile_ok =
@@ -723,18 +732,16 @@ int effective_config(const sf_plan* P, const SfStepArgs& a) {
 //           (0.716) 20.5 and 21.1, 176 x 152 x 144 (0.696) 23.7 and 23.4
 //   none    400^3 (0.87) 236 and 318, 256^3 (0.81) 67 and 84, 130 x 140 x 148 (0.72) 13.6
 //           and 14.9, 203 x 167 x 184 (0.65) 32.8 and 34.8
-// A plane source along y or z acts in every plane of the blocks it crosses, which
-// the others then wait for: those plans keep single steps.
+// Plans with a plane source along y or z keep single steps (tb_suits).
 int default_pair(const sf_plan* P, const SfStepArgs& a) {
     if (P->variant != SF_CFG_AUTO || P->tuned > 0 || P->i_chunk > 0 || !tb_fits(P, a) || !sf_tile_supported(a, 4))
         return -1;
-    for (int q = 0; q < P->src.n; ++q)
-        if (P->src.s[q].kind != 0 && P->src.s[q].a != 0) return -1;
     const bool walls = a.flags != nullptr;
     int best = -1;
     double best_share = 0.0;
     for (int q = 0; q < kSfTbConfigCount; ++q) {
         if (kSfTbConfigs[q].quads == 0 || (!walls && kSfTbConfigs[q].rows != 20)) continue;
+        if (!tb_suits(P, SF_CFG_TB_FIRST + q)) return -1;
         double share = 0.0;
         tbq_chunk(P, kSfTbConfigs[q], &share);
         if (best < 0 || share > 1.05 * best_share) {
@@ -1468,6 +1475,8 @@ int sf_plan_autotune(sf_plan* P, int launches, void* stream, float* ms_out, int*
         // slower than single steps, and their fewer launches per step would
         // win a trial timed under a profiler that serialises launches
         if (is_pipe(cfg)) continue;
+        // trials have no sources: a choice that the plan's rule out is not timed
+        if (is_tb(cfg) && !tb_suits(P, cfg)) continue;
         float ms = 0.0f;
         if ((rc = trial(cfg, chunk_for(P, cfg), &ms))) break;
         if (ms_out) ms_out[cfg] = ms;

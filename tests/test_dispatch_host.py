@@ -116,3 +116,20 @@ def test_steps_beside_tuned_pairs_run_the_default_kernel(ask):
     assert walls == ["tb2q_r16"] * 2 + ["tile_r1_w4_m6_wb"] * 3 + ["0"]
     assert plain == ["tile_r1_w4_m6_wb"] * 3 + ["0"]
     assert free[:2] == ["tb2q_r20"] * 2 and free[2:] == ["tile_r1_w4"] + ["0"]
+
+
+@pytest.mark.parametrize("axis", [-1, 0, 1, 2])
+def test_windows_are_left_out_with_a_plane_source_across_their_planes(ask, axis):
+    """By the automatic choice and by a tuned plan alike (-1: a point source)."""
+    auto, tuned = ask(["pair 300 300 300 1 %d" % axis, "tuned 300 300 300 1 %d tb2q_r16 4" % axis])
+    assert auto == (["tb2q_r16"] if axis < 1 else ["-"])
+    assert tuned == (["tb2q_r16"] * 2 if axis < 1 else ["tile_r1_w4_m6_wb"] * 4) + ["0"]
+
+
+# grids of test_gpu_pairs.py: pairs run on them (the padded twin of 223 is 224 wide)
+@pytest.mark.parametrize("walls", [0, 1])
+@pytest.mark.parametrize("shape,axis,pairs", [((210, 132, 224), 0, True), ((131, 204, 168), 0, True),
+                                              ((131, 204, 168), 2, False), ((400, 400, 400), -1, True)])
+def test_where_pairs_run(ask, shape, walls, axis, pairs):
+    ((name,),) = ask(["pair %d %d %d %d %d" % (shape + (walls, axis))])
+    assert name.startswith("tb2q") if pairs else name == "-"

@@ -55,3 +55,10 @@ def test_automatic_choice_equals_single_steps(shape, plane_axis, walls):
     ta, tb = a.get_probe_data(), b.get_probe_data()
     for k in tb:
         np.testing.assert_array_equal(ta[k], tb[k], err_msg=k)
+
+
+def test_the_tuner_leaves_windows_out_with_a_plane_source_across_their_planes():
+    a, b = _build((131, 204, 168), True, 2), _build((131, 204, 168), True, 0)
+    names = [c for c in S.solver.kernel_configs() if c.startswith("tb2q")]
+    assert not set(names) & set(a.autotune(launches=2))
+    assert set(names) <= set(b.autotune(launches=2))
