@@ -289,7 +289,9 @@ int sf_plan_set_wait_limit(sf_plan* plan, int64_t spins, int hold_first_item);
  * makes the fastest the plan's automatic choice, then times that one with
  * 8-48 planes per block (pipelines: 1-8 planes per chunk) unless
  * sf_plan_set_kernel fixed i_chunk, and keeps the fastest; with ADE poles
- * only the warp-tile configurations, timed outside their ADE region.  ms_out
+ * only the warp-tile configurations, timed outside their ADE region.  Where
+ * the state-on-chip kernel takes the plan (sf_plan_resident) it is timed
+ * against that choice, and keeps the calls it takes if it is faster.  ms_out
  * (host, may be NULL) receives sf_kernel_config_count() times per step (-1 =
  * not run);
  * best_out (may be NULL) the chosen configuration.  Synchronises the stream.

@@ -1150,13 +1150,13 @@ bool resident_buffers(ResDevice& D, const sf_plan* P, int n_mic, int64_t n_steps
 }
 
 // Whether n steps of this plan run on the state-on-chip path: automatic
-// kernel choice, no ADE poles, a grid whose blocks fit on the SMs, enough steps
+// kernel choice (the faster one by measurement, if the plan was tuned), no ADE poles, a grid whose blocks fit on the SMs, enough steps
 // to pay for loading the state, room for its buffers, and no stream capture (a
 // captured launch would keep its message tags).
 bool resident_fits(sf_plan* P, const SfStepArgs& a, int64_t n_steps, bool deferred, bool mics,
                    cudaStream_t st) {
     if (P->variant != SF_CFG_AUTO || P->i_chunk != 0 || P->poles.n > 0 || n_steps < kResMinSteps ||
-        P->n_probe > 1024 || stream_capturing(st))
+        P->n_probe > 1024 || (P->tuned > 0 && !P->tuned_on_chip) || stream_capturing(st))
         return false;
     const long long key = P->tables * 4 + (mics ? 2 : 0) + (a.n_probe > 0 ? 1 : 0);
     if (P->res_key != key) {
@@ -1507,6 +1507,35 @@ int sf_plan_autotune(sf_plan* P, int launches, void* stream, float* ms_out, int*
         }
         if (!rc && is_pipe(best)) rc = pipe_check(P, st);
         if (!rc && best_ich != auto_ich) P->tuned_ich = best_ich;
+    }
+    // and whether the state-on-chip kernel, where it takes the plan, is faster still: an
+    // odd number of its steps, which leaves the current set as it is, by a copy of the
+    // plan with nothing between the steps
+    P->tuned_on_chip = false;
+    if (!rc && resident_slot(P)) {
+        constexpr int kSteps = 33;
+        sf_plan T = *P;
+        T.variant = SF_CFG_AUTO;
+        T.tuned = T.n_probe = T.n_plane = T.n_mic = 0;
+        T.src = none;
+        T.res_key = -1;
+        float ms = 0.0f;
+        if (resident_fits(&T, a, kSteps, false, false, st)) {
+            for (int q = 0; q <= launches && !rc; ++q) {
+                if (q == 1 && cudaEventRecord(e0, st) != cudaSuccess) rc = sf_fail("event record failed");
+                T.cur = P->cur;
+                if (!rc) rc = step_resident(&T, a, kSteps, nullptr, nullptr, nullptr, st);
+            }
+            if (rc == kResNoMemory) {
+                rc = 0;
+            } else if (!rc) {
+                if (cudaEventRecord(e1, st) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess)
+                    rc = sf_fail("sf_plan_autotune: timing failed");
+                cudaEventElapsedTime(&ms, e0, e1);
+                P->tuned_on_chip = !rc && ms / (launches * kSteps) < best_ms;
+            }
+            if (!rc) rc = resident_status(P);
+        }
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);

@@ -43,6 +43,7 @@ struct sf_plan {
     int i_chunk = 0;               // planes per block in march / column kernels (0 = auto)
     int tuned = 0;                 // configuration chosen by sf_plan_autotune (0 = none)
     int tuned_ich = 0;             // its planes per block, when the autotuner chose them
+    bool tuned_on_chip = false;    // the autotuner found the state-on-chip kernel faster than it
     long long steps_done = 0;      // steps issued so far (alternates the chunk order)
     int n_mic = 0;                 // microphone rows: 8 corner cells and weights each
     long long* mic_idx = nullptr;  // owned

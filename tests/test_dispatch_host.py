@@ -133,3 +133,11 @@ def test_windows_are_left_out_with_a_plane_source_across_their_planes(ask, axis)
 def test_where_pairs_run(ask, shape, walls, axis, pairs):
     ((name,),) = ask(["pair %d %d %d %d %d" % (shape + (walls, axis))])
     assert name.startswith("tb2q") if pairs else name == "-"
+
+
+def test_a_tuned_choice_decides_for_small_grids_too(ask):
+    """A plan that the tuner has decided on, without having found the state-on-chip
+    kernel faster, runs that choice; one that was not tuned stays on the chip."""
+    tuned, plain = ask(["tuned 40 40 40 0 -1 tile_r1_w8 9", "tuned 40 40 40 0 -1 - 9"])
+    assert tuned == ["tile_r1_w8"] * 9 + ["0"]
+    assert plain.count("launch") == 1 and not any(c.startswith("tile") for c in plain)

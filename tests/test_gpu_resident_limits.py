@@ -123,3 +123,22 @@ def test_buffers_are_released_behind_a_run_in_flight():
     _check(b, ref, "behind the release")
     _check(c, ref, "new mailboxes")
     a.synchronize()
+
+
+@pytest.mark.parametrize("shape", [(40, 41, 44), (96, 92, 100)])
+def test_the_tuner_times_the_state_on_chip_kernel(shape):
+    """It is the faster one on these grids and keeps its calls; the trials leave the
+    state alone, with an odd number of steps behind it too."""
+    out = []
+    for tune in (False, True):
+        s = S.FDTDSolver(shape=shape, resolution=1e-3, c=343.0, rho=1.2, courant=0.6)
+        s.add_boundary(S.ABCFirstOrder())
+        s.add_source(S.GaussianPulse(position=(20, 20, 20), frequency=20000.0))
+        s.add_probe("a", (30, 30, 30))
+        s.run_steps(11)
+        if tune:
+            s.autotune(launches=3)
+        assert _resident(s, 40)
+        s.run_steps(9)
+        out.append(s)
+    _check(*out, shape)
