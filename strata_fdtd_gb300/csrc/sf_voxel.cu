@@ -1091,6 +1091,7 @@ Kept g_keep[kKeepDevices];
 class Scratch {
   public:
     char* p = nullptr;
+    bool idle = true;  // nothing queued uses it
     int take(size_t bytes, cudaStream_t st) {
         st_ = st;
         cudaGetDevice(&dev_);
@@ -1117,8 +1118,9 @@ class Scratch {
         SF_CUDA_OK(cudaMallocAsync(reinterpret_cast<void**>(&p), bytes, st));
         return 0;
     }
-    ~Scratch() {  // the call has waited for its stream by now
+    ~Scratch() {
         if (kept_) {
+            if (!idle) (void)cudaStreamSynchronize(st_);  // a call that failed on its way
             std::lock_guard<std::mutex> lock(g_keep_mu);
             g_keep[dev_].lent = false;
         } else if (p) {
@@ -1189,6 +1191,7 @@ int sf_launch_voxelize(const sf_sdf_node* nodes, int n_nodes, int nx, int ny, in
     Scratch scratch;
     if (int rc = scratch.take(off_q + sizeof(unsigned) * (size_t)blocks, st)) return rc;
     char* b = scratch.p;
+    scratch.idle = false;
     if (cudaMemcpyAsync(b, host.data(), sent, cudaMemcpyHostToDevice, st) != cudaSuccess)
         return sf_fail("sf_voxelize: upload failed");
     const VxGrid g{nx, ny, nz, invert, res, coords ? reinterpret_cast<const double*>(b + off_co) : nullptr,
@@ -1210,6 +1213,7 @@ int sf_launch_voxelize(const sf_sdf_node* nodes, int n_nodes, int nx, int ny, in
     k_vx_cells<<<152 * 16, 128, 0, st>>>(g, ivp, prog, n_marked);
     if (cudaGetLastError() != cudaSuccess) return sf_fail("k_voxelize launch failed");
     if (cudaStreamSynchronize(st) != cudaSuccess) return sf_fail("sf_voxelize: kernel failed");
+    scratch.idle = true;
     return 0;
 }
 

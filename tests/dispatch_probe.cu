@@ -47,8 +47,14 @@ cudaError_t launch(const cudaLaunchConfig_t* cfg, A...) {
 #define cudaHostAlloc(p, n, ...) (*(p) = ::calloc(1, n), cudaSuccess)
 #define cudaHostGetDevicePointer(d, h, ...) (*(d) = (h), cudaSuccess)
 #define cudaEventCreateWithFlags(e, ...) (*(e) = reinterpret_cast<cudaEvent_t>(uintptr_t(4096)), cudaSuccess)
+#define cudaGetDevice(d) (*(d) = 0, cudaSuccess)
+#define cudaMallocAsync(p, n, ...) probe::malloc(p, n)
+#define cudaFreeAsync(...) probe::note("free-behind")
+#define cudaMemcpyAsync(...) probe::note("copy")
+#define cudaStreamSynchronize(...) probe::note("sync")
 #include "sf_api.cu"
 #include "sf_step.cu"
+#include "sf_voxel.cu"
 
 int sf_launch_step_tile_cfg(const SfStepArgs&, const SfSources&, bool, int cfg, int, cudaStream_t) {
     probe::note(kSfTileConfigs[cfg].name);
@@ -155,6 +161,20 @@ void tuned(std::istringstream& in) {
     std::printf("%s%d\n", probe::calls.c_str(), rc);
 }
 
+// nx ny nz: the calls of a mask (without a device its kernels fail to launch) and
+// whether its scratch memory may be lent again
+void mask(std::istringstream& in) {
+    int nx, ny, nz;
+    in >> nx >> ny >> nz;
+    sf_sdf_node ball{};
+    ball.op = 2;
+    ball.s0 = 1.0;
+    probe::calls.clear();
+    const int rc = sf_voxelize(&ball, 1, nx, ny, nz, 0.1, 0, reinterpret_cast<uint8_t*>(uintptr_t(4096)),
+                               nullptr);
+    std::printf("%s%s%d\n", probe::calls.c_str(), g_keep[0].lent ? "lent " : "", rc);
+}
+
 void ade(std::istringstream& in) {  // density poles, modulus poles, serial: the launches of a step
     SfPoles poles{};
     int serial;
@@ -182,6 +202,7 @@ int main() {
         else if (what == "weighted") weighted(in);
         else if (what == "steps") steps(in);
         else if (what == "tuned") tuned(in);
+        else if (what == "mask") mask(in);
         else if (what == "room") in >> probe::room;
         else if (what == "ade") ade(in);
         else return 2;

@@ -141,3 +141,10 @@ def test_a_tuned_choice_decides_for_small_grids_too(ask):
     tuned, plain = ask(["tuned 40 40 40 0 -1 tile_r1_w8 9", "tuned 40 40 40 0 -1 - 9"])
     assert tuned == ["tile_r1_w8"] * 9 + ["0"]
     assert plain.count("launch") == 1 and not any(c.startswith("tile") for c in plain)
+
+
+def test_a_mask_that_fails_waits_before_its_scratch_is_lent_again(ask):
+    """Copies and kernels queued before the failure still use it."""
+    (calls,) = ask(["mask 40 40 40"])
+    assert int(calls[-1]) != 0 and "lent" not in calls
+    assert "sync" in calls[calls.index("copy"):]
