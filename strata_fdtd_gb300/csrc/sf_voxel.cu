@@ -646,15 +646,11 @@ __device__ float2 eval_iv(const IvNode* __restrict__ prog, int n, float2 x, floa
 
 // ---- the mask -----------------------------------------------------------------
 
-__device__ __forceinline__ double cell_centre(const double* __restrict__ coords, int off, int i,
-                                              double res) {
-    return coords ? coords[off + i] : d_add(d_mul((double)i, res), d_mul(res, 0.5));
-}
-
 struct VxGrid {
     int nx, ny, nz, invert;
+    int first, planes;     // the grid's plane that is plane 0 here (a slab), its planes
     double res;
-    const double* coords;  // nx + ny + nz cell centres of a nonuniform grid, or null
+    const double* coords;  // planes + ny + nz cell centres of a nonuniform grid, or null
     float2* axis;          // the same centres as intervals (k_vx_axes)
     unsigned* count;       // queued blocks
     unsigned* queue;
@@ -664,13 +660,19 @@ struct VxGrid {
     uint8_t* out;
 };
 
+__device__ __forceinline__ double cell_centre(const VxGrid& g, int axis, int i) {
+    if (axis == 0) i += g.first;
+    if (g.coords) return g.coords[(axis > 0 ? g.planes : 0) + (axis > 1 ? g.ny : 0) + i];
+    return d_add(d_mul((double)i, g.res), d_mul(g.res, 0.5));
+}
+
 // Cell centres as intervals, and an empty queue.
 __global__ void k_vx_axes(VxGrid g) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t == 0) *g.count = 0;
     if (t >= g.nx + g.ny + g.nz) return;
-    const int i = t < g.nx ? t : (t < g.nx + g.ny ? t - g.nx : t - g.nx - g.ny);
-    const double c = cell_centre(g.coords, t - i, i, g.res);
+    const int axis = t < g.nx ? 0 : (t < g.nx + g.ny ? 1 : 2);
+    const double c = cell_centre(g, axis, t - (axis > 0 ? g.nx : 0) - (axis > 1 ? g.ny : 0));
     g.axis[t] = iv(__double2float_rd(c), __double2float_ru(c));
 }
 
@@ -795,8 +797,8 @@ __global__ void __launch_bounds__(128) k_vx_cells(VxGrid g, const IvNode* __rest
         int i, j, k, err = 0;  // the program has passed check_program
         queued_cell(g, t, i, j, k);
         put(i, j, k,
-            eval_sdf<true>(prog, n, cell_centre(g.coords, 0, i, g.res), cell_centre(g.coords, g.nx, j, g.res),
-                           cell_centre(g.coords, g.nx + g.ny, k, g.res), &err, lost[t >> 6]) <= 0.0);
+            eval_sdf<true>(prog, n, cell_centre(g, 0, i), cell_centre(g, 1, j), cell_centre(g, 2, k), &err,
+                           lost[t >> 6]) <= 0.0);
     };
     __syncthreads();
     for (unsigned long long first = (unsigned long long)blockIdx.x * 128; first < cells;
@@ -1078,7 +1080,7 @@ std::vector<sf_sdf_node> mark_program(const sf_sdf_node* nodes, int n, std::vect
 // Device memory of a voxelisation, kept between calls (one block per device
 // of at most kKeepBytes, lent to one call at a time; released with the
 // deferred frees): a call's allocation took longer than its kernels.
-constexpr size_t kKeepBytes = size_t(72) << 20;  // 500^3 cells: 26 MB
+constexpr size_t kKeepBytes = size_t(72) << 20;  // 500^3 cells: 25 MB
 constexpr int kKeepDevices = 64;
 struct Kept {
     char* p = nullptr;
@@ -1115,7 +1117,11 @@ class Scratch {
                 }
             }
         }
-        SF_CUDA_OK(cudaMallocAsync(reinterpret_cast<void**>(&p), bytes, st));
+        if (const cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&p), bytes, st)) {
+            p = nullptr;
+            (void)cudaGetLastError();
+            return sf_fail_cuda(e, "sf_voxelize: scratch memory", __FILE__, __LINE__);
+        }
         return 0;
     }
     ~Scratch() {
@@ -1157,11 +1163,7 @@ int sf_launch_voxelize(const sf_sdf_node* nodes, int n_nodes, int nx, int ny, in
                        const double* const* coords, int invert, uint8_t* out, cudaStream_t st) {
     if (!check_program(nodes, n_nodes))
         return sf_fail("sf_voxelize: malformed SDF program (stack error)");
-    const int si = (nx + 15) / 16, sj = (ny + 15) / 16, sk = (nz + 31) / 32;
-    const long long supers = (long long)si * sj * sk;
-    const long long blocks =
-        (long long)((nx + 3) / 4) * ((ny + 3) / 4) * ((nz + 3) / 4);
-    if (blocks > 0xffffffffLL) return sf_fail("sf_voxelize: grid too large");
+    const int sj = (ny + 15) / 16, sk = (nz + 31) / 32;
     std::vector<int> first_bit;
     const std::vector<sf_sdf_node> marked = mark_program(nodes, n_nodes, first_bit);
     const int n_marked = (int)marked.size();
@@ -1169,8 +1171,33 @@ int sf_launch_voxelize(const sf_sdf_node* nodes, int n_nodes, int nx, int ny, in
     const size_t off_iv = up16(sizeof(sf_sdf_node) * n_marked);
     const size_t off_co = off_iv + up16(sizeof(IvNode) * n_marked);
     const size_t sent = off_co + (coords ? up16(sizeof(double) * n_axis) : 0);
-    const size_t off_ax = sent, off_ct = off_ax + up16(sizeof(float2) * n_axis), off_sd = off_ct + 16,
-                 off_l = off_sd + up16((size_t)supers), off_q = off_l + 8 * (size_t)(supers + blocks);
+    // Large grids are done in slabs of planes, so that the scratch memory (12 bytes a
+    // block) stays within what is kept; a device with less room gets smaller slabs.
+    struct Slab {
+        long long supers, blocks;
+        size_t ax, ct, sd, l, q, end;
+    };
+    auto slab_of = [&](int planes) {
+        Slab b;
+        b.supers = (long long)((planes + 15) / 16) * sj * sk;
+        b.blocks = (long long)((planes + 3) / 4) * ((ny + 3) / 4) * ((nz + 3) / 4);
+        b.ax = sent;
+        b.ct = b.ax + up16(sizeof(float2) * n_axis);
+        b.sd = b.ct + 16;
+        b.l = b.sd + up16((size_t)b.supers);
+        b.q = b.l + 8 * (size_t)(b.supers + b.blocks);
+        b.end = b.q + sizeof(unsigned) * (size_t)b.blocks;
+        return b;
+    };
+    auto half = [](int planes) {  // in whole blocks, from 32 planes on in whole super-blocks
+        const int h = (planes + 1) / 2, unit = h > 16 ? 16 : 4;
+        return (h + unit - 1) / unit * unit;
+    };
+    int planes = nx;
+    Slab slab = slab_of(planes);
+    while (planes > 4 && (slab.end - slab.ct > kKeepBytes || slab.blocks > 0xffffffffLL))
+        slab = slab_of(planes = half(planes));
+    if (slab.blocks > 0xffffffffLL) return sf_fail("sf_voxelize: grid too large");
     std::vector<char> host(sent);
     std::memcpy(host.data(), marked.data(), sizeof(sf_sdf_node) * n_marked);
     for (int q = 0; q < n_marked; ++q) {
@@ -1189,28 +1216,36 @@ int sf_launch_voxelize(const sf_sdf_node* nodes, int n_nodes, int nx, int ny, in
     }
     SfRelaxedCapture relaxed;  // (the call allocates and waits)
     Scratch scratch;
-    if (int rc = scratch.take(off_q + sizeof(unsigned) * (size_t)blocks, st)) return rc;
+    while (int rc = scratch.take(slab.end, st)) {
+        if (planes <= 4) return rc;
+        slab = slab_of(planes = half(planes));
+    }
     char* b = scratch.p;
     scratch.idle = false;
     if (cudaMemcpyAsync(b, host.data(), sent, cudaMemcpyHostToDevice, st) != cudaSuccess)
         return sf_fail("sf_voxelize: upload failed");
-    const VxGrid g{nx, ny, nz, invert, res, coords ? reinterpret_cast<const double*>(b + off_co) : nullptr,
-                   reinterpret_cast<float2*>(b + off_ax), reinterpret_cast<unsigned*>(b + off_ct),
-                   reinterpret_cast<unsigned*>(b + off_q), si, sj, sk,
-                   reinterpret_cast<unsigned long long*>(b + off_l),
-                   reinterpret_cast<unsigned char*>(b + off_sd), out};
     const sf_sdf_node* prog = reinterpret_cast<const sf_sdf_node*>(b);
     const IvNode* ivp = reinterpret_cast<const IvNode*>(b + off_iv);
-    k_vx_axes<<<(unsigned)((n_axis + 127) / 128), 128, 0, st>>>(g);
-    // One thread walks the whole program for a super-block, so that takes its
-    // latency however few there are, and pays where they fill the chip.  Calls with
-    // and without (16 resonators): 180 x 240 x 157 (900 super-blocks) 293 and 273
-    // us, 300^3 (3610) 313 and 481, 400^3 313 and 747; enclosure 200^3 (1183) 129
-    // and 112 to 131, 400^3 (8125) 138 and 172.
-    const bool look = supers >= kSuperMin;
-    if (look) k_vx_super<<<(unsigned)((supers + 31) / 32), 32, 0, st>>>(g, ivp, n_marked);
-    k_vx_blocks<<<(unsigned)supers, 128, 0, st>>>(g, ivp, n_marked, look);
-    k_vx_cells<<<152 * 16, 128, 0, st>>>(g, ivp, prog, n_marked);
+    for (int first = 0; first < nx; first += planes) {
+        const int n = nx - first < planes ? nx - first : planes, si = (n + 15) / 16;
+        const VxGrid g{n, ny, nz, invert, first, nx, res,
+                       coords ? reinterpret_cast<const double*>(b + off_co) : nullptr,
+                       reinterpret_cast<float2*>(b + slab.ax), reinterpret_cast<unsigned*>(b + slab.ct),
+                       reinterpret_cast<unsigned*>(b + slab.q), si, sj, sk,
+                       reinterpret_cast<unsigned long long*>(b + slab.l),
+                       reinterpret_cast<unsigned char*>(b + slab.sd), out + (long long)first * ny * nz};
+        const long long supers = (long long)si * sj * sk;
+        k_vx_axes<<<(unsigned)(((long long)n + ny + nz + 127) / 128), 128, 0, st>>>(g);
+        // One thread walks the whole program for a super-block, so that takes its
+        // latency however few there are, and pays where they fill the chip.  Calls with
+        // and without (16 resonators): 180 x 240 x 157 (900 super-blocks) 293 and 273
+        // us, 300^3 (3610) 313 and 481, 400^3 313 and 747; enclosure 200^3 (1183) 129
+        // and 112 to 131, 400^3 (8125) 138 and 172.
+        const bool look = supers >= kSuperMin;
+        if (look) k_vx_super<<<(unsigned)((supers + 31) / 32), 32, 0, st>>>(g, ivp, n_marked);
+        k_vx_blocks<<<(unsigned)supers, 128, 0, st>>>(g, ivp, n_marked, look);
+        k_vx_cells<<<152 * 16, 128, 0, st>>>(g, ivp, prog, n_marked);
+    }
     if (cudaGetLastError() != cudaSuccess) return sf_fail("k_voxelize launch failed");
     if (cudaStreamSynchronize(st) != cudaSuccess) return sf_fail("sf_voxelize: kernel failed");
     scratch.idle = true;

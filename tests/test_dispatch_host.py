@@ -148,3 +148,12 @@ def test_a_mask_that_fails_waits_before_its_scratch_is_lent_again(ask):
     (calls,) = ask(["mask 40 40 40"])
     assert int(calls[-1]) != 0 and "lent" not in calls
     assert "sync" in calls[calls.index("copy"):]
+
+
+def test_a_mask_takes_what_memory_there_is(ask):
+    """12 MB of scratch for 400^3 cells: with less room the planes are done in slabs."""
+    full, less, none = ask(["mask 400 400 400", "room 600000", "mask 500 500 500", "room 1000",
+                            "mask 600 600 600"])
+    for calls in (full, less):
+        assert "malloc" in calls and "copy" in calls
+    assert "copy" not in none and int(none[-1]) != 0

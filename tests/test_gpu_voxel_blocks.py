@@ -77,3 +77,30 @@ def test_stretched_grid_equals_point_evaluation(name):
     pts = np.stack(np.meshgrid(grid.x_coords, grid.y_coords, grid.z_coords, indexing="ij"), -1)
     want = solid.contains(pts.reshape(-1, 3)).reshape(grid.shape)
     assert np.array_equal(solid.voxelize(grid), want)
+
+
+@pytest.mark.parametrize("stretched", [False, True])
+def test_slabs_of_a_large_grid(stretched):
+    """270 million cells of a thin grid are done in two slabs of planes: cells of the
+    planes around their border, and cells drawn from the whole grid."""
+    shape = (450, 5, 120001)
+    rng = np.random.default_rng(7)
+    if stretched:
+        coords = [np.cumsum(rng.uniform(0.7, 1.3, n)) * R for n in shape]
+        grid = S.NonuniformGrid(*coords)
+    else:
+        coords = [np.arange(n) * R + R / 2 for n in shape]
+        grid = S.UniformGrid(shape, R)
+    solid = S.Difference(
+        S.Union(S.Cylinder(p1=(0.2, 0.002, 0.0), p2=(0.25, 0.003, 121.0), radius=0.1),
+                S.Sphere(center=(0.24, 0.002, 60.0), radius=0.21)),
+        S.Sphere(center=(0.23, 0.0025, 30.0), radius=0.05))
+    mask = solid.voxelize(grid)
+    cells = [rng.integers(0, n, 1_000_000) for n in shape]
+    border = [rng.integers(236, 244, 300_000), rng.integers(0, 5, 300_000),
+              np.concatenate([rng.integers(0, 120001, 100_000), rng.integers(59700, 60300, 100_000),
+                              rng.integers(29900, 30100, 100_000)])]
+    for i, j, k in (cells, border):
+        points = np.stack([coords[0][i], coords[1][j], coords[2][k]], axis=1)
+        np.testing.assert_array_equal(mask[i, j, k], solid.contains(points))
+        assert 0.02 < mask[i, j, k].mean() < 0.98
