@@ -314,11 +314,16 @@ int sf_plan_step_ex(sf_plan* plan, int64_t n_steps, const double* src_values_dev
                     float* trace_dev, float* mic_trace_dev, void* stream);
 
 /* Whether sf_plan_step_ex with n_steps steps (and, with_mics != 0, microphone
- * rows) on this stream now runs the state-on-chip kernel, which advances all of
- * them in one launch (automatic kernel choice, grids that fit on the SMs, no
- * ADE poles, plane boundaries or weighted sources, no stream capture): 1 or 0.
- * A caller that replays captured launches of its own need not do so then.  No
- * counterpart in the reference. */
+ * rows) on this stream now runs the state-on-chip kernel, which advances up to
+ * 4096 of them per launch: 1 or 0.  It does for 8 steps or more with the automatic
+ * kernel choice (and, after sf_plan_autotune, where it was the faster one) on grids
+ * that fit on the SMs, with plane boundaries, sources weighted on the pressure (no
+ * cell listed twice) and up to 64 microphone rows, without ADE poles and outside
+ * stream capture, while there is device memory for its mailboxes (at most 64 MiB,
+ * shared by all plans of a device until sf_release_deferred).  Its launches of one
+ * device run one after another, whatever their streams.  A caller that replays
+ * captured launches of its own need not do so then.  No counterpart in the
+ * reference. */
 int sf_plan_resident(sf_plan* plan, int64_t n_steps, int with_mics, void* stream);
 /* Nonzero, once, when a bounded wait of an earlier state-on-chip launch of this
  * plan expired (that call's results are void).  The launch itself is

@@ -778,14 +778,6 @@ void ade_region(const sf_plan* P, int cfg, int ich, int lo[3], int hi[3]) {
     }
 }
 
-
-// Planes per block of a float4 warp-tile configuration: of 4 to 8 and
-// auto_chunk's choice where that is larger, the number with the best product of
-// (blocks / whole waves of resident blocks) and (planes / planes + half a plane
-// for the chunk's prologue), among those that fill one wave.  Against
-// auto_chunk alone (4 planes for these): 203 x 167 x 184 with walls 40.8 -> 39.9
-// us a step, 176 x 152 x 144 27.2 -> 26.3, free 300 x 90 x 120 20.5 -> 18.7.
-int tile_chunk(const sf_plan* P, const SfTileConfig& t);
 // Planes per block of a window configuration of the two-step kernel: the number of
 // chunks with the best product of (blocks / whole waves) and (planes / planes + 2
 // for the overlap and the lag).  *share: of the threads' cells, those that are
@@ -807,6 +799,13 @@ int tbq_chunk(const sf_plan* P, const SfTbConfig& c, double* share) {
     if (share) *share = best_eff * P->d.nz / (double)(ck * w) * P->d.ny / (double)(cj * h);
     return best;
 }
+
+// Planes per block of a float4 warp-tile configuration: of 4 to 8 and
+// auto_chunk's choice where that is larger, the number with the best product of
+// (blocks / whole waves of resident blocks) and (planes / planes + half a plane
+// for the chunk's prologue), among those that fill one wave.  Against
+// auto_chunk alone (4 planes for these): 203 x 167 x 184 with walls 40.8 -> 39.9
+// us a step, 176 x 152 x 144 27.2 -> 26.3, free 300 x 90 x 120 20.5 -> 18.7.
 int tile_chunk(const sf_plan* P, const SfTileConfig& t) {
     const int jspan = 4 * t.rows * t.warps;
     const long long cols = (long long)((P->d.nz + 31) / 32) * ((P->d.ny + jspan - 1) / jspan);

@@ -1032,9 +1032,10 @@ __global__ void __launch_bounds__(MAXT, 1) k_resident(const __grid_constant__ Sf
 // ---- partition ----------------------------------------------------------------
 
 // Planes per thread, threads at most (512 of 128 registers: with 640 to 768 the
-// kernels spilled, 52 x 44 x 48 0.73 ms against 0.69 for 250 steps, 100^3 2.44
-// against 2.22 for 500; loading operands ahead of the stores spilled again, 2.36
-// to 2.46).
+// kernels spilled more, 52 x 44 x 48 0.73 ms against 0.69 for 250 steps, 100^3 2.44
+// against 2.22 for 500; loading operands ahead of the stores too, 2.36 to 2.46.  At
+// 128 the variants of one and two planes do not spill, those of four store 32 to 52
+// bytes, those of eight 24 to 136).
 // More planes hold more cells per SM (the registers of a thread grow more
 // slowly than its cells) but make a longer chain per phase: the smallest L
 // whose blocks fit is taken.

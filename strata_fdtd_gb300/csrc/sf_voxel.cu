@@ -1079,7 +1079,8 @@ std::vector<sf_sdf_node> mark_program(const sf_sdf_node* nodes, int n, std::vect
 
 // Device memory of a voxelisation, kept between calls (one block per device
 // of at most kKeepBytes, lent to one call at a time; released with the
-// deferred frees): a call's allocation took longer than its kernels.
+// deferred frees): a call's allocation took longer than its kernels.  Grids that
+// need more are done in slabs of planes.
 constexpr size_t kKeepBytes = size_t(72) << 20;  // 500^3 cells: 25 MB
 constexpr int kKeepDevices = 64;
 struct Kept {
