@@ -335,15 +335,19 @@ class FDTDSolver:
     def _check_status(self, since: int | None = None):
         """Raise when an earlier asynchronous run of this solver failed and some of
         its state is still in place, or when a run failed after ``since`` of them."""
-        twin = getattr(self, "_pad_twin", None)
-        for plan in (self._plan,) if twin is None else (self._plan, twin.plan):
-            self._checked(self._lib.sf_plan_status(plan), "sf_plan_step", status=True)
+        status, twin = self._lib.sf_plan_status, self.__dict__.get("_pad_twin")
+        rc = status(self._plan)
+        if twin is not None:
+            rc = rc or status(twin.plan)
+        if rc:
+            self._checked(rc, "sf_plan_step", status=True)
         if self._void or (since is not None and since != self._failures):
             raise _native.NativeError(self._failure)
 
     def _given(self, name):
         """The host has given this field's state."""
-        self._void = self._void - {name}
+        if self._void:
+            self._void = self._void - {name}
 
     def _set_field(self, name, value):
         arr = np.asarray(value)
@@ -969,7 +973,8 @@ class FDTDSolver:
         self._step_count += n
 
     def _flush_traces(self):
-        self._check_status()
+        if not (self._pending_traces or self._pending_mics):
+            self._check_status()
         while self._pending_traces:  # off the list as they are appended
             trace, names = self._pending_traces[0]
             host = trace.cpu().numpy()

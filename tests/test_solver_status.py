@@ -73,7 +73,7 @@ class _Recorder:
 
 
 def test_microphones_alone_report_a_failed_run():
-    s = _solver(0, 1)
+    s = _solver(1)
     s._microphones["m"] = _Recorder()
     s._pending_mics = [(torch.ones(3, 1), [("m", 1)], [0.0] * 3)]
     with pytest.raises(_native.NativeError):
@@ -122,7 +122,7 @@ def test_fields_given_by_the_host_end_a_failed_run():
 
 def test_a_trace_that_was_appended_leaves_the_list():
     """A failure between two traces: the first stays with its probe, once."""
-    s = _solver(0, 0, 1)
+    s = _solver(0, 1)  # (asked once behind each trace's copy)
     s._probes["a"] = _Recorder()
     s._pending_traces = [(torch.ones(3, 1), ["a"]), (torch.ones(2, 1), ["a"])]
     for _ in range(2):
