@@ -1148,10 +1148,10 @@ bool resident_buffers(ResDevice& D, const sf_plan* P, int n_mic, int64_t n_steps
                 sizeof(float) * 8 * n_mic * (size_t)std::min<int64_t>(kResChunk, n_steps));
 }
 
-// Whether n steps of this plan run on the state-on-chip path: automatic
-// kernel choice (the faster one by measurement, if the plan was tuned), no ADE poles, a grid whose blocks fit on the SMs, enough steps
-// to pay for loading the state, room for its buffers, and no stream capture (a
-// captured launch would keep its message tags).
+// Whether n steps of this plan run on the state-on-chip path: automatic kernel
+// choice (for a tuned plan where the tuner found this the faster one), no ADE poles, a
+// grid whose blocks fit on the SMs, enough steps to pay for loading the state, room for
+// its buffers, and no stream capture (a captured launch would keep its message tags).
 bool resident_fits(sf_plan* P, const SfStepArgs& a, int64_t n_steps, bool deferred, bool mics,
                    cudaStream_t st) {
     if (P->variant != SF_CFG_AUTO || P->i_chunk != 0 || P->poles.n > 0 || n_steps < kResMinSteps ||

@@ -1168,7 +1168,7 @@ class FDTDSolver:
         names = kernel_configs()
         ms = (C.c_float * len(names))()
         best = C.c_int()
-        _native.check(self._lib.sf_plan_autotune(self._plan, int(launches), self._stream(),
+        self._checked(self._lib.sf_plan_autotune(self._plan, int(launches), self._stream(),
                                                  ms, C.byref(best)), "sf_plan_autotune")
         self._graph_epoch += 1
         out = {n: float(ms[q]) for q, n in enumerate(names) if ms[q] >= 0}

@@ -129,3 +129,23 @@ def test_a_trace_that_was_appended_leaves_the_list():
         with pytest.raises(_native.NativeError):
             s._flush_traces()
         assert len(s._probes["a"]._samples) == 3
+
+
+def test_a_failed_run_that_the_tuner_reports_is_not_forgotten(monkeypatch):
+    """sf_plan_autotune synchronises and reports it; the fields are void all the same."""
+    s = _solver()
+    s._lib.sf_plan_autotune = lambda *a: 1
+    s._sync_tables = lambda: None
+    s._stream = lambda: None
+    s._graph_epoch = 0
+    monkeypatch.setattr(_native, "check", _failing_check)
+    with pytest.raises(_native.NativeError):
+        s.autotune()
+    for f in FIELDS:
+        with pytest.raises(_native.NativeError):
+            getattr(s, f)
+
+
+def _failing_check(rc, what=""):
+    if rc:
+        raise _native.NativeError(what + ": k_resident: a dependency wait expired (results ...)")
