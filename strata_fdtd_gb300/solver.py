@@ -1219,8 +1219,8 @@ class FDTDSolver:
         if name is not None:
             if name not in self._probes:
                 raise KeyError(f"Probe '{name}' not found")
-            return {name: self._probes[name].get_data()}
-        return {n: pr.get_data() for n, pr in self._probes.items()}
+            return {name: np.array(self._probes[name]._samples, dtype=np.float32)}
+        return {n: np.array(pr._samples, dtype=np.float32) for n, pr in self._probes.items()}
 
     def get_snapshots(self):
         self._snap_collect()
